@@ -171,7 +171,8 @@ def _wire(sim, case, L):
             n -= 1
         cm = f"cutoff {rc!r} nx {n} ny {n} nz {n}" + skin
     else:
-        cm = f"cutoff {rc!r} maxneighbors 512 each 5" + skin
+        # without a skin the reference's own rebuild clock, with one the displacement rule
+        cm = f"cutoff {rc!r} maxneighbors 512" + (skin if skin else " each 5")
     sim.set_cell_manager(gbmd.Plugin(case["cm"], cm))
     sim.add_potential(gbmd.Plugin(plugin, args))
     sim.set_integrator(gbmd.Plugin(case.get("integ", "velocityverlet"), f"dt {dt!r}"))
