@@ -77,7 +77,7 @@ def draw(rng):
     kind = rng.choice(["static", "small", "lj", "lj", "metal", "metal", "ensemble", "integrator", "forces"])
     if kind == "static":
         k = k_between(3, 8)
-        return dict(do="static", k=k, drop=drop_of(k))
+        return dict(do="static", k=k, drop=rng.randrange(1, k**3))
     precision = rng.choice(["fp64", "mixed"])
     if kind == "small":
         k = k_between(5, 8)
