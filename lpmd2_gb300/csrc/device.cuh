@@ -22,7 +22,7 @@ namespace gbmd {
 
 constexpr int TILE = 128;          // atoms per tile = threads per block of the per-atom kernels
 constexpr int THERMO_LEN = 22;
-constexpr int PART_D = 16;         // FP64 per-tile partial sums
+constexpr int PART_D = 16;         // partial sums of a block of the FP64 passes
 constexpr int CODE_SHIFT = 25;
 constexpr unsigned LOCAL_MASK = (1u << CODE_SHIFT) - 1u;
 constexpr int MAX_SYSTEM_ATOMS = (1 << CODE_SHIFT);
@@ -50,7 +50,7 @@ constexpr int ERR_WAIT = 16;       // a bounded wait on an asynchronous copy gav
 constexpr int RING = GBMD_RING;
 static_assert((RING & (RING - 1)) == 0 && RING >= 2, "the list ring needs a power-of-two stage count");
 
-// Per-tile partial-sum slots (FP64)
+// Partial-sum slots of a block of the FP64 passes
 enum { PD_EPAIR = 0, PD_EEMBED = 1, PD_VIR = 2, PD_STRESS = 3, PD_KE = 12, PD_PX = 13 };
 // Per-system int64 fixed-point accumulators of the mixed path (atomics from every block)
 enum { SA_EPAIR = 0, SA_VIR = 1, SA_STRESS = 2, SA_KE = 11, SA_P = 12, SA_EEMBED = 15, SA_LEN = 16 };
@@ -105,6 +105,13 @@ struct SysState {
   unsigned long long rechecks;
 };
 
+// One block of the FP64 passes: `count` atoms from `first`, `lanes` lanes an atom, `apw` atoms a
+// warp (a multiple of 32 / lanes).
+struct Blk64 {
+  int sys, first, count;
+  short lanes, apw;
+};
+
 struct Dev {
   long long N;
   // positions are double-buffered: (x, y, z, g32, g64) are the positions a launch evaluates
@@ -156,7 +163,9 @@ struct Dev {
   // passes that read them from global memory instead of shared memory (GBMD_SHIFTS_GLOBAL)
   float4* shift_tab;
   // reductions
-  double* tile_d;
+  const Blk64* blk64;  // blocks of the FP64 passes
+  const int2* sys64;   // per system: its first block and how many
+  double* part64;      // PART_D partial sums per block
   unsigned long long* sys_acc;  // nsys * SA_LEN
   const SysDev* sysd;
   SysState* sst;

@@ -358,6 +358,7 @@ struct Engine::Impl {
   int *d_tile_sys = nullptr, *d_tile_first = nullptr, *d_tile_count = nullptr;
   std::vector<std::pair<void*, size_t>> allocs;       // set-up pool: (pointer, bytes)
   std::vector<std::pair<void*, size_t>> cell_allocs;  // grid pool (cells, then the list last)
+  std::vector<std::pair<void*, size_t>> scratch;      // workspaces a checkpoint does not hold
   size_t bytes = 0, cell_bytes = 0;
   bool configured = false, forces_valid = false, initialized = false, flags_any = false;
   Stats st;
@@ -464,6 +465,70 @@ struct Engine::Impl {
     (cellpool ? cell_bytes : bytes) += b;
     return (T*)p;
   }
+
+  // Workspaces outside the two pools that a checkpoint holds (so that snapshots keep their layout).
+  template <class T>
+  T* alloc_scratch(size_t n) {
+    T* p = alloc<T>(n);
+    scratch.push_back(allocs.back());
+    allocs.pop_back();
+    return p;
+  }
+  void free_scratch() {
+    for (auto& a : scratch) {
+      dev_free(a.first);
+      bytes -= a.second;
+    }
+    scratch.clear();
+  }
+
+  // How the FP64 passes cut a system (by its size and neighbour mode alone, so that its sums have the
+  // same order in a batch and by itself).  List mode: 8 lanes an atom; fewer atoms a warp while the
+  // system is small, so that there are several blocks for every SM.  Below 2,400 atoms, and where
+  // every candidate is tested (stencils, all pairs), a whole warp works on an atom.
+  static void plan64(int natoms, int mode, int& lanes, int& apw) {
+    if (mode != NB_LIST || natoms < 2400) {
+      lanes = 32;
+      apw = natoms < 4096 ? 1 : natoms < 32768 ? 4 : 16;
+    } else {
+      lanes = 8;
+      apw = natoms < 65536 ? 4 : natoms < 262144 ? 8 : 16;
+    }
+  }
+
+  // Block table and partial sums of the FP64 passes.
+  void alloc_blocks64() {
+    std::vector<Blk64> blk;
+    std::vector<int2> per(nsys);
+    for (int s = 0; s < nsys; ++s) {
+      Blk64 b{};
+      int lanes = 0, apw = 0;
+      plan64(sysd[s].natoms, sysd[s].mode, lanes, apw);
+      b.sys = s;
+      b.lanes = (short)lanes;
+      b.apw = (short)apw;
+      const int apb = apw * (TILE / 32);
+      per[s].x = (int)blk.size();
+      for (long long k = 0; k < natoms[s]; k += apb) {
+        b.first = (int)(atom_base[s] + k);
+        b.count = (int)std::min<long long>(apb, natoms[s] - k);
+        blk.push_back(b);
+      }
+      per[s].y = (int)blk.size() - per[s].x;
+    }
+    nblk64 = (int)blk.size();
+    Blk64* db = alloc_scratch<Blk64>(blk.size());
+    int2* dp = alloc_scratch<int2>(per.size());
+    CK(cudaMemcpyAsync(db, blk.data(), sizeof(Blk64) * blk.size(), cudaMemcpyHostToDevice, stream));
+    CK(cudaMemcpyAsync(dp, per.data(), sizeof(int2) * per.size(), cudaMemcpyHostToDevice, stream));
+    CK(cudaStreamSynchronize(stream));
+    D.blk64 = db;
+    D.sys64 = dp;
+    // one partial record per tile is part of the set-up pool; finer cuts have their own
+    D.part64 = nblk64 == ntiles ? tile_part : alloc_scratch<double>((size_t)nblk64 * PART_D);
+  }
+  int nblk64 = 0;
+  double* tile_part = nullptr;
 
   void free_cells() {
     for (auto& a : cell_allocs) dev_free(a.first);
@@ -581,7 +646,7 @@ struct Engine::Impl {
     D.phif = alloc<float>(n);
     D.facc = alloc<long long>(3 * n);
     D.dacc = alloc<double>(3 * n);
-    D.tile_d = alloc<double>((size_t)ntiles * PART_D);
+    tile_part = alloc<double>((size_t)ntiles * PART_D);
     {
       int nsm = 0;
       CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, device));
@@ -669,6 +734,7 @@ struct Engine::Impl {
     }
     for (cudaEvent_t e : event_pool) cudaEventDestroy(e);
     for (auto& a : allocs) dev_free(a.first);
+    free_scratch();
     free_cells();
     if (stream) cudaStreamDestroy(stream);
     if (stream2) cudaStreamDestroy(stream2);
@@ -802,6 +868,8 @@ struct Engine::Impl {
         throw Error(1, "every system of a batch must use the same neighbour mode (box too small for a Verlet list?)");
     // cell arrays and neighbour list
     free_cells();
+    free_scratch();
+    if (precision == PREC_FP64) alloc_blocks64();
     alloc_cells(total_cells);
     int maxnb = 0;
     if (any_list) {
@@ -940,12 +1008,8 @@ struct Engine::Impl {
         else if (mixed)
           ring ? k_eam_density32<0, FEED_RING><<<ntiles, TILE, 0, s>>>(D, Pe)
                : k_eam_density32<0, FEED_REGS><<<ntiles, TILE, 0, s>>>(D, Pe);
-        else if (mode == NB_LIST)
-          k_eam_density<NB_LIST><<<ntiles, TILE, 0, s>>>(D, P, first);
-        else if (mode == NB_CELLS)
-          k_eam_density<NB_CELLS><<<ntiles, TILE, 0, s>>>(D, P, first);
         else
-          k_eam_density<NB_ALLPAIRS><<<ntiles, TILE, 0, s>>>(D, P, first);
+          launch_density64(s, P, mode, first);
         launched();
       }
       if (mixed) {
@@ -982,21 +1046,8 @@ struct Engine::Impl {
             ring ? k_force32<PC_EAM, 0, 0, 0, FEED_RING><<<ntiles, TILE, 0, s>>>(D, Pe, sp)
                  : k_force32<PC_EAM, 0, 0, 0, FEED_REGS><<<ntiles, TILE, 0, s>>>(D, Pe, sp);
         }
-      } else if (mode == NB_LIST) {
-        if (pair_kind(P.kind))
-          k_force64<NB_LIST, PC_PAIR><<<ntiles, TILE, 0, s>>>(D, P, sp);
-        else
-          k_force64<NB_LIST, PC_EAM><<<ntiles, TILE, 0, s>>>(D, P, sp);
-      } else if (mode == NB_CELLS) {
-        if (pair_kind(P.kind))
-          k_force64<NB_CELLS, PC_PAIR><<<ntiles, TILE, 0, s>>>(D, P, sp);
-        else
-          k_force64<NB_CELLS, PC_EAM><<<ntiles, TILE, 0, s>>>(D, P, sp);
-      } else {
-        if (pair_kind(P.kind))
-          k_force64<NB_ALLPAIRS, PC_PAIR><<<ntiles, TILE, 0, s>>>(D, P, sp);
-        else
-          k_force64<NB_ALLPAIRS, PC_EAM><<<ntiles, TILE, 0, s>>>(D, P, sp);
+      } else if (nblk64 > 0) {
+        launch_force64(s, P, sp, mode);
       }
       launched();
     }
@@ -1005,8 +1056,48 @@ struct Engine::Impl {
       k_tail<<<nblocks(nsys, TAIL_THREADS), TAIL_THREADS, 0, s>>>(D, count_step, decide_next,
                                                                   (unsigned long long)cond_next);
     else
-      k_thermo<<<nsys, TILE, 0, s>>>(D, count_step);
+      k_thermo<<<nsys, PART_D * THERMO_ROWS, 0, s>>>(D, count_step);
     launched();
+  }
+
+  void launch_density64(cudaStream_t s, const PotParams& P, int mode, int first) {
+    if (nblk64 == 0) return;
+    const Pair64 c = pair64_constants(P);
+    if (P.kind == POT_SC && P.int_m == 6) {
+      if (mode == NB_LIST)
+        k_eam_density<NB_LIST, 6><<<nblk64, TILE, 0, s>>>(D, P, c, first);
+      else if (mode == NB_CELLS)
+        k_eam_density<NB_CELLS, 6><<<nblk64, TILE, 0, s>>>(D, P, c, first);
+      else
+        k_eam_density<NB_ALLPAIRS, 6><<<nblk64, TILE, 0, s>>>(D, P, c, first);
+    } else if (mode == NB_LIST) {
+      k_eam_density<NB_LIST, 0><<<nblk64, TILE, 0, s>>>(D, P, c, first);
+    } else if (mode == NB_CELLS) {
+      k_eam_density<NB_CELLS, 0><<<nblk64, TILE, 0, s>>>(D, P, c, first);
+    } else {
+      k_eam_density<NB_ALLPAIRS, 0><<<nblk64, TILE, 0, s>>>(D, P, c, first);
+    }
+  }
+
+  template <int PC, int SCN>
+  void launch_force64_mode(cudaStream_t s, const PotParams& P, const StepParams& sp, int mode) {
+    const Pair64 c = pair64_constants(P);
+    if (mode == NB_LIST)
+      k_force64<NB_LIST, PC, SCN><<<nblk64, TILE, 0, s>>>(D, P, c, sp);
+    else if (mode == NB_CELLS)
+      k_force64<NB_CELLS, PC, SCN><<<nblk64, TILE, 0, s>>>(D, P, c, sp);
+    else
+      k_force64<NB_ALLPAIRS, PC, SCN><<<nblk64, TILE, 0, s>>>(D, P, c, sp);
+  }
+  void launch_force64(cudaStream_t s, const PotParams& P, const StepParams& sp, int mode) {
+    if (pair_kind(P.kind))
+      launch_force64_mode<PC_PAIR, 0>(s, P, sp, mode);
+    else if (P.kind == POT_SC && P.int_m == 6 && P.int_n == 9)
+      launch_force64_mode<PC_EAM, 9>(s, P, sp, mode);
+    else if (P.kind == POT_SC && P.int_m == 6 && P.int_n == 12)
+      launch_force64_mode<PC_EAM, 12>(s, P, sp, mode);
+    else
+      launch_force64_mode<PC_EAM, 0>(s, P, sp, mode);
   }
 
   void ensure_ready() {
@@ -1338,8 +1429,8 @@ struct Engine::Impl {
       k_tail<<<nblocks(nsys, TAIL_THREADS), TAIL_THREADS, 0, stream>>>(D, 1, 0, 0ull);
       launched(3);
     } else {
-      k_step_kinetic<0><<<ntiles, TILE, 0, stream>>>(D);
-      k_thermo<<<nsys, TILE, 0, stream>>>(D, 1);
+      k_step_kinetic<0><<<nblk64, TILE, 0, stream>>>(D);
+      k_thermo<<<nsys, PART_D * THERMO_ROWS, 0, stream>>>(D, 1);
       launched(2);
     }
     check_launch("step");

@@ -143,111 +143,6 @@ __device__ __forceinline__ void warp_kinetic_fix(double ke, double px, double py
   for (int k = 0; k < 4; ++k) k4[k] = lead ? __double2ll_rn(s[k] * FIX_KE) : 0ll;
 }
 
-// Writes the tile's FP64 partials (slots [lo, hi) of the 16) with overwrite or accumulate.
-__device__ __forceinline__ void store_tile_d(const Dev& D, int tile, const double* v, int lo, int hi, bool first) {
-  double* t = D.tile_d + (long long)tile * PART_D;
-  for (int k = lo; k < hi; ++k) t[k] = first ? v[k] : t[k] + v[k];
-}
-
-// ------------------------------------------------------------------------------------------
-// FP64 force pass: pair (LJ) or EAM force.
-// ------------------------------------------------------------------------------------------
-
-template <int NB, int PC>
-__global__ void __launch_bounds__(TILE) k_force64(Dev D, PotParams P, StepParams sp) {
-  const int tile = blockIdx.x;
-  const int s = D.tile_sys[tile];
-  const SysDev& S = D.sysd[s];
-  if (!S.active) {  // whole block: one tile belongs to one system
-    if (sp.epi == EPI_KICK_DRIFT && sp.last) hold_tile(D, S, tile, true);
-    return;
-  }
-  const long long i = D.tile_first[tile] + threadIdx.x;
-  const bool active = (int)threadIdx.x < D.tile_count[tile];
-  double fx = 0.0, fy = 0.0, fz = 0.0, ep = 0.0, vir = 0.0;
-  double sxx = 0.0, sxy = 0.0, sxz = 0.0, syy = 0.0, syz = 0.0, szz = 0.0;
-  if (active) {
-    const double4_32a pi = D.g64[i];
-    const int ti = (int)pi.w;
-    const double phi_i = (PC == PC_EAM) ? D.phi[i] : 0.0;
-    for_each_candidate<NB>(D, S, i, [&](long long j, unsigned) {
-      const double4_32a pj = D.g64[j];
-      double dx = ref_wrap(dsub(pj.x, pi.x), S.L[0], S.Lh[0]);
-      double dy = ref_wrap(dsub(pj.y, pi.y), S.L[1], S.Lh[1]);
-      double dz = ref_wrap(dsub(pj.z, pi.z), S.L[2], S.Lh[2]);
-      double r2 = ref_sq(dx, dy, dz);
-      if (r2 < P.rc2 && applies_to(P.spc_sum, ti, (int)pj.w)) {
-        double g, e;
-        if (PC == PC_PAIR) {
-          if (P.kind == POT_FASTLJ)
-            fastlj_pair64(P, r2, g, e);
-          else
-            lj_pair64(P, r2, g, e);
-        } else {
-          double r = sqrt(r2);
-          double sc;
-          eam_pair64(P, r, phi_i, D.phi[j], sc, e);
-          g = ddiv(sc, r);
-        }
-        fx += g * dx;
-        fy += g * dy;
-        fz += g * dz;
-        ep += e;
-        vir -= g * r2;
-        sxx -= g * dx * dx;
-        sxy -= g * dx * dy;
-        sxz -= g * dx * dz;
-        syy -= g * dy * dy;
-        syz -= g * dy * dz;
-        szz -= g * dz * dz;
-      }
-    });
-  }
-  double ke = 0.0, px = 0.0, py = 0.0, pz = 0.0;
-  float d2 = 0.0f;
-  if (active) {
-    long long N = D.N;
-    if (!sp.first) {
-      fx += D.dacc[i];
-      fy += D.dacc[N + i];
-      fz += D.dacc[2 * N + i];
-    }
-    if (sp.last) {
-      d2 = finish_atom<0>(D, S, i, fx, fy, fz, sp, ke, px, py, pz);
-    } else {
-      D.dacc[i] = fx;
-      D.dacc[N + i] = fy;
-      D.dacc[2 * N + i] = fz;
-    }
-  }
-  track_displacement_warp(D, s, d2);
-  // the full list counts each pair twice: halve energy, virial and stress
-  double v[13] = {0.5 * ep, 0.5 * vir, 0.5 * sxx, 0.5 * sxy, 0.5 * sxz, 0.5 * sxy, 0.5 * syy,
-                  0.5 * syz, 0.5 * sxz, 0.5 * syz, 0.5 * szz, ke, 0.0};
-  double tot[13];
-  block_sum<double, 13>(v, tot);
-  if (threadIdx.x == 0) {
-    double out[PART_D] = {0};
-    out[PD_EPAIR] = tot[0];
-    out[PD_VIR] = tot[1];
-    for (int k = 0; k < 9; ++k) out[PD_STRESS + k] = tot[2 + k];
-    store_tile_d(D, tile, out, PD_EPAIR, PD_EPAIR + 1, sp.first);
-    store_tile_d(D, tile, out, PD_VIR, PD_STRESS + 9, sp.first);
-  }
-  if (sp.last) {
-    double k4[4] = {ke, px, py, pz};
-    double kt[4];
-    block_sum<double, 4>(k4, kt);
-    if (threadIdx.x == 0) {
-      double* t = D.tile_d + (long long)tile * PART_D;
-      t[PD_KE] = kt[0];
-      t[PD_PX] = kt[1];
-      t[PD_PX + 1] = kt[2];
-      t[PD_PX + 2] = kt[3];
-    }
-  }
-}
-
 // ------------------------------------------------------------------------------------------
 // Mixed force pass: FP32 pair maths, int64 fixed-point force sums, FP64 cutoff test inside a
 // guard band around rc^2 so the set of interacting pairs is the FP64 reference's.
@@ -1156,60 +1051,30 @@ __global__ void GBMD_DENSITY_BOUNDS k_eam_density32(Dev D, PotParams P) {
   release_tile(D);
 }
 
-// FP64 density pass (the plain path, any neighbour mode): reference r and rhoij, FP64
-// embedding, per-tile FP64 partial of the embedding energy.
-template <int NB>
-__global__ void __launch_bounds__(TILE) k_eam_density(Dev D, PotParams P, int first) {
-  const int tile = blockIdx.x;
-  const int s = D.tile_sys[tile];
-  const SysDev& S = D.sysd[s];
-  if (!S.active) return;  // whole block: one tile belongs to one system
-  const long long i = D.tile_first[tile] + threadIdx.x;
-  const bool active = (int)threadIdx.x < D.tile_count[tile];
-  double F = 0.0;
-  if (active) {
-    double rho = 0.0;
-    const double4_32a pi = D.g64[i];
-    for_each_candidate<NB>(D, S, i, [&](long long j, unsigned) {
-      const double4_32a pj = D.g64[j];
-      double dx = ref_wrap(dsub(pj.x, pi.x), S.L[0], S.Lh[0]);
-      double dy = ref_wrap(dsub(pj.y, pi.y), S.L[1], S.Lh[1]);
-      double dz = ref_wrap(dsub(pj.z, pi.z), S.L[2], S.Lh[2]);
-      double r2 = ref_sq(dx, dy, dz);
-      if (r2 < P.rc2) rho += eam_rho64(P, sqrt(r2));
-    });
-    double phi;
-    eam_embed64(P, rho, F, phi);
-    D.rho[i] = rho;
-    D.phi[i] = phi;
-    D.phif[i] = (float)phi;
-  }
-  double v[1] = {F};
-  double t[1];
-  block_sum<double, 1>(v, t);
-  if (threadIdx.x == 0) {
-    double* td = D.tile_d + (long long)tile * PART_D;
-    td[PD_EEMBED] = first ? t[0] : td[PD_EEMBED] + t[0];
-  }
-}
-
 // ------------------------------------------------------------------------------------------
-// Thermo record per system of the FP64 path (one block per system; fixed-order tile sums).
+// Thermo record per system of the FP64 path: one block per system sums the partial records of the
+// system's blocks in a fixed order, a slot per thread (coalesced rows of 16 doubles; a thread per
+// row and all slots took 18 us for 844 rows, this 4).
 // ------------------------------------------------------------------------------------------
 
-__global__ void __launch_bounds__(TILE) k_thermo(Dev D, int count_step) {
+constexpr int THERMO_ROWS = 32;
+__global__ void __launch_bounds__(PART_D * THERMO_ROWS) k_thermo(Dev D, int count_step) {
+  __shared__ double sh[THERMO_ROWS][PART_D];
   const int s = blockIdx.x;
-  const SysDev& S = D.sysd[s];
-  if (!S.active) return;
-  double v[PART_D];
-  for (int k = 0; k < PART_D; ++k) v[k] = 0.0;
-  for (int t = threadIdx.x; t < S.ntiles; t += blockDim.x) {
-    const double* td = D.tile_d + (long long)(S.tile_base + t) * PART_D;
-    for (int k = 0; k < PART_D; ++k) v[k] += td[k];
+  if (!D.sysd[s].active) return;
+  const int k = threadIdx.x % PART_D, row = threadIdx.x / PART_D;
+  const int n = D.sys64[s].y;
+  const double* t = D.part64 + (long long)D.sys64[s].x * PART_D + k;
+  double v = 0.0;
+#pragma unroll 4
+  for (int r = row; r < n; r += THERMO_ROWS) v += t[(long long)r * PART_D];
+  sh[row][k] = v;
+  __syncthreads();
+  for (int h = THERMO_ROWS / 2; h > 0; h >>= 1) {
+    if (row < h) sh[row][k] += sh[row + h][k];
+    __syncthreads();
   }
-  double tot[PART_D];
-  block_sum<double, PART_D>(v, tot);
-  if (threadIdx.x == 0) thermo_record(D, s, tot, count_step);
+  if (threadIdx.x == 0) thermo_record(D, s, sh[0], count_step);
 }
 
 }  // namespace gbmd

@@ -17,7 +17,7 @@
 // mixed path differs only in its forces).
 #pragma once
 
-#include "forces.cuh"
+#include "force64.cuh"
 
 namespace gbmd {
 
@@ -254,12 +254,22 @@ __global__ void k_kinetic_slots_clear(Dev D) {
 
 template <int MIXED>
 __global__ void __launch_bounds__(TILE) k_step_kinetic(Dev D) {
-  const int tile = blockIdx.x;
-  const int s = D.tile_sys[tile];
+  int s, first, count;
+  if (MIXED) {
+    const int tile = blockIdx.x;
+    s = D.tile_sys[tile];
+    first = D.tile_first[tile];
+    count = D.tile_count[tile];
+  } else {
+    const Blk64 B = D.blk64[blockIdx.x];
+    s = B.sys;
+    first = B.first;
+    count = B.count;
+  }
   if (!D.sysd[s].active) return;
-  const long long i = D.tile_first[tile] + threadIdx.x;
+  const long long i = first + threadIdx.x;
   double ke = 0.0, px = 0.0, py = 0.0, pz = 0.0;
-  if ((int)threadIdx.x < D.tile_count[tile]) {
+  if ((int)threadIdx.x < count) {
     const unsigned char fl = D.has_flags ? D.flags[i] : 0;
     if (!(fl & (FLAG_FIXEDVEL | FLAG_FIXEDPOS))) {
       const double m = D.mass[i], vx = D.vx[i], vy = D.vy[i], vz = D.vz[i];
@@ -285,7 +295,7 @@ __global__ void __launch_bounds__(TILE) k_step_kinetic(Dev D) {
     double kt[4];
     block_sum<double, 4>(k4, kt);
     if (threadIdx.x == 0) {
-      double* t = D.tile_d + (long long)tile * PART_D;
+      double* t = D.part64 + (long long)blockIdx.x * PART_D;
       t[PD_KE] = kt[0];
       for (int k = 0; k < 3; ++k) t[PD_PX + k] = kt[1 + k];
     }

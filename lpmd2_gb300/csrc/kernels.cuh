@@ -681,9 +681,9 @@ __device__ __forceinline__ float drift_atom(const Dev& D, const SysDev& S, long 
 // the committed one (xo), after which the buffers swap roles: copy xo -> x (to_read = true).
 // A stand-alone drift reads the committed buffer (x) and writes the pending one (xo): copy
 // x -> xo (to_read = false).
-__device__ __forceinline__ void hold_tile(const Dev& D, const SysDev& S, int tile, bool to_read) {
-  if ((int)threadIdx.x >= D.tile_count[tile]) return;
-  const long long i = D.tile_first[tile] + threadIdx.x;
+__device__ __forceinline__ void hold_range(const Dev& D, const SysDev& S, int first, int count, bool to_read) {
+  if ((int)threadIdx.x >= count) return;
+  const long long i = first + threadIdx.x;
   if (to_read) {
     D.x[i] = D.xo[i];
     D.y[i] = D.yo[i];
@@ -697,6 +697,9 @@ __device__ __forceinline__ void hold_tile(const Dev& D, const SysDev& S, int til
     D.g64o[i] = D.g64[i];
     if (S.mode == NB_LIST) D.g32o[i] = D.g32[i];
   }
+}
+__device__ __forceinline__ void hold_tile(const Dev& D, const SysDev& S, int tile, bool to_read) {
+  hold_range(D, S, D.tile_first[tile], D.tile_count[tile], to_read);
 }
 
 // Stand-alone drift (the first step of a run, before any fused force/drift launch).

@@ -18,16 +18,6 @@ __device__ __forceinline__ bool applies_to(int spc_sum, int s1, int s2) {
   return (spc_sum < 0) || ((s1 + s2) == spc_sum);  // liblpmd/simulation/potential.cc:25-27
 }
 
-__device__ __forceinline__ double ipow_d(double x, int n) {
-  double r = 1.0, b = x;
-  while (n > 0) {
-    if (n & 1) r = dmul(r, b);
-    b = dmul(b, b);
-    n >>= 1;
-  }
-  return r;
-}
-
 __device__ __forceinline__ float ipow_f(float x, int n) {
   float r = 1.0f, b = x;
   while (n > 0) {
@@ -64,33 +54,6 @@ __device__ __forceinline__ void fastlj_pair64(const PotParams& P, double r2, dou
   g = P.tab[bins + k];
 }
 
-// rhoij(r) for the EAM density pass.
-__device__ __forceinline__ double eam_rho64(const PotParams& P, double r) {
-  if (P.kind == POT_GUPTA) {  // plugins/gupta.cc:56: exp(-2 q (r - r0) / r0)
-    const double r0 = P.p[1], q = P.p[4];
-    return exp(ddiv(dmul(dmul(-2.0, q), dsub(r, r0)), r0));
-  }
-  if (P.kind == POT_SC) {
-    double ir = ddiv(1.0, r);
-    double pw = (P.int_m >= 0) ? ipow_d(ir, P.int_m) : pow(ir, P.p[3]);
-    return dmul(P.am, pw);
-  } else if (P.kind == POT_FS) {
-    const double B = P.p[4], d = P.p[6];
-    if (r <= d) {
-      double rd = dsub(r, d);
-      return dmul(dmul(rd, rd), dadd(1.0, ddiv(dmul(B, rd), d)));
-    }
-    return 0.0;
-  } else {
-    const double B = P.p[6], d = P.p[8];
-    if (r <= d) {
-      double rd = dsub(r, d);
-      return dmul(dmul(rd, rd), dadd(1.0, dmul(dmul(dmul(B, B), rd), rd)));
-    }
-    return 0.0;
-  }
-}
-
 // Embedding F(rho) and 1/sqrt(rho) (the per-atom factor of ManyBodies).
 __device__ __forceinline__ void eam_embed64(const PotParams& P, double rho, double& F, double& phi) {
   double sq = sqrt(rho);
@@ -101,74 +64,6 @@ __device__ __forceinline__ void eam_embed64(const PotParams& P, double rho, doub
   else
     F = dmul(-P.p[5], sq);
   phi = ddiv(1.0, sq);
-}
-
-// Pair energy V(r) and the scalar s with PairForce + ManyBodies = s * r^ (r^ = r_ij / r).
-__device__ __forceinline__ void eam_pair64(const PotParams& P, double r, double phi_i, double phi_j,
-                                           double& s, double& e) {
-  if (P.kind == POT_GUPTA) {
-    // plugins/gupta.cc:54,60-70: V = A exp(-p (r - r0) / r0), PairForce = -(A p / r0) exp(..),
-    // ManyBodies = (B q / r0) (1/sqrt(rho_i) + 1/sqrt(rho_j)) exp(-2 q (r - r0) / r0)
-    const double A = P.p[0], r0 = P.p[1], pp = P.p[2], B = P.p[3], q = P.p[4];
-    const double dr = dsub(r, r0);
-    const double ex = exp(ddiv(dmul(-pp, dr), r0));
-    e = dmul(A, ex);
-    const double pf = dmul(-ddiv(dmul(A, pp), r0), ex);
-    const double mb = dmul(dmul(ddiv(dmul(B, q), r0), dadd(phi_i, phi_j)), exp(ddiv(dmul(dmul(-2.0, q), dr), r0)));
-    s = dadd(pf, mb);
-  } else if (P.kind == POT_SC) {
-    const double eps = P.p[0], n = P.p[2], m = P.p[3], c = P.p[4];
-    double ir = ddiv(1.0, r);
-    double irn = (P.int_n >= 0) ? ipow_d(ir, P.int_n) : pow(ir, n);
-    double irm1 = (P.int_m >= 0) ? ipow_d(ir, P.int_m + 1) : pow(ir, m + 1);
-    e = dmul(dmul(eps, P.an), irn);
-    double pf = dmul(dmul(dmul(-n, eps), P.an), dmul(irn, ir));
-    double mb = dmul(dmul(dmul(dmul(dmul(dmul(0.5, m), c), eps), dadd(phi_i, phi_j)), P.am), irm1);
-    s = dadd(pf, mb);
-  } else if (P.kind == POT_FS) {
-    const double c0 = P.p[0], c1 = P.p[1], c2 = P.p[2], A = P.p[3], B = P.p[4], c = P.p[5], d = P.p[6];
-    double pf = 0.0, mb = 0.0;
-    e = 0.0;
-    if (r <= c) {
-      double rc = dsub(r, c);
-      double poly = dadd(dadd(c0, dmul(c1, r)), dmul(dmul(c2, r), r));
-      e = dmul(dmul(rc, rc), poly);
-      double t1 = dmul(dmul(2.0, rc), poly);
-      double t2 = dmul(dmul(rc, rc), dadd(c1, dmul(dmul(2.0, c2), r)));
-      pf = dadd(t1, t2);
-    }
-    if (r <= d) {
-      double rd = dsub(r, d);
-      double t1 = ddiv(dmul(dadd(phi_i, phi_j), A), 2.0);
-      double t2 = dadd(dmul(2.0, rd), ddiv(dmul(dmul(dmul(3.0, B), rd), rd), d));
-      mb = dmul(-t1, t2);
-    }
-    s = dadd(pf, mb);
-  } else {
-    const double c0 = P.p[0], c1 = P.p[1], c2 = P.p[2], c3 = P.p[3], c4 = P.p[4];
-    const double A = P.p[5], B = P.p[6], c = P.p[7], d = P.p[8];
-    double pf = 0.0, mb = 0.0;
-    e = 0.0;
-    if (r <= c) {
-      double r2 = dmul(r, r);
-      double rc = dsub(r, c);
-      double poly = dadd(dadd(dadd(dadd(c0, dmul(c1, r)), dmul(c2, r2)), dmul(dmul(c3, r2), r)),
-                         dmul(dmul(c4, r2), r2));
-      e = dmul(dmul(rc, rc), poly);
-      double t1 = dmul(dmul(2.0, rc), poly);
-      double dp = dadd(dadd(dadd(c1, dmul(dmul(2.0, c2), r)), dmul(dmul(3.0, c3), r2)),
-                       dmul(dmul(dmul(4.0, c4), r2), r));
-      double t2 = dmul(dmul(dp, rc), rc);
-      pf = dadd(t1, t2);
-    }
-    if (r <= d) {
-      double rd = dsub(r, d);
-      double t1 = dmul(dmul(A, 0.5), dadd(phi_i, phi_j));
-      double t2 = dadd(dmul(2.0, rd), dmul(dmul(dmul(dmul(dmul(4.0, B), B), rd), rd), rd));
-      mb = dmul(-t1, t2);
-    }
-    s = dadd(pf, mb);
-  }
 }
 
 // ------------------------------------------------------------------------------------------
