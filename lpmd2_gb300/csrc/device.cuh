@@ -166,6 +166,8 @@ struct Dev {
   const Blk64* blk64;  // blocks of the FP64 passes
   const int2* sys64;   // per system: its first block and how many
   double* part64;      // PART_D partial sums per block
+  double* share64;     // the same per share of a system's blocks, and how many shares are done
+  unsigned* ticket64;  // (zero between launches)
   unsigned long long* sys_acc;  // nsys * SA_LEN
   const SysDev* sysd;
   SysState* sst;

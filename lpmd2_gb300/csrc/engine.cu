@@ -526,8 +526,12 @@ struct Engine::Impl {
     D.sys64 = dp;
     // one partial record per tile is part of the set-up pool; finer cuts have their own
     D.part64 = nblk64 == ntiles ? tile_part : alloc_scratch<double>((size_t)nblk64 * PART_D);
+    shares64 = 1;
+    for (const int2& x : per) shares64 = std::max(shares64, thermo_shares(x.y));
+    D.share64 = alloc_scratch<double>((size_t)nsys * shares64 * PART_D);
+    D.ticket64 = alloc_scratch<unsigned>(nsys);  // zeroed
   }
-  int nblk64 = 0;
+  int nblk64 = 0, shares64 = 1;
   double* tile_part = nullptr;
 
   void free_cells() {
@@ -934,8 +938,8 @@ struct Engine::Impl {
   // --------------------------------------------------------------------------------------
 
   void launch_decide(cudaStream_t s, int ucall_inc, int force_all, cudaGraphConditionalHandle h, int use_cond) {
-    k_decide<<<nblocks(nsys, DECIDE_THREADS), DECIDE_THREADS, 0, s>>>(D, nsys, ucall_inc, force_all,
-                                                                      (unsigned long long)h, use_cond);
+    k_decide<<<nblocks(nsys, SYS_WARPS), 32 * SYS_WARPS, 0, s>>>(D, nsys, ucall_inc, force_all, (unsigned long long)h,
+                                                                 use_cond);
     launched();
   }
 
@@ -962,8 +966,8 @@ struct Engine::Impl {
     mark_end(s, T_REBUILD);
   }
 
-  // decide_next / cond_next: the mixed path's tail kernel also decides the next step's rebuild
-  // and sets that step's graph conditional (0: a k_decide launch does it instead).
+  // decide_next / cond_next: the tail kernel also decides the next step's rebuild and sets that
+  // step's graph conditional (0: a k_decide launch does it instead).
   // raw: keep fixedvel atoms' accelerations (a bare UpdateForces outside an integrator step).
   void launch_force_passes(cudaStream_t s, int epi, int count_step, int decide_next = 0,
                            cudaGraphConditionalHandle cond_next = 0, int raw = 0) {
@@ -1053,10 +1057,10 @@ struct Engine::Impl {
     }
     mark_end(s, T_FORCE);
     if (mixed)
-      k_tail<<<nblocks(nsys, TAIL_THREADS), TAIL_THREADS, 0, s>>>(D, count_step, decide_next,
-                                                                  (unsigned long long)cond_next);
+      k_tail<<<nblocks(nsys, SYS_WARPS), 32 * SYS_WARPS, 0, s>>>(D, count_step, decide_next,
+                                                                 (unsigned long long)cond_next);
     else
-      k_thermo<<<nsys, PART_D * THERMO_ROWS, 0, s>>>(D, count_step);
+      k_thermo<<<dim3(nsys, shares64), PART_D * THERMO_ROWS, 0, s>>>(D, count_step, decide_next, (unsigned long long)cond_next);
     launched();
   }
 
@@ -1253,15 +1257,14 @@ struct Engine::Impl {
     int64_t saved = st.kernel_launches;
     const int cbuf0 = cbuf;
     capturing = true;
-    // mixed path: the tail kernel of step k decides step k+1, so only the first step of the
-    // graph launches k_decide
-    const bool fused = precision == PREC_MIXED;
+    // the tail kernel of step k decides step k+1, so only the first step of the graph launches
+    // k_decide
     int64_t base_launches = 0;
     try {
       for (int k = 0; k < nsteps; ++k) {
         set_buffers(1 - cbuf);
         int64_t before = st.kernel_launches;
-        if (!(fused && k > 0)) launch_decide(stream, 2, 0, cond ? handles[k] : 0, cond ? 1 : 0);
+        if (k == 0) launch_decide(stream, 2, 0, cond ? handles[k] : 0, cond ? 1 : 0);
         if (!cond) launch_rebuild(stream);
         base_launches += st.kernel_launches - before;
         if (cond) {
@@ -1284,7 +1287,7 @@ struct Engine::Impl {
           cudaGraph_t bout;
           CK(cudaStreamEndCapture(stream2, &bout));
         }
-        const bool decide_next = fused && k + 1 < nsteps;
+        const bool decide_next = k + 1 < nsteps;
         before = st.kernel_launches;
         launch_step_tail(stream, decide_next ? 1 : 0, (decide_next && cond) ? handles[k + 1] : 0);
         base_launches += st.kernel_launches - before;
@@ -1426,11 +1429,11 @@ struct Engine::Impl {
     if (mixed) {
       k_kinetic_slots_clear<<<1, 256, 0, stream>>>(D);
       k_step_kinetic<1><<<ntiles, TILE, 0, stream>>>(D);
-      k_tail<<<nblocks(nsys, TAIL_THREADS), TAIL_THREADS, 0, stream>>>(D, 1, 0, 0ull);
+      k_tail<<<nblocks(nsys, SYS_WARPS), 32 * SYS_WARPS, 0, stream>>>(D, 1, 0, 0ull);
       launched(3);
     } else {
       k_step_kinetic<0><<<nblk64, TILE, 0, stream>>>(D);
-      k_thermo<<<nsys, PART_D * THERMO_ROWS, 0, stream>>>(D, 1);
+      k_thermo<<<dim3(nsys, shares64), PART_D * THERMO_ROWS, 0, stream>>>(D, 1, 0, 0ull);
       launched(2);
     }
     check_launch("step");

@@ -148,70 +148,63 @@ __device__ __forceinline__ void warp_kinetic_fix(double ke, double px, double py
 // guard band around rc^2 so the set of interacting pairs is the FP64 reference's.
 // ------------------------------------------------------------------------------------------
 
-// Thermo record of system s (one thread): SetSimulationTags' quantities from the FP64 tile
-// sums `tot` (FP64 path) or, with tot == nullptr, from the system's int64 accumulators.
-__device__ __forceinline__ void thermo_record(const Dev& D, int s, const double* tot_in, int count_step) {
+// Thermo record of system s (one warp, a lane per sum and per field): SetSimulationTags' quantities
+// from the FP64 sums `sums` (PD_* order; FP64 path) or, with sums == nullptr, from the system's int64
+// accumulators.
+__device__ __forceinline__ void thermo_record(const Dev& D, int s, const double* sums, int count_step) {
+  const unsigned all = 0xffffffffu;
   const SysDev& S = D.sysd[s];
   SysState& st = D.sst[s];
-  double tot[PART_D];
-  for (int k = 0; k < PART_D; ++k) tot[k] = tot_in ? tot_in[k] : 0.0;
-  double epair = tot[PD_EPAIR], vir = tot[PD_VIR];
-  double stress[9];
-  for (int k = 0; k < 9; ++k) stress[k] = tot[PD_STRESS + k];
-  if (!tot_in) {
-    const long long* acc = (const long long*)D.sys_acc + (long long)s * SA_LEN;
-    const double inv = 1.0 / FIX_E, invk = 1.0 / FIX_KE;
-    epair = (double)__ldcg(acc + SA_EPAIR) * inv;
-    vir = (double)__ldcg(acc + SA_VIR) * inv;
-    for (int k = 0; k < 9; ++k) stress[k] = (double)__ldcg(acc + SA_STRESS + k) * inv;
-    tot[PD_EEMBED] = (double)__ldcg(acc + SA_EEMBED) * inv;
-    tot[PD_KE] = (double)__ldcg(acc + SA_KE) * invk;
-    for (int k = 0; k < 3; ++k) tot[PD_PX + k] = (double)__ldcg(acc + SA_P + k) * invk;
+  const int lane = threadIdx.x & 31;
+  const long long step = st.step + (count_step ? 1 : 0);
+  double x = 0.0;
+  if (lane < PART_D) {
+    if (sums) {
+      x = sums[lane];
+    } else {
+      // the accumulators hold the same slots with the embedding energy last
+      const int slot = lane == PD_EEMBED ? (int)SA_EEMBED : lane == PD_EPAIR ? (int)SA_EPAIR : lane - 1;
+      x = (double)(long long)__ldcg(D.sys_acc + (long long)s * SA_LEN + slot) *
+          (lane >= PD_KE ? 1.0 / FIX_KE : 1.0 / FIX_E);
+    }
   }
-  if (count_step) st.step += 1;
+  const double epot = __shfl_sync(all, x, PD_EPAIR) + __shfl_sync(all, x, PD_EEMBED);
+  const double vir = __shfl_sync(all, x, PD_VIR);
   const double KIN2EV = 103.64269;  // liblpmd/lpmd/properties.h:10
-  double epot = epair + tot[PD_EEMBED];
-  double kin = dmul(tot[PD_KE], KIN2EV);
-  double temp = (S.natoms == 0) ? 0.0 : ddiv(dmul(2.0 / 3.0, kin), S.kbn);
+  const double kin = dmul(__shfl_sync(all, x, PD_KE), KIN2EV);
+  const double sum = __shfl_sync(all, x, lane >= 13 ? lane - 13 + PD_STRESS : PD_PX + ((lane - 6) & 3));
   const double vol = S.vol, pv = S.pv;  // volume and pressfactor/volume, computed on the host
-  double r[THERMO_LEN];
-  r[0] = (double)st.step;
-  r[1] = epot;
-  r[2] = kin;
-  r[3] = epot + kin;
-  r[4] = temp;
-  r[5] = vir;
-  r[6] = tot[PD_PX];
-  r[7] = tot[PD_PX + 1];
-  r[8] = tot[PD_PX + 2];
-  r[9] = vol;
-  r[10] = dmul(dmul(pv, 1.0 / 3.0), vir);
-  r[11] = dmul(dmul(pv, 2.0 / 3.0), kin);
-  r[12] = dmul(pv, dadd(dmul(2.0 / 3.0, kin), dmul(1.0 / 3.0, vir)));
-  for (int k = 0; k < 9; ++k) r[13 + k] = stress[k];
-  double* last = D.thermo_last + (long long)s * THERMO_LEN;
-  double* log = D.thermo_log + ((long long)s * D.log_cap + (st.step % D.log_cap)) * THERMO_LEN;
-  for (int k = 0; k < THERMO_LEN; ++k) {
-    last[k] = r[k];
-    if (count_step) log[k] = r[k];
+  double r = sum;                       // momentum (6..8) and stress (13..21)
+  if (lane == 0) r = (double)step;
+  if (lane == 1) r = epot;
+  if (lane == 2) r = kin;
+  if (lane == 3) r = epot + kin;
+  if (lane == 4) r = (S.natoms == 0) ? 0.0 : ddiv(dmul(2.0 / 3.0, kin), S.kbn);
+  if (lane == 5) r = vir;
+  if (lane == 9) r = vol;
+  if (lane == 10) r = dmul(dmul(pv, 1.0 / 3.0), vir);
+  if (lane == 11) r = dmul(dmul(pv, 2.0 / 3.0), kin);
+  if (lane == 12) r = dmul(pv, dadd(dmul(2.0 / 3.0, kin), dmul(1.0 / 3.0, vir)));
+  if (lane < THERMO_LEN) {
+    D.thermo_last[(long long)s * THERMO_LEN + lane] = r;
+    if (count_step) D.thermo_log[((long long)s * D.log_cap + (step % D.log_cap)) * THERMO_LEN + lane] = r;
   }
+  __syncwarp();
+  if (lane == 0 && count_step) st.step = step;
 }
 
-// Tail of a mixed force evaluation, one thread per system: the thermo records from the int64
+// Tail of a mixed force evaluation, one warp per system: the thermo records from the int64
 // accumulators and, inside a step sequence, the next step's rebuild decision and graph
 // conditional -- one launch instead of a k_thermo and a k_decide.  The conditional starts every
-// graph launch at 0 (cudaGraphCondAssignDefault), so a block raises it only when one of its
-// systems rebuilds and no block ever lowers it.
-constexpr int TAIL_THREADS = 128;
-__global__ void __launch_bounds__(TAIL_THREADS) k_tail(Dev D, int count_step, int decide_next,
-                                                       unsigned long long cond_next) {
-  const int s = blockIdx.x * TAIL_THREADS + threadIdx.x;
-  int need = 0;
-  if (s < D.nsys) {
-    if (D.sysd[s].active) thermo_record(D, s, nullptr, count_step);
-    if (decide_next) need = decide_system(D, s, 2, 0);
-  }
-  if (__syncthreads_or(need) && threadIdx.x == 0 && cond_next)
+// graph launch at 0 (cudaGraphCondAssignDefault), so a warp raises it only when its system
+// rebuilds and none ever lowers it.  (One thread per system wrote the 44 doubles of a record one
+// after the other: 4.6 us for one system, 12 us for 128; a warp 3.7 and 4.7 us.)
+__global__ void __launch_bounds__(32 * SYS_WARPS) k_tail(Dev D, int count_step, int decide_next,
+                                                         unsigned long long cond_next) {
+  const int s = blockIdx.x * SYS_WARPS + (threadIdx.x >> 5);
+  if (s >= D.nsys) return;
+  if (D.sysd[s].active) thermo_record(D, s, nullptr, count_step);
+  if (decide_next && decide_system(D, s, 2, 0) && cond_next && (threadIdx.x & 31) == 0)
     cudaGraphSetConditional((cudaGraphConditionalHandle)cond_next, 1u);
 }
 
@@ -1052,29 +1045,64 @@ __global__ void GBMD_DENSITY_BOUNDS k_eam_density32(Dev D, PotParams P) {
 }
 
 // ------------------------------------------------------------------------------------------
-// Thermo record per system of the FP64 path: one block per system sums the partial records of the
-// system's blocks in a fixed order, a slot per thread (coalesced rows of 16 doubles; a thread per
-// row and all slots took 18 us for 844 rows, this 4).
+// Tail of an FP64 force evaluation: sums the partial records of the system's blocks in a fixed
+// order, a slot per thread (coalesced rows of 16 doubles), writes the thermo record and, inside a
+// step sequence, decides the next step's rebuild (as k_tail does).  The sums are FP64 additions at 2
+// a clock and SM -- 14 us for the 3,400 rows of a 108k system on one SM -- so the rows of a large
+// system are shared by several blocks (about THERMO_SHARE each, by the system's own count) and the
+// last of them to finish adds their sums up.
 // ------------------------------------------------------------------------------------------
 
 constexpr int THERMO_ROWS = 32;
-__global__ void __launch_bounds__(PART_D * THERMO_ROWS) k_thermo(Dev D, int count_step) {
+constexpr int THERMO_SHARE = 128;
+__host__ __device__ inline int thermo_shares(int rows) {
+  if (rows <= 2 * THERMO_SHARE) return 1;
+  const int n = (rows + THERMO_SHARE - 1) / THERMO_SHARE;
+  return n < 64 ? n : 64;
+}
+__global__ void __launch_bounds__(PART_D * THERMO_ROWS) k_thermo(Dev D, int count_step, int decide_next,
+                                                                 unsigned long long cond_next) {
   __shared__ double sh[THERMO_ROWS][PART_D];
+  __shared__ int last;
   const int s = blockIdx.x;
-  if (!D.sysd[s].active) return;
-  const int k = threadIdx.x % PART_D, row = threadIdx.x / PART_D;
-  const int n = D.sys64[s].y;
-  const double* t = D.part64 + (long long)D.sys64[s].x * PART_D + k;
-  double v = 0.0;
+  const long long n = D.sys64[s].y;
+  const int parts = thermo_shares((int)n);
+  const bool active = D.sysd[s].active;
+  if ((int)blockIdx.y >= parts || (!active && blockIdx.y != 0)) return;
+  if (active) {
+    const int k = threadIdx.x % PART_D, row = threadIdx.x / PART_D;
+    auto sum_rows = [&](const double* t, int lo, int hi) {
+      double v = 0.0;
 #pragma unroll 4
-  for (int r = row; r < n; r += THERMO_ROWS) v += t[(long long)r * PART_D];
-  sh[row][k] = v;
-  __syncthreads();
-  for (int h = THERMO_ROWS / 2; h > 0; h >>= 1) {
-    if (row < h) sh[row][k] += sh[row + h][k];
-    __syncthreads();
+      for (int r = lo + row; r < hi; r += THERMO_ROWS) v += __ldcg(t + (long long)r * PART_D + k);
+      sh[row][k] = v;
+      __syncthreads();
+      for (int h = THERMO_ROWS / 2; h > 0; h >>= 1) {
+        if (row < h) sh[row][k] += sh[row + h][k];
+        __syncthreads();
+      }
+    };
+    sum_rows(D.part64 + (long long)D.sys64[s].x * PART_D, (int)(n * blockIdx.y / parts),
+             (int)(n * (blockIdx.y + 1) / parts));
+    if (parts > 1) {
+      double* mine = D.share64 + (long long)s * gridDim.y * PART_D;
+      if (row == 0) {
+        __stcg(mine + blockIdx.y * PART_D + k, sh[0][k]);
+        __threadfence();
+      }
+      __syncthreads();
+      if (threadIdx.x == 0) last = atomicAdd(D.ticket64 + s, 1u) == (unsigned)parts - 1u;
+      __syncthreads();
+      if (!last) return;
+      __threadfence();
+      sum_rows(mine, 0, parts);
+      if (threadIdx.x == 0) D.ticket64[s] = 0u;
+    }
   }
-  if (threadIdx.x == 0) thermo_record(D, s, sh[0], count_step);
+  if (threadIdx.x >= 32) return;
+  if (active) thermo_record(D, s, sh[0], count_step);
+  if (decide_next && decide_system(D, s, 2, 0) && cond_next && threadIdx.x == 0)
+    cudaGraphSetConditional((cudaGraphConditionalHandle)cond_next, 1u);
 }
 
 }  // namespace gbmd

@@ -46,46 +46,52 @@ struct StepParams {
 // ---------------------------------------------------------------------------------------------
 
 // ucall_inc: how many emulated UpdateCell calls this evaluation stands for (verletlist "each").
-// Rebuild decision of one system for the next force evaluation (one thread): clears the
-// system's fixed-point accumulators and returns whether its cells/list are rebuilt.
+// Rebuild decision of one system for the next force evaluation (one warp): clears the system's
+// fixed-point accumulators and returns whether its cells/list are rebuilt.
 __device__ __forceinline__ int decide_system(const Dev& D, int s, int ucall_inc, int force_all) {
   const SysDev& S = D.sysd[s];
   SysState& st = D.sst[s];
+  const int lane = threadIdx.x & 31;
   if (!S.active) {
-    st.need_rebuild = 0;
+    if (lane == 0) st.need_rebuild = 0;
     return 0;
   }
-  int need = force_all | st.force_rebuild;
-  if (S.mode == NB_CELLS) need = 1;
-  if (S.mode == NB_LIST) {
-    float md2 = __int_as_float((int)__ldcg(&st.maxdisp2));  // atomics of the previous launch
-    if ((S.rebuild_policy == REBUILD_SKIN || S.rebuild_policy == REBUILD_BOTH) && (double)md2 > S.thresh2)
-      need = 1;
-    if (S.rebuild_policy == REBUILD_EACH || S.rebuild_policy == REBUILD_BOTH) {
-      for (int k = 0; k < ucall_inc; ++k)
-        if (((st.ucalls + k) % S.each) == 0) need = 1;
+  if (lane < SA_LEN) D.sys_acc[(long long)s * SA_LEN + lane] = 0ull;
+  int need = 0;
+  if (lane == 0) {
+    need = force_all | st.force_rebuild;
+    const long long ucalls = st.ucalls;
+    if (S.mode == NB_CELLS) need = 1;
+    if (S.mode == NB_LIST) {
+      float md2 = __int_as_float((int)__ldcg(&st.maxdisp2));  // atomics of the previous launch
+      if ((S.rebuild_policy == REBUILD_SKIN || S.rebuild_policy == REBUILD_BOTH) && (double)md2 > S.thresh2)
+        need = 1;
+      if (S.rebuild_policy == REBUILD_EACH || S.rebuild_policy == REBUILD_BOTH) {
+        for (int k = 0; k < ucall_inc; ++k)
+          if (((ucalls + k) % S.each) == 0) need = 1;
+      }
+    }
+    st.ucalls = ucalls + ucall_inc;
+    if (S.mode == NB_ALLPAIRS) need = 0;
+    st.need_rebuild = need;
+    st.force_rebuild = 0;
+    if (need) {
+      st.maxdisp2 = 0u;
+      st.rebuilds += (S.mode == NB_LIST) ? 1 : 0;
     }
   }
-  st.ucalls += ucall_inc;
-  if (S.mode == NB_ALLPAIRS) need = 0;
-  for (int k = 0; k < SA_LEN; ++k) D.sys_acc[(long long)s * SA_LEN + k] = 0ull;
-  st.need_rebuild = need;
-  st.force_rebuild = 0;
-  if (need) {
-    st.maxdisp2 = 0u;
-    st.rebuilds += (S.mode == NB_LIST) ? 1 : 0;
-  }
-  return need;
+  return __shfl_sync(0xffffffffu, need, 0);
 }
 
-// One thread per system.  Inside a graph the conditional of the step starts at 0 at every graph
-// launch (cudaGraphCondAssignDefault): a block raises it when one of its systems rebuilds.
-constexpr int DECIDE_THREADS = 128;
-__global__ void __launch_bounds__(DECIDE_THREADS) k_decide(Dev D, int nsys, int ucall_inc, int force_all,
+// One warp per system.  Inside a graph the conditional of the step starts at 0 at every graph
+// launch (cudaGraphCondAssignDefault): a warp raises it when its system rebuilds.
+constexpr int SYS_WARPS = 4;  // systems per block of the per-system kernels
+__global__ void __launch_bounds__(32 * SYS_WARPS) k_decide(Dev D, int nsys, int ucall_inc, int force_all,
                                                            unsigned long long cond_handle, int use_cond) {
-  const int s = blockIdx.x * DECIDE_THREADS + threadIdx.x;
-  const int need = s < nsys ? decide_system(D, s, ucall_inc, force_all) : 0;
-  if (__syncthreads_or(need) && use_cond && threadIdx.x == 0)
+  const int s = blockIdx.x * SYS_WARPS + (threadIdx.x >> 5);
+  if (s >= nsys) return;
+  const int need = decide_system(D, s, ucall_inc, force_all);
+  if (need && use_cond && (threadIdx.x & 31) == 0)
     cudaGraphSetConditional((cudaGraphConditionalHandle)cond_handle, 1u);
 }
 
