@@ -134,9 +134,12 @@ struct Dev {
   int* cell_sys;     // system of each cell (flat cell index over every system)
   double* ccentre;   // cell centres (x, y, z per flat cell index) of Verlet-list grids
   int total_cells;
-  int* lblk_sys;     // list-build blocks: system and first flat cell of each block
-  int* lblk_cell;
-  int list_blocks;
+  // batches: the systems that rebuild before the next evaluation, in system order, with the running
+  // totals of their 256-atom chunks and of their cells (rb_n + 1 entries each)
+  int* rb_n;
+  int* rb_sys;
+  int* rb_chunk0;
+  int* rb_cell0;
   // permutation scratch
   double* sdbl;   // 11*N doubles
   // integrator history of the integrators other than velocityverlet (IST_K*N doubles, moved

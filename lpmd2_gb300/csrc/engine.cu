@@ -358,7 +358,7 @@ struct Engine::Impl {
   int *d_tile_sys = nullptr, *d_tile_first = nullptr, *d_tile_count = nullptr;
   std::vector<std::pair<void*, size_t>> allocs;       // set-up pool: (pointer, bytes)
   std::vector<std::pair<void*, size_t>> cell_allocs;  // grid pool (cells, then the list last)
-  std::vector<std::pair<void*, size_t>> scratch;      // workspaces a checkpoint does not hold
+  std::vector<std::pair<void*, size_t>> scratch, work;  // workspaces a checkpoint does not hold
   size_t bytes = 0, cell_bytes = 0;
   bool configured = false, forces_valid = false, initialized = false, flags_any = false;
   Stats st;
@@ -466,13 +466,22 @@ struct Engine::Impl {
     return (T*)p;
   }
 
-  // Workspaces outside the two pools that a checkpoint holds (so that snapshots keep their layout).
+  // Workspaces outside the two pools that a checkpoint holds (so that snapshots keep their layout):
+  // scratch is remade with the configuration, work stays for the engine's life.
   template <class T>
-  T* alloc_scratch(size_t n) {
+  T* alloc_aside(size_t n, std::vector<std::pair<void*, size_t>>& to) {
     T* p = alloc<T>(n);
-    scratch.push_back(allocs.back());
+    to.push_back(allocs.back());
     allocs.pop_back();
     return p;
+  }
+  template <class T>
+  T* alloc_scratch(size_t n) {
+    return alloc_aside<T>(n, scratch);
+  }
+  template <class T>
+  T* alloc_work(size_t n) {
+    return alloc_aside<T>(n, work);
   }
   void free_scratch() {
     for (auto& a : scratch) {
@@ -676,6 +685,12 @@ struct Engine::Impl {
     D.tile_sys = d_tile_sys;
     D.tile_first = d_tile_first;
     D.tile_count = d_tile_count;
+    if (nsys > 1) {
+      D.rb_n = alloc_work<int>(1);
+      D.rb_sys = alloc_work<int>(nsys);
+      D.rb_chunk0 = alloc_work<int>((size_t)nsys + 1);
+      D.rb_cell0 = alloc_work<int>((size_t)nsys + 1);
+    }
     upload_sysd();
     for (int s = 0; s < nsys; ++s)
       if (na[s] > 0) {
@@ -739,6 +754,7 @@ struct Engine::Impl {
     for (cudaEvent_t e : event_pool) cudaEventDestroy(e);
     for (auto& a : allocs) dev_free(a.first);
     free_scratch();
+    for (auto& a : work) dev_free(a.first);
     free_cells();
     if (stream) cudaStreamDestroy(stream);
     if (stream2) cudaStreamDestroy(stream2);
@@ -904,18 +920,11 @@ struct Engine::Impl {
     CK(cudaStreamSynchronize(stream));
     D.total_cells = total;
     D.ccentre = alloc<double>(3 * (size_t)total, true);
-    std::vector<int> bs, bc;
-    for (int q = 0; q < nsys; ++q)
-      for (int c = 0; c < sysd[q].ncells; c += LIST_WARPS) {
-        bs.push_back(q);
-        bc.push_back(sysd[q].cell_base + c);
-      }
-    D.list_blocks = (int)bs.size();
-    D.lblk_sys = alloc<int>(bs.size(), true);
-    D.lblk_cell = alloc<int>(bc.size(), true);
-    CK(cudaMemcpyAsync(D.lblk_sys, bs.data(), sizeof(int) * bs.size(), cudaMemcpyHostToDevice, stream));
-    CK(cudaMemcpyAsync(D.lblk_cell, bc.data(), sizeof(int) * bc.size(), cudaMemcpyHostToDevice, stream));
-    CK(cudaStreamSynchronize(stream));
+    // two words per four cells that nothing reads any more: part of the layout of saved snapshots
+    size_t quads = 0;
+    for (int q = 0; q < nsys; ++q) quads += (sysd[q].ncells + 3) / 4;
+    alloc<int>(quads, true);
+    alloc<int>(quads, true);
   }
 
   void alloc_list(int maxnb) {
@@ -949,19 +958,41 @@ struct Engine::Impl {
     if (lcb_exact() && !capturing) lcb_grow_until_single(s);
   }
 
+  static constexpr unsigned REBUILD_GRID = 4864;  // 32 blocks for each of the 152 SMs
   void launch_rebuild_kernels(cudaStream_t s) {
-    const unsigned nb = nblocks(N, 256);
     mark_begin(s, T_REBUILD);
-    k_bin<<<nb, 256, 0, s>>>(D);
+    // a batch's chain runs over the systems listed by its first kernel, in grids that the list may
+    // exceed or fall short of
+    unsigned nb = 0, nc = (unsigned)D.total_cells;
+    for (int q = 0; q < nsys; ++q) nb += nblocks(natoms[q], REBUILD_CHUNK);
+    if (nsys > 1) {
+      nb = std::min(nb, REBUILD_GRID);
+      nc = std::min(nc, REBUILD_GRID);
+      k_rebuild_list<<<1, RLIST_THREADS, 0, s>>>(D);
+      launched();
+    }
+    k_bin<<<nb, REBUILD_CHUNK, 0, s>>>(D);
     k_scan<<<nsys, 1024, 0, s>>>(D);
-    k_scatter<<<nb, 256, 0, s>>>(D);
-    k_cellsort<<<nblocks(D.total_cells, SORT_WARPS), 32 * SORT_WARPS, 0, s>>>(D);
-    k_permute<<<nb, 256, 0, s>>>(D);
-    k_copyback<<<nb, 256, 0, s>>>(D);
+    k_scatter<<<nb, REBUILD_CHUNK, 0, s>>>(D);
+    k_cellsort<<<nblocks(nc, SORT_WARPS), 32 * SORT_WARPS, 0, s>>>(D);
+    k_permute<<<nb, REBUILD_CHUNK, 0, s>>>(D);
+    k_copyback<<<nb, REBUILD_CHUNK, 0, s>>>(D);
     launched(6);
     if (any_list) {
-      k_buildlist<<<D.list_blocks, 32 * LIST_WARPS, 0, s>>>(D);
-      launched();
+      bool block = false, warp = false;
+      for (const auto& S : sysd) (S.ncells > LIST_BLOCK_CELLS ? warp : block) = true;
+      if (block) {
+        const int batch = list_batch(D.maxnb);
+        if (batch > 0)
+          k_buildlist_block<true><<<nc, 32 * LIST_WARPS, sizeof(unsigned) * batch * (D.maxnb + 4), s>>>(D, batch);
+        else
+          k_buildlist_block<false><<<nc, 32 * LIST_WARPS, 0, s>>>(D, 0);
+        launched();
+      }
+      if (warp) {
+        k_buildlist_warp<<<nblocks(nc, LIST_CELLS), 32 * LIST_CELLS, 0, s>>>(D);
+        launched();
+      }
     }
     mark_end(s, T_REBUILD);
   }

@@ -1,5 +1,6 @@
 // kernels.cuh -- the sm_103a kernels of the MD timestep.
 //
+//   k_rebuild_list the systems of a batch that rebuild, for the kernels of the chain
 //   k_decide       per system: does this force evaluation need a cell/list rebuild?
 //                  (LinkedCell rebuilds at every UpdateCell, plugins/linkedcell.cc:112-267;
 //                   the Verlet list on displacement > skin/2 and/or every `each` UpdateCell
@@ -21,6 +22,8 @@
 //   k_thermo       per-system reduction of the tile sums into the thermo record
 //                  (SetSimulationTags, liblpmd/simulation/simulationbuilder.cc:84-124)
 #pragma once
+
+#include <type_traits>
 
 #include "device.cuh"
 #include "potentials.cuh"
@@ -99,70 +102,161 @@ __global__ void __launch_bounds__(32 * SYS_WARPS) k_decide(Dev D, int nsys, int 
 // Binning and counting sort
 // ---------------------------------------------------------------------------------------------
 
-// Sort-chain options: warp-aggregated cell atomics in k_bin / k_scatter (one atomic per cell
-// and warp instead of one per atom), several cells per thread in k_scan.
-#ifndef GBMD_SORT_AGGREGATE
-#define GBMD_SORT_AGGREGATE 1
-#endif
-#ifndef GBMD_SCAN_CELLS
-#define GBMD_SCAN_CELLS 4
-#endif
+// Work of the rebuild chain.  A batch rebuilds a few of its systems at a time (each by its own
+// displacements), so the chain's kernels do not run over every atom and cell of the batch: their
+// units (chunks of REBUILD_CHUNK atoms, or cells) are numbered over the rebuilding systems alone,
+// listed by k_rebuild_list.  A single system needs no list.
+constexpr int REBUILD_CHUNK = 256;
 
-__global__ void k_bin(Dev D) {
-  long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= D.N) return;
-  int s = D.sysid[i];
-  if (!D.sst[s].need_rebuild) return;
-  const SysDev& S = D.sysd[s];
-  bool ok = true;
-  int cx, cy, cz;
-  if (S.mode == NB_LIST) {
-    // Verlet-list grid: cells are wider than the list radius by a margin, so the binning may
-    // round differently from LinkedCell's; one multiply instead of a division per axis
-    cx = list_cell_coord(D.x[i] * S.ninv[0], S.n[0], ok);
-    cy = list_cell_coord(D.y[i] * S.ninv[1], S.n[1], ok);
-    cz = list_cell_coord(D.z[i] * S.ninv[2], S.n[2], ok);
-  } else {
-    cx = ref_cell_coord(D.x[i], S.L[0], S.n[0], ok);
-    cy = ref_cell_coord(D.y[i], S.L[1], S.n[1], ok);
-    cz = ref_cell_coord(D.z[i], S.L[2], S.n[2], ok);
+constexpr int RLIST_THREADS = 1024;
+__global__ void __launch_bounds__(RLIST_THREADS) k_rebuild_list(Dev D) {
+  __shared__ int part[RLIST_THREADS / 32][3];
+  __shared__ int carry[3];
+  const unsigned all = 0xffffffffu;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  if (threadIdx.x < 3) carry[threadIdx.x] = 0;
+  __syncthreads();
+  for (int base = 0; base < D.nsys; base += RLIST_THREADS) {
+    const int s = base + (int)threadIdx.x;
+    const bool need = s < D.nsys && D.sst[s].need_rebuild;
+    int v[3] = {need ? 1 : 0, need ? (D.sysd[s].natoms + REBUILD_CHUNK - 1) / REBUILD_CHUNK : 0,
+                need ? D.sysd[s].ncells : 0};
+    int x[3];
+    for (int k = 0; k < 3; ++k) {
+      x[k] = v[k];
+      for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(all, x[k], o);
+        if (lane >= o) x[k] += y;
+      }
+      if (lane == 31) part[w][k] = x[k];
+    }
+    __syncthreads();
+    if (w < 3) {
+      int t = part[lane][w];
+      for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(all, t, o);
+        if (lane >= o) t += y;
+      }
+      part[lane][w] = t;
+    }
+    __syncthreads();
+    for (int k = 0; k < 3; ++k) x[k] += carry[k] + (w > 0 ? part[w - 1][k] : 0);
+    if (need) {
+      const int r = x[0] - 1;
+      D.rb_sys[r] = s;
+      D.rb_chunk0[r] = x[1] - v[1];
+      D.rb_cell0[r] = x[2] - v[2];
+    }
+    __syncthreads();
+    if (threadIdx.x == RLIST_THREADS - 1)
+      for (int k = 0; k < 3; ++k) carry[k] = x[k];
+    __syncthreads();
   }
-  if (!ok) {
-    atomicOr(&D.sst[s].error, ERR_OUTSIDE);
-    cx = cy = cz = 0;
+  if (threadIdx.x == 0) {
+    *D.rb_n = carry[0];
+    D.rb_chunk0[carry[0]] = carry[1];
+    D.rb_cell0[carry[0]] = carry[2];
   }
-  int c = S.cell_base + (cz * S.n[1] + cy) * S.n[0] + cx;
-  D.acell[i] = c;
-#if GBMD_SORT_AGGREGATE
-  // consecutive atoms mostly share a cell (the arrays are in the previous cell order): one
-  // atomic per cell and warp
-  const unsigned peers = __match_any_sync(__activemask(), c);
-  if ((threadIdx.x & 31) == __ffs(peers) - 1) atomicAdd(&D.ccount[c], __popc(peers));
-#else
-  atomicAdd(&D.ccount[c], 1);
-#endif
 }
 
-// One block per system: exclusive scan of the cell counts, GBMD_SCAN_CELLS consecutive cells
-// per thread; resets counts and cursors.
-__global__ void k_scan(Dev D) {
+// System and chunk (CELLS: cell) of unit u, false past the last one.
+template <bool CELLS>
+__device__ __forceinline__ bool rebuild_unit(const Dev& D, int u, int& s, int& v) {
+  if (D.nsys == 1) {
+    s = 0;
+    v = u;
+    if (!D.sst[0].need_rebuild) return false;
+    return u < (CELLS ? D.sysd[0].ncells : (D.sysd[0].natoms + REBUILD_CHUNK - 1) / REBUILD_CHUNK);
+  }
+  const int* pre = CELLS ? D.rb_cell0 : D.rb_chunk0;
+  int lo = 0, hi = *D.rb_n;
+  if (u >= pre[hi]) return false;
+  while (hi - lo > 1) {
+    const int mid = (lo + hi) >> 1;
+    if (pre[mid] <= u)
+      lo = mid;
+    else
+      hi = mid;
+  }
+  s = D.rb_sys[lo];
+  v = u - pre[lo];
+  return true;
+}
+
+// Calls body(system, atom) for this thread's atoms of the rebuilding systems.
+template <class F>
+__device__ __forceinline__ void for_rebuild_atoms(const Dev& D, F&& body) {
+  int s, v;
+  for (int u = blockIdx.x; rebuild_unit<false>(D, u, s, v); u += gridDim.x) {
+    const int k = v * REBUILD_CHUNK + (int)threadIdx.x;
+    if (k < D.sysd[s].natoms) body(s, D.sysd[s].atom_base + k);
+  }
+}
+
+__global__ void __launch_bounds__(REBUILD_CHUNK) k_bin(Dev D) {
+  for_rebuild_atoms(D, [&](int s, long long i) {
+    const SysDev& S = D.sysd[s];
+    bool ok = true;
+    int cx, cy, cz;
+    if (S.mode == NB_LIST) {
+      // Verlet-list grid: cells are wider than the list radius by a margin, so the binning may
+      // round differently from LinkedCell's; one multiply instead of a division per axis
+      cx = list_cell_coord(D.x[i] * S.ninv[0], S.n[0], ok);
+      cy = list_cell_coord(D.y[i] * S.ninv[1], S.n[1], ok);
+      cz = list_cell_coord(D.z[i] * S.ninv[2], S.n[2], ok);
+    } else {
+      cx = ref_cell_coord(D.x[i], S.L[0], S.n[0], ok);
+      cy = ref_cell_coord(D.y[i], S.L[1], S.n[1], ok);
+      cz = ref_cell_coord(D.z[i], S.L[2], S.n[2], ok);
+    }
+    if (!ok) {
+      atomicOr(&D.sst[s].error, ERR_OUTSIDE);
+      cx = cy = cz = 0;
+    }
+    const int c = S.cell_base + (cz * S.n[1] + cy) * S.n[0] + cx;
+    D.acell[i] = c;
+    // consecutive atoms mostly share a cell (the arrays are in the previous cell order): one
+    // atomic per cell and warp
+    const unsigned peers = __match_any_sync(__activemask(), c);
+    if ((threadIdx.x & 31) == __ffs(peers) - 1) atomicAdd(&D.ccount[c], __popc(peers));
+  });
+}
+
+// One block per system: exclusive scan of the cell counts; resets counts and cursors.  A thread takes
+// 16 consecutive cells as four 16-byte words (from the aligned word that holds the system's first
+// cell on), so that a pass of the block covers 16,384 cells: the block's chain of load, scan and
+// barriers, not bandwidth, is the time (4 cells a thread: 123 us for the 110,592 cells of a 2 M atom
+// liquid, 63 so; 16 -> 9 us for 13,824).
+constexpr int SCAN_CELLS = 16;
+__global__ void __launch_bounds__(1024) k_scan(Dev D) {
   const int s = blockIdx.x;
   if (!D.sst[s].need_rebuild) return;
   const SysDev& S = D.sysd[s];
-  const int nc = S.ncells, cb = S.cell_base;
+  const int cb = S.cell_base, ce = cb + S.ncells, a0 = cb & ~3;
   __shared__ int warp_tot[32];
-  __shared__ int carry;
-  if (threadIdx.x == 0) carry = 0;
-  __syncthreads();
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = blockDim.x >> 5;
-  for (int base = 0; base < nc; base += blockDim.x * GBMD_SCAN_CELLS) {
-    const int c0 = base + threadIdx.x * GBMD_SCAN_CELLS;
-    int v[GBMD_SCAN_CELLS];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  int carry = (int)S.atom_base;  // global slots
+  for (int base = a0; base < ce; base += 1024 * SCAN_CELLS) {
+    const int c0 = base + threadIdx.x * SCAN_CELLS;
+    int v[SCAN_CELLS];
     int sum = 0;
 #pragma unroll
-    for (int k = 0; k < GBMD_SCAN_CELLS; ++k) {
-      v[k] = (c0 + k < nc) ? D.ccount[cb + c0 + k] : 0;
-      sum += v[k];
+    for (int k = 0; k < SCAN_CELLS; k += 4) {
+      const bool whole = c0 + k >= cb && c0 + k + 4 <= ce;
+      int4 x = make_int4(0, 0, 0, 0);
+      if (whole) {
+        x = *reinterpret_cast<const int4*>(D.ccount + c0 + k);
+      } else {
+        if (c0 + k >= cb && c0 + k < ce) x.x = D.ccount[c0 + k];
+        if (c0 + k + 1 >= cb && c0 + k + 1 < ce) x.y = D.ccount[c0 + k + 1];
+        if (c0 + k + 2 >= cb && c0 + k + 2 < ce) x.z = D.ccount[c0 + k + 2];
+        if (c0 + k + 3 >= cb && c0 + k + 3 < ce) x.w = D.ccount[c0 + k + 3];
+      }
+      v[k] = x.x;
+      v[k + 1] = x.y;
+      v[k + 2] = x.z;
+      v[k + 3] = x.w;
+      sum += (x.x + x.y) + (x.z + x.w);
     }
     int x = sum;
 #pragma unroll
@@ -172,30 +266,37 @@ __global__ void k_scan(Dev D) {
     }
     if (lane == 31) warp_tot[w] = x;
     __syncthreads();
-    if (w == 0) {
-      int t = (lane < nw) ? warp_tot[lane] : 0;
+    int t = warp_tot[lane];  // every warp scans the 32 totals for itself
 #pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        int y = __shfl_up_sync(0xffffffffu, t, o);
-        if (lane >= o) t += y;
-      }
-      if (lane < nw) warp_tot[lane] = t;
+    for (int o = 1; o < 32; o <<= 1) {
+      int y = __shfl_up_sync(0xffffffffu, t, o);
+      if (lane >= o) t += y;
     }
-    __syncthreads();
-    int excl = x - sum + (w > 0 ? warp_tot[w - 1] : 0) + carry;
+    const int before = __shfl_sync(0xffffffffu, t, w > 0 ? w - 1 : 0);
+    int excl = x - sum + (w > 0 ? before : 0) + carry;
+    carry += __shfl_sync(0xffffffffu, t, 31);
 #pragma unroll
-    for (int k = 0; k < GBMD_SCAN_CELLS; ++k) {
-      if (c0 + k < nc) {
-        D.cstart[cb + c0 + k] = (int)(S.atom_base) + excl;  // global slot
-        D.ccnt[cb + c0 + k] = v[k];
-        D.ccount[cb + c0 + k] = 0;
-        D.ccursor[cb + c0 + k] = 0;
+    for (int k = 0; k < SCAN_CELLS; k += 4) {
+      const int4 st = make_int4(excl, excl + v[k], excl + v[k] + v[k + 1], excl + v[k] + v[k + 1] + v[k + 2]);
+      if (c0 + k >= cb && c0 + k + 4 <= ce) {
+        *reinterpret_cast<int4*>(D.cstart + c0 + k) = st;
+        *reinterpret_cast<int4*>(D.ccnt + c0 + k) = make_int4(v[k], v[k + 1], v[k + 2], v[k + 3]);
+        *reinterpret_cast<int4*>(D.ccount + c0 + k) = make_int4(0, 0, 0, 0);
+        *reinterpret_cast<int4*>(D.ccursor + c0 + k) = make_int4(0, 0, 0, 0);
+      } else {
+        const int start[4] = {st.x, st.y, st.z, st.w};
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+          if (c0 + k + q >= cb && c0 + k + q < ce) {
+            D.cstart[c0 + k + q] = start[q];
+            D.ccnt[c0 + k + q] = v[k + q];
+            D.ccount[c0 + k + q] = 0;
+            D.ccursor[c0 + k + q] = 0;
+          }
       }
-      excl += v[k];
+      excl += v[k] + v[k + 1] + v[k + 2] + v[k + 3];
     }
-    __syncthreads();
-    if (threadIdx.x == blockDim.x - 1) carry = excl;  // the block's running total
-    __syncthreads();
+    __syncthreads();  // warp_tot is written again
   }
 }
 
@@ -213,43 +314,28 @@ __global__ void k_binary_clear(Dev D) {
   for (int s = threadIdx.x; s < D.nsys; s += blockDim.x) D.sst[s].collide = 0;
 }
 
-__global__ void k_scatter(Dev D) {
-  long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= D.N) return;
-  int s = D.sysid[i];
-  if (!D.sst[s].need_rebuild) return;
-  int c = D.acell[i];
-#if GBMD_SORT_AGGREGATE
-  // the warp's atoms of one cell take consecutive slots from one atomic (their order inside
-  // the cell is set by k_cellsort either way)
-  const unsigned peers = __match_any_sync(__activemask(), c);
-  const int lane = threadIdx.x & 31, lead = __ffs(peers) - 1;
-  int first = 0;
-  if (lane == lead) first = atomicAdd(&D.ccursor[c], __popc(peers));
-  first = __shfl_sync(peers, first, lead);
-  int p = D.cstart[c] + first + __popc(peers & ((1u << lane) - 1u));
-#else
-  int p = D.cstart[c] + atomicAdd(&D.ccursor[c], 1);
-#endif
-  D.perm[p] = (int)i;
+__global__ void __launch_bounds__(REBUILD_CHUNK) k_scatter(Dev D) {
+  for_rebuild_atoms(D, [&](int, long long i) {
+    const int c = D.acell[i];
+    // the warp's atoms of one cell take consecutive slots from one atomic (their order inside
+    // the cell is set by k_cellsort either way)
+    const unsigned peers = __match_any_sync(__activemask(), c);
+    const int lane = threadIdx.x & 31, lead = __ffs(peers) - 1;
+    int first = 0;
+    if (lane == lead) first = atomicAdd(&D.ccursor[c], __popc(peers));
+    first = __shfl_sync(peers, first, lead);
+    D.perm[D.cstart[c] + first + __popc(peers & ((1u << lane) - 1u))] = (int)i;
+  });
 }
 
-// One warp per cell over the cells of every system (flat index g; cell_sys maps it back):
-// orders the cell's slots by original index, the order in which LinkedCell's head/next lists
+// One warp per cell of the rebuilding systems: orders the cell's slots by original index, the order in which LinkedCell's head/next lists
 // visit them.  Each atom's rank is the number of smaller tags in its cell: up to 32 atoms the
 // lanes compare through shuffles, up to SORT_STAGE atoms (dense cells of a liquid, coarse
 // LinkedCell grids) through a copy of the cell's tags in shared memory, and beyond that through
 // global scratch (n^2/32 compares per lane).
 constexpr int SORT_WARPS = 4;    // cells per block
 constexpr int SORT_STAGE = 256;  // atoms per cell ranked in shared memory
-__global__ void __launch_bounds__(32 * SORT_WARPS) k_cellsort(Dev D) {
-  __shared__ int s_tag[SORT_WARPS][SORT_STAGE];
-  __shared__ int s_idx[SORT_WARPS][SORT_STAGE];
-  const int w = threadIdx.x >> 5;
-  const int g = blockIdx.x * SORT_WARPS + w;
-  if (g >= D.total_cells) return;
-  const int s = D.cell_sys[g];
-  if (!D.sst[s].need_rebuild) return;
+__device__ __forceinline__ void sort_cell(const Dev& D, int g, int* tg, int* ix) {
   const int lane = threadIdx.x & 31;
   const int b = D.cstart[g], n = D.ccnt[g];
   if (n <= 32) {
@@ -265,8 +351,6 @@ __global__ void __launch_bounds__(32 * SORT_WARPS) k_cellsort(Dev D) {
     return;
   }
   if (n <= SORT_STAGE) {
-    int* tg = s_tag[w];
-    int* ix = s_idx[w];
     for (int k = lane; k < n; k += 32) {
       const int v = D.perm[b + k];
       ix[k] = v;
@@ -296,33 +380,41 @@ __global__ void __launch_bounds__(32 * SORT_WARPS) k_cellsort(Dev D) {
   __syncwarp();
   for (int k = lane; k < n; k += 32) D.perm[b + k] = sorted[b + k];
 }
+__global__ void __launch_bounds__(32 * SORT_WARPS) k_cellsort(Dev D) {
+  __shared__ int s_tag[SORT_WARPS][SORT_STAGE];
+  __shared__ int s_idx[SORT_WARPS][SORT_STAGE];
+  const int w = threadIdx.x >> 5;
+  int s, v;
+  for (int u = blockIdx.x * SORT_WARPS + w; rebuild_unit<true>(D, u, s, v); u += gridDim.x * SORT_WARPS) {
+    sort_cell(D, D.sysd[s].cell_base + v, s_tag[w], s_idx[w]);
+    __syncwarp();
+  }
+}
 
-__global__ void k_permute(Dev D) {
-  long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= D.N) return;
-  int s = D.sysid[p];
-  if (!D.sst[s].need_rebuild) return;
-  const long long N = D.N;
-  int o = D.perm[p];
-  double* sd = D.sdbl;
-  sd[0 * N + p] = D.x[o];
-  sd[1 * N + p] = D.y[o];
-  sd[2 * N + p] = D.z[o];
-  sd[3 * N + p] = D.vx[o];
-  sd[4 * N + p] = D.vy[o];
-  sd[5 * N + p] = D.vz[o];
-  sd[6 * N + p] = D.ax[o];
-  sd[7 * N + p] = D.ay[o];
-  sd[8 * N + p] = D.az[o];
-  sd[9 * N + p] = D.mass[o];
-  sd[10 * N + p] = D.fm[o];
-  int* si = D.sint;
-  si[0 * N + p] = D.type[o];
-  si[1 * N + p] = D.tag[o];
-  si[2 * N + p] = D.acell[o];
-  if (D.has_flags) D.sflags[p] = D.flags[o];
-  if (D.ist)
-    for (int k = 0; k < IST_K; ++k) D.ist_alt[k * N + p] = D.ist[k * N + o];
+__global__ void __launch_bounds__(REBUILD_CHUNK) k_permute(Dev D) {
+  for_rebuild_atoms(D, [&](int, long long p) {
+    const long long N = D.N;
+    const int o = D.perm[p];
+    double* sd = D.sdbl;
+    sd[0 * N + p] = D.x[o];
+    sd[1 * N + p] = D.y[o];
+    sd[2 * N + p] = D.z[o];
+    sd[3 * N + p] = D.vx[o];
+    sd[4 * N + p] = D.vy[o];
+    sd[5 * N + p] = D.vz[o];
+    sd[6 * N + p] = D.ax[o];
+    sd[7 * N + p] = D.ay[o];
+    sd[8 * N + p] = D.az[o];
+    sd[9 * N + p] = D.mass[o];
+    sd[10 * N + p] = D.fm[o];
+    int* si = D.sint;
+    si[0 * N + p] = D.type[o];
+    si[1 * N + p] = D.tag[o];
+    si[2 * N + p] = D.acell[o];
+    if (D.has_flags) D.sflags[p] = D.flags[o];
+    if (D.ist)
+      for (int k = 0; k < IST_K; ++k) D.ist_alt[k * N + p] = D.ist[k * N + o];
+  });
 }
 
 // Offset of x from the centre xc of its home cell, wrapped into [-L/2, L/2).  Two FP64-pipe
@@ -375,32 +467,30 @@ __device__ __forceinline__ void track_displacement_warp(const Dev& D, int s, flo
   if ((threadIdx.x & 31) == 0 && m) atomicMax(&D.sst[s].maxdisp2, m);
 }
 
-__global__ void k_copyback(Dev D) {
-  long long p = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= D.N) return;
-  int s = D.sysid[p];
-  if (!D.sst[s].need_rebuild) return;
-  const long long N = D.N;
-  const double* sd = D.sdbl;
-  D.x[p] = sd[0 * N + p];
-  D.y[p] = sd[1 * N + p];
-  D.z[p] = sd[2 * N + p];
-  D.vx[p] = sd[3 * N + p];
-  D.vy[p] = sd[4 * N + p];
-  D.vz[p] = sd[5 * N + p];
-  D.ax[p] = sd[6 * N + p];
-  D.ay[p] = sd[7 * N + p];
-  D.az[p] = sd[8 * N + p];
-  D.mass[p] = sd[9 * N + p];
-  D.fm[p] = sd[10 * N + p];
-  const int* si = D.sint;
-  D.type[p] = si[0 * N + p];
-  D.tag[p] = si[1 * N + p];
-  D.home[p] = si[2 * N + p];
-  if (D.has_flags) D.flags[p] = D.sflags[p];
-  if (D.ist)
-    for (int k = 0; k < IST_K; ++k) D.ist[k * N + p] = D.ist_alt[k * N + p];
-  refresh_gather(D, D.sysd[s], p, true);
+__global__ void __launch_bounds__(REBUILD_CHUNK) k_copyback(Dev D) {
+  for_rebuild_atoms(D, [&](int s, long long p) {
+    const long long N = D.N;
+    const double* sd = D.sdbl;
+    D.x[p] = sd[0 * N + p];
+    D.y[p] = sd[1 * N + p];
+    D.z[p] = sd[2 * N + p];
+    D.vx[p] = sd[3 * N + p];
+    D.vy[p] = sd[4 * N + p];
+    D.vz[p] = sd[5 * N + p];
+    D.ax[p] = sd[6 * N + p];
+    D.ay[p] = sd[7 * N + p];
+    D.az[p] = sd[8 * N + p];
+    D.mass[p] = sd[9 * N + p];
+    D.fm[p] = sd[10 * N + p];
+    const int* si = D.sint;
+    D.type[p] = si[0 * N + p];
+    D.tag[p] = si[1 * N + p];
+    D.home[p] = si[2 * N + p];
+    if (D.has_flags) D.flags[p] = D.sflags[p];
+    if (D.ist)
+      for (int k = 0; k < IST_K; ++k) D.ist[k * N + p] = D.ist_alt[k * N + p];
+    refresh_gather(D, D.sysd[s], p, true);
+  });
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -409,41 +499,247 @@ __global__ void k_copyback(Dev D) {
 
 __device__ __forceinline__ int shift_code(int kx, int ky, int kz) { return (kx + 2) + 5 * ((ky + 2) + 5 * (kz + 2)); }
 
-// One warp per home cell (per-block table of system and cells): the lanes hold up to 32 atoms
-// of the cell, and the atoms of each stencil cell are staged through shared memory 32 at a
-// time; every lane then tests the staged candidate against its own atom (broadcast reads, no
-// divergence between lanes, since all atoms of a cell share the stencil and its cell-shift
-// codes), and appends its hits in candidate order through a bit mask.
-constexpr int LIST_WARPS = 4;
-// Candidate tests four at a time over a sentinel-padded stage, appends through a running write
-// position (1); or one candidate per iteration with the entry address recomputed per append (0).
-#ifndef GBMD_LIST_UNROLL4
-#define GBMD_LIST_UNROLL4 1
-#endif
-// Resident blocks per SM the register allocation of the list build is sized for.
-#ifndef GBMD_LIST_MIN_BLOCKS
-#define GBMD_LIST_MIN_BLOCKS 4
-#endif
+// The Verlet list is built by one of two kernels, by the size of the system's grid: up to
+// LIST_BLOCK_CELLS cells a block works on a home cell, above that a warp.  Both make the same list.
+// A warp per cell needs fewer instructions an atom, but is a serial chain 27 cells long, which is
+// all there is where the grid does not fill the GPU several times over, or where a few systems of a
+// batch rebuild in a step; the block's chain is a quarter of that.  Measured (block / warp per cell):
+// 125 cells (4,000 atoms) 25 / 69 us, 1,728 cells (32,000) 32 / 40, an ensemble of 128 systems
+// 88 / 159 us a step; but 5,832 cells (32,000 atoms of iron) 45.6 / 39.0, 12,167 (256k LJ liquid)
+// 173 / 157, 13,824 (495k copper) 590 / 569, 97,336 (2 M atoms) 1396 / 1146.  (The warp form with
+// its distance tests as compares and selects instead of shifted signs: 171, 629 and 1239.)
+constexpr int LIST_BLOCK_CELLS = 4096;
+constexpr int LIST_WARPS = 8;
+constexpr int LIST_STAGE = 1024;
+constexpr int LIST_STENCIL = 125;       // cells of the widest stencil (radius 2)
+constexpr int LIST_ROWS_BYTES = 28672;  // shared memory of the rows (the rest is 20 KB)
 
-__global__ void __launch_bounds__(32 * LIST_WARPS, GBMD_LIST_MIN_BLOCKS) k_buildlist(Dev D) {
-#if GBMD_LIST_UNROLL4 && GBMD_F32X2
-  // coordinates staged as three arrays, so that one 16-byte shared load gives the x (y, z)
-  // of four consecutive candidates: two packed pairs
-  __shared__ __align__(16) float stage[LIST_WARPS][3][32];
-#else
-  __shared__ float4 stage[LIST_WARPS][32];
-#endif
+// Home atoms whose rows fit in shared memory (0: none, entries then go straight to the list).
+inline int list_batch(int maxnb) {
+  const int n = LIST_ROWS_BYTES / ((maxnb + 4) * 4);
+  return n > 32 ? 32 : n;
+}
+
+// The list's test of entry e of an atom at offset gi, in k_buildlist_warp's operation order.
+__device__ __noinline__ bool list_pair(const SysDev& S, const float4& gi, const float4* g32, unsigned e) {
+  const int code = (int)(e >> CODE_SHIFT);
+  const float4 g = g32[e & LOCAL_MASK];
+  const float ox = (float)(code % 5 - 2) * S.df[0] - gi.x, oy = (float)(code / 5 % 5 - 2) * S.df[1] - gi.y,
+              oz = (float)(code / 25 - 2) * S.df[2] - gi.z;
+  const float rx = ox + g.x, ry = oy + g.y, rz = oz + g.z;
+  return fmaf(rx, rx, fmaf(ry, ry, rz * rz)) < S.rlist2f;
+}
+
+// One block per home cell.  The atoms of the stencil's cells are staged in shared memory as one
+// run, LIST_STAGE at a time, each shifted by its cell's offset from the home cell and with its list
+// entry beside it; each warp takes home atoms in turn and tests 64 candidates at a time (two a
+// lane, in packed FP32 pairs), the hits' places in the atom's row by ballot.  The rows of `batch`
+// home atoms are put together in shared memory and leave as whole 16-byte groups of neighbouring
+// atoms (written straight to the list, the half-filled sectors cost more than the tests).
+// (A pair so close to the list radius that the staged sums' rounding could decide it, by at most
+// 4e-6 rl^2, sends its atom through the same loop once more with k_buildlist_warp's operation order,
+// one atom in a few hundred: so the lists are the same.)
+// ROWS: `batch` rows are put together in shared memory; else the entries go straight to the list.
+template <bool ROWS>
+__global__ void __launch_bounds__(32 * LIST_WARPS, 4) k_buildlist_block(Dev D, int batch) {
+  extern __shared__ __align__(16) unsigned rows[];  // batch rows of maxnb + 4 words
+  __shared__ __align__(16) float cx[LIST_STAGE], cy[LIST_STAGE], cz[LIST_STAGE];
+  __shared__ __align__(16) unsigned ce[LIST_STAGE];
+  __shared__ float4 c_shift[LIST_STENCIL];  // offset of the stencil cell, and its entries' code bits
+  __shared__ int c_first[LIST_STENCIL];     // its first atom (index within the system)
+  __shared__ int c_off[LIST_STENCIL + 4];   // running total of the atoms of the cells before it
+  __shared__ int count[32];                 // entries of the batch's atoms
+  const unsigned all = 0xffffffffu;
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  // every block covers LIST_WARPS cells of one system (a per-block table), so the system
-  // index is the same for the whole block and the grid holds no block of an empty range
-  const int s = D.lblk_sys[blockIdx.x];
-  const int g0 = D.lblk_cell[blockIdx.x] + w;
-  if (g0 >= D.sysd[s].cell_base + D.sysd[s].ncells) return;
-  if (!D.sst[s].need_rebuild) return;
+  const unsigned below = (1u << lane) - 1u;
+  const int maxnb = D.maxnb, rs = maxnb + 4, nbatch = ROWS ? batch : 32;
+  int s, c;
+  for (int u = blockIdx.x; rebuild_unit<true>(D, u, s, c); u += gridDim.x) {
+    const SysDev& S = D.sysd[s];
+    const int cell_base = S.cell_base;
+    const int n0 = D.ccnt[cell_base + c];
+    if (S.mode != NB_LIST || S.ncells > LIST_BLOCK_CELLS || n0 == 0) continue;
+    const long long atom_base = S.atom_base;
+    const int b0 = (int)(D.cstart[cell_base + c] - atom_base);
+    const int R = S.stencil_r, W = 2 * R + 1, nst = W * W * W;
+    const int nx = S.n[0], ny = S.n[1], nz = S.n[2];
+    for (int t = threadIdx.x; t < nst; t += blockDim.x) {
+      const int dx = t % W - R, dy = (t / W) % W - R, dz = t / (W * W) - R;
+      const int xc = wrap_around(c % nx + dx, nx), yc = wrap_around((c / nx) % ny + dy, ny),
+                zc = wrap_around(c / (nx * ny) + dz, nz);
+      const int g = cell_base + (zc * ny + yc) * nx + xc;
+      c_first[t] = (int)(D.cstart[g] - atom_base);
+      c_off[t + 1] = D.ccnt[g];
+      c_shift[t] = make_float4((float)dx * S.df[0], (float)dy * S.df[1], (float)dz * S.df[2],
+                               __uint_as_float((unsigned)shift_code(dx, dy, dz) << CODE_SHIFT));
+    }
+    __syncthreads();
+    if (w == 0) {  // exclusive running totals, four cells a lane
+      int v[4], sum = 0;
+      for (int k = 0; k < 4; ++k) {
+        v[k] = 4 * lane + k < nst ? c_off[4 * lane + k + 1] : 0;
+        sum += v[k];
+      }
+      int x = sum;
+      for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(all, x, o);
+        if (lane >= o) x += y;
+      }
+      x -= sum;
+      __syncwarp();
+      for (int k = 0; k < 4; ++k) {
+        if (4 * lane + k <= nst) c_off[4 * lane + k] = x;
+        x += v[k];
+      }
+    }
+    __syncthreads();
+    const int total = c_off[nst];
+    const float4* __restrict__ g32 = D.g32 + atom_base;
+    unsigned* const nl = D.nl + S.nl_base;
+    const long long na = S.natoms;
+    const float rl2 = S.rlist2f;
+    const float tol = 1e-5f * rl2;
+    int most = 0, staged = -1;
+    for (int a0 = 0; a0 < n0; a0 += nbatch) {
+      const int nb = min(nbatch, n0 - a0);
+      if ((int)threadIdx.x < nb) count[threadIdx.x] = 0;
+      for (int w0 = 0; w0 < total; w0 += LIST_STAGE) {
+        const int m = min(LIST_STAGE, total - w0), mp = (m + 63) & ~63;
+        if (staged != w0) {
+          for (int t = w; t < nst; t += LIST_WARPS) {
+            const int n = c_off[t + 1] - c_off[t], p0 = c_off[t] - w0, first = c_first[t];
+            const float4 sh = c_shift[t];
+            for (int k = lane; k < n; k += 32)
+              if (p0 + k >= 0 && p0 + k < LIST_STAGE) {
+                const float4 g = g32[first + k];
+                cx[p0 + k] = g.x + sh.x;
+                cy[p0 + k] = g.y + sh.y;
+                cz[p0 + k] = g.z + sh.z;
+                ce[p0 + k] = __float_as_uint(sh.w) | (unsigned)(first + k);
+              }
+          }
+          // far-away sentinels fill the last 64 (r^2 ~ 1e36 never hits)
+          for (int k = m + (int)threadIdx.x; k < mp; k += blockDim.x) {
+            cx[k] = 1e18f;
+            cy[k] = cz[k] = 0.0f;
+            ce[k] = 0u;
+          }
+          staged = w0;
+        }
+        __syncthreads();
+        for (int a = w; a < nb; a += LIST_WARPS) {
+          const int li = b0 + a0 + a;
+          const float4 gi = g32[li];
+          const f32x2 gx = f2_pack(gi.x, gi.x), gy = f2_pack(gi.y, gi.y), gz = f2_pack(gi.z, gi.z),
+                      out2 = f2_pack(-rl2, -rl2);
+          const unsigned self = ((unsigned)shift_code(0, 0, 0) << CODE_SHIFT) | (unsigned)li;
+          unsigned* const row = rows + a * rs;
+          const int cnt0 = count[a];
+          int cnt = 0;
+          bool near = false;
+          auto scan = [&](auto exact) {
+            cnt = cnt0;
+            int k = 2 * lane;
+            unsigned h0, h1;
+            bool in0, in1;
+            uint2 e;
+            auto test = [&]() {
+              e = *reinterpret_cast<const uint2*>(ce + k);
+              if (decltype(exact)::value) {
+                in0 = k < m && list_pair(S, gi, g32, e.x);
+                in1 = k + 1 < m && list_pair(S, gi, g32, e.y);
+              } else {
+                const float2 X = *reinterpret_cast<const float2*>(cx + k), Y = *reinterpret_cast<const float2*>(cy + k),
+                             Z = *reinterpret_cast<const float2*>(cz + k);
+                const f32x2 rx = f2_sub(f2_pack(X.x, X.y), gx), ry = f2_sub(f2_pack(Y.x, Y.y), gy),
+                            rz = f2_sub(f2_pack(Z.x, Z.y), gz);
+                float d0, d1;  // r^2 - rl^2
+                f2_unpack(f2_fma(rx, rx, f2_fma(ry, ry, f2_fma(rz, rz, out2))), d0, d1);
+                in0 = d0 < 0.0f;
+                in1 = d1 < 0.0f;
+                near = near || fminf(fabsf(d0), fabsf(d1)) < tol;
+              }
+              in0 = in0 && e.x != self;
+              in1 = in1 && e.y != self;
+              h0 = __ballot_sync(all, in0);
+              h1 = __ballot_sync(all, in1);
+            };
+            if (ROWS) {
+              // while 64 more entries surely fit
+              const int room = maxnb - 64;
+              for (; k < mp && cnt <= room; k += 64) {
+                test();
+                unsigned* at = row + (cnt + __popc(h0 & below) + __popc(h1 & below));
+                if (in0) *at++ = e.x;
+                if (in1) *at = e.y;
+                cnt += __popc(h0) + __popc(h1);
+              }
+            }
+            for (; k < mp; k += 64) {
+              test();
+              int p = cnt + __popc(h0 & below) + __popc(h1 & below);
+              auto put = [&](unsigned v) {
+                if (p < maxnb) {
+                  if (ROWS)
+                    row[p] = v;
+                  else
+                    nl[((long long)(p >> 2) * na + li) * 4 + (p & 3)] = v;
+                }
+                ++p;
+              };
+              if (in0) put(e.x);
+              if (in1) put(e.y);
+              cnt += __popc(h0) + __popc(h1);
+            }
+          };
+          scan(std::false_type());
+          if (__any_sync(all, near)) scan(std::true_type());
+          __syncwarp();  // every lane has read the atom's count
+          if (lane == 0) count[a] = cnt;
+        }
+        __syncthreads();
+      }
+      // lane = atom of the batch, warps over the groups of four; words past the end are written as
+      // entry 0, which the force passes may load but do not count
+      const int cnt = lane < nb ? count[lane] : 0;
+      const int kept = min(cnt, maxnb);
+      most = max(most, cnt);
+      if (ROWS) {
+        const int ng = (int)__reduce_max_sync(all, (unsigned)(kept + 3) >> 2);
+        for (int q = w; q < ng; q += LIST_WARPS)
+          if (4 * q < kept) {
+            uint4 v = *reinterpret_cast<const uint4*>(rows + lane * rs + 4 * q);
+            const int left = kept - 4 * q;
+            if (left < 2) v.y = 0u;
+            if (left < 3) v.z = 0u;
+            if (left < 4) v.w = 0u;
+            reinterpret_cast<uint4*>(nl)[q * na + b0 + a0 + lane] = v;
+          }
+      }
+      if (w == 0 && lane < nb) D.ncount[atom_base + b0 + a0 + lane] = kept;
+      __syncthreads();
+    }
+    if (w == 0) {
+      most = (int)__reduce_max_sync(all, (unsigned)most);
+      if (lane == 0) {
+        if (most > *(volatile int*)&D.sst[s].max_count) atomicMax(&D.sst[s].max_count, most);
+        if (most > maxnb) atomicOr(&D.sst[s].error, ERR_LIST);
+      }
+    }
+  }
+}
+
+// The atoms of home cell c of system S, up to 32 at a time a lane each: the atoms of each stencil
+// cell are staged through shared memory 32 at a time; every lane then tests the staged candidates
+// against its own atom (broadcast reads, no divergence between lanes, since all atoms of a cell share
+// the stencil and its cell-shift codes; the sign of r^2 - rl^2 shifts into a mask), and appends its
+// hits in candidate order.
+constexpr int LIST_CELLS = 4;  // home cells (warps) of a block
+__device__ __forceinline__ void list_cell(const Dev& D, const SysDev& S, int s, int c, float* stx, float* sty,
+                                          float* stz) {
+  const int lane = threadIdx.x & 31;
   // the system's grid in registers: the list stores below may alias any global memory, so
   // fields read through the SysDev reference would be re-read after every store
-  const SysDev& S = D.sysd[s];
-  if (S.mode != NB_LIST) return;
   const int nx = S.n[0], ny = S.n[1], nz = S.n[2];
   const float dfx = S.df[0], dfy = S.df[1], dfz = S.df[2];
   const int cell_base = S.cell_base;
@@ -456,28 +752,19 @@ __global__ void __launch_bounds__(32 * LIST_WARPS, GBMD_LIST_MIN_BLOCKS) k_build
   const int* __restrict__ ccnt = D.ccnt;
   const float4* __restrict__ g32 = D.g32;
   const int maxnb = D.maxnb;
-  const int c = g0 - cell_base;
-  const int b0 = cstart[g0], n0 = ccnt[g0];
+  const int b0 = cstart[cell_base + c], n0 = ccnt[cell_base + c];
   const int cx = c % nx, cy = (c / nx) % ny, cz = c / (nx * ny);
-#if GBMD_LIST_UNROLL4 && GBMD_F32X2
-  float* const stx = stage[w][0];
-  float* const sty = stage[w][1];
-  float* const stz = stage[w][2];
-#else
-  float4* st = stage[w];
-#endif
+  int most = 0;
   for (int base = 0; base < n0; base += 32) {
     const bool has = base + lane < n0;
     const long long i = (long long)b0 + base + lane;
     const int li = (int)(i - atom_base);
     const float4 gi = has ? g32[i] : make_float4(0.f, 0.f, 0.f, 0.f);
-    const float rl2 = has ? rlist2 : -1.0f;  // lanes without an atom never match
-    unsigned* out = nl + (long long)li * 4;
+    const float out = has ? -rlist2 : 1.0f;  // lanes without an atom never match
+    const f32x2 out2 = f2_pack(out, out);
     const long long gstride = (long long)na * 4;  // words between consecutive groups of four
     int cnt = 0;
-#if GBMD_LIST_UNROLL4
-    unsigned* wp = out;
-#endif
+    unsigned* wp = nl + (long long)li * 4;
     for (int dz = -R; dz <= R; ++dz) {
       const int zc = wrap_around(cz + dz, nz);
       const float sz = (float)dz * dfz;
@@ -491,33 +778,23 @@ __global__ void __launch_bounds__(32 * LIST_WARPS, GBMD_LIST_MIN_BLOCKS) k_build
           const int b = cstart[g], n = ccnt[g];
           const unsigned code = (unsigned)shift_code(dx, dy, dz) << CODE_SHIFT;
           const float ox = sx - gi.x, oy = sy - gi.y, oz = sz - gi.z;
-#if GBMD_LIST_UNROLL4 && GBMD_F32X2
           const f32x2 ox2 = f2_pack(ox, ox), oy2 = f2_pack(oy, oy), oz2 = f2_pack(oz, oz);
-#endif
           for (int jb = 0; jb < n; jb += 32) {
             __syncwarp();
-#if GBMD_LIST_UNROLL4 && GBMD_F32X2
             {
               const float4 gj = jb + lane < n ? g32[b + jb + lane] : make_float4(1e18f, 1e18f, 1e18f, 0.f);
               stx[lane] = gj.x;
               sty[lane] = gj.y;
               stz[lane] = gj.z;
             }
-#elif GBMD_LIST_UNROLL4
-            // every stage slot is written: past the cell's atoms a far-away sentinel, so the test
-            // loop runs in whole quads of candidates (the sentinel never hits: r^2 ~ 3e36)
-            st[lane] = jb + lane < n ? g32[b + jb + lane] : make_float4(1e18f, 1e18f, 1e18f, 0.f);
-#else
-            if (jb + lane < n) st[lane] = g32[b + jb + lane];
-#endif
             __syncwarp();
             const int m = min(32, n - jb);
             const int jl0 = b + jb - (int)atom_base;
-            // pass 1: a bit per staged candidate inside the list radius (branch-free)
+            // pass 1: a bit per staged candidate inside the list radius (branch-free), candidate k
+            // in bit 31 - k
             unsigned hits = 0u;
-#if GBMD_LIST_UNROLL4 && GBMD_F32X2
             for (int k = 0; k < m; k += 4) {
-              // candidates k..k+3 as two packed pairs, in the scalar form's operation order
+              // candidates k..k+3 as two packed pairs
               const float4 X = *reinterpret_cast<const float4*>(stx + k);
               const float4 Y = *reinterpret_cast<const float4*>(sty + k);
               const float4 Z = *reinterpret_cast<const float4*>(stz + k);
@@ -526,46 +803,24 @@ __global__ void __launch_bounds__(32 * LIST_WARPS, GBMD_LIST_MIN_BLOCKS) k_build
               const f32x2 rz01 = f2_add(oz2, f2_pack(Z.x, Z.y)), rz23 = f2_add(oz2, f2_pack(Z.z, Z.w));
               const f32x2 q01 = f2_fma(rx01, rx01, f2_fma(ry01, ry01, f2_mul(rz01, rz01)));
               const f32x2 q23 = f2_fma(rx23, rx23, f2_fma(ry23, ry23, f2_mul(rz23, rz23)));
-              float r0, r1, r2, r3;
-              f2_unpack(q01, r0, r1);
-              f2_unpack(q23, r2, r3);
-              const unsigned nib = (r0 < rl2 ? 1u : 0u) | (r1 < rl2 ? 2u : 0u) | (r2 < rl2 ? 4u : 0u) |
-                                   (r3 < rl2 ? 8u : 0u);
-              hits |= nib << k;
+              float d0, d1, d2, d3;  // r^2 - rl^2, whose sign no rounding changes
+              f2_unpack(f2_add(q01, out2), d0, d1);
+              f2_unpack(f2_add(q23, out2), d2, d3);
+              hits = __funnelshift_l(__float_as_uint(d0), hits, 1);
+              hits = __funnelshift_l(__float_as_uint(d1), hits, 1);
+              hits = __funnelshift_l(__float_as_uint(d2), hits, 1);
+              hits = __funnelshift_l(__float_as_uint(d3), hits, 1);
             }
-#elif GBMD_LIST_UNROLL4
-            for (int k = 0; k < m; k += 4) {
-              unsigned nib = 0u;
-#pragma unroll
-              for (int u = 0; u < 4; ++u) {
-                const float4 gj = st[k + u];
-                const float rx = ox + gj.x, ry = oy + gj.y, rz = oz + gj.z;
-                const float r2 = fmaf(rx, rx, fmaf(ry, ry, rz * rz));
-                nib |= (r2 < rl2 ? 1u : 0u) << u;
-              }
-              hits |= nib << k;
-            }
-#else
-            for (int k = 0; k < m; ++k) {
-              const float4 gj = st[k];
-              const float rx = ox + gj.x, ry = oy + gj.y, rz = oz + gj.z;
-              const float r2 = fmaf(rx, rx, fmaf(ry, ry, rz * rz));
-              hits |= (r2 < rl2 ? 1u : 0u) << k;
-            }
-#endif
+            hits <<= 32 - ((m + 3) & ~3);
             const int self = li - jl0;  // drop the atom itself
-            if (self >= 0 && self < 32) hits &= ~(1u << self);
+            if (self >= 0 && self < 32) hits &= ~(0x80000000u >> self);
             // pass 2: append the hits in candidate order
             while (hits) {
-              const int k = __ffs(hits) - 1;
-              hits &= hits - 1u;
-#if GBMD_LIST_UNROLL4
+              const int k = __clz(hits);
+              hits ^= 0x80000000u >> k;
               // running write position: entry cnt of the atom lives at group cnt/4, slot cnt%4
               if (cnt < maxnb) *wp = code | (unsigned)(jl0 + k);
               wp += (cnt & 3) == 3 ? gstride - 3 : 1;
-#else
-              if (cnt < maxnb) out[(cnt >> 2) * gstride + (cnt & 3)] = code | (unsigned)(jl0 + k);
-#endif
               ++cnt;
             }
           }
@@ -574,10 +829,25 @@ __global__ void __launch_bounds__(32 * LIST_WARPS, GBMD_LIST_MIN_BLOCKS) k_build
     }
     if (has) {
       D.ncount[i] = cnt < maxnb ? cnt : maxnb;
-      atomicMax(&D.sst[s].max_count, cnt);
-      if (cnt > maxnb) atomicOr(&D.sst[s].error, ERR_LIST);
+      most = max(most, cnt);
     }
   }
+  most = (int)__reduce_max_sync(0xffffffffu, (unsigned)most);
+  if (lane == 0) {
+    if (most > *(volatile int*)&D.sst[s].max_count) atomicMax(&D.sst[s].max_count, most);
+    if (most > maxnb) atomicOr(&D.sst[s].error, ERR_LIST);
+  }
+}
+
+__global__ void __launch_bounds__(32 * LIST_CELLS, 4) k_buildlist_warp(Dev D) {
+  // coordinates staged as three arrays, so that one 16-byte shared load gives the x (y, z)
+  // of four consecutive candidates: two packed pairs
+  __shared__ __align__(16) float stage[LIST_CELLS][3][32];
+  const int w = threadIdx.x >> 5;
+  int s, c;
+  for (int u = blockIdx.x * LIST_CELLS + w; rebuild_unit<true>(D, u, s, c); u += gridDim.x * LIST_CELLS)
+    if (D.sysd[s].mode == NB_LIST && D.sysd[s].ncells > LIST_BLOCK_CELLS)
+      list_cell(D, D.sysd[s], s, c, stage[w][0], stage[w][1], stage[w][2]);
 }
 
 // ---------------------------------------------------------------------------------------------
