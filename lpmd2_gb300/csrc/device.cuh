@@ -227,10 +227,11 @@ __device__ __forceinline__ double ref_fitted(double v, double L) {
   return v;
 }
 
-// WrapAround (plugins/linkedcell.cc:9-15).
+// WrapAround (plugins/linkedcell.cc:9-15), whose result for a negative multiple of n is n itself: a
+// cell past the grid's last, taken as cell 0 here.
 __device__ __forceinline__ int wrap_around(int i, int n) {
   if (i < 0)
-    i += ((-i / n) + 1) * n;
+    i = i % n == 0 ? 0 : i + ((-i / n) + 1) * n;
   else if (i > n - 1)
     i -= (i / n) * n;
   return i;
