@@ -180,9 +180,10 @@ gbmd_status gbmd_sim_set_precision(gbmd_sim* sim, int precision);
  *   "time_kernels"     1: CUDA-event timing of every kernel class (graph_mode 0), see gbmd_stats
  *   "stream_priority"  1: the highest stream priority, 0: the lowest (default); replaces the
  *                      stream, so read gbmd_*_stream afterwards
- *   "lanes_per_atom"   mixed Lennard-Jones force pass: 1 (default), 2, 4, 8, 16 or 32 lanes
- *                      share an atom's neighbour list, i.e. 32 to 1 atoms per warp (same
- *                      forces bit for bit; for small systems)
+ *   "lanes_per_atom"   mixed Lennard-Jones force pass: 1, 2, 4, 8, 16 or 32 lanes share an
+ *                      atom's neighbour list, i.e. 32 to 1 atoms per warp (same forces,
+ *                      energies and virials bit for bit; stress moves by FP32 rounding).  Unset,
+ *                      as many as keep every block resident: 8 to 2 for small systems, else 1
  *   "list_feed"        how the mixed passes read their Verlet-list rows: 0 auto (default:
  *                      registers for a single EAM system, a shared-memory ring of bulk copies
  *                      otherwise), 1 registers, 2 ring (the same results either way) */

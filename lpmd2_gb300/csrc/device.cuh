@@ -112,6 +112,11 @@ struct Blk64 {
   short lanes, apw;
 };
 
+// One block of the mixed passes: `count` atoms of one system from `first` (TILE, or TILE / lanes).
+struct __align__(16) Blk32 {
+  int sys, first, count, pad;
+};
+
 struct Dev {
   long long N;
   // positions are double-buffered: (x, y, z, g32, g64) are the positions a launch evaluates
@@ -158,10 +163,6 @@ struct Dev {
   // multi-potential accumulation
   long long* facc;   // 3*N fixed point
   double* dacc;      // 3*N FP64
-  // SM-local tile claims of the mixed force and density passes: one counter per SM slot and a
-  // completion counter (claim_slots + 1 entries, zero between launches)
-  unsigned* tile_claim;
-  int claim_slots;
   // per-system cell-shift tables (128 float4 per system, entries 0..124 used) for the mixed
   // passes that read them from global memory instead of shared memory (GBMD_SHIFTS_GLOBAL)
   float4* shift_tab;
@@ -318,6 +319,23 @@ __device__ __forceinline__ T warp_sum(T v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
   return v;
+}
+
+// Sums 16 values per lane over the warp with 16 additions a lane: each exchange halves the values
+// a lane carries.  Lane l returns the total of value l >> 1.
+template <typename T>
+__device__ __forceinline__ T warp_sum16(T (&v)[16]) {
+  const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int h = 8, m = 16; h > 0; h >>= 1, m >>= 1) {
+    const bool up = (lane & m) != 0;
+#pragma unroll
+    for (int k = 0; k < h; ++k) {
+      const T keep = up ? v[k + h] : v[k], send = up ? v[k] : v[k + h];
+      v[k] = keep + __shfl_xor_sync(0xffffffffu, send, m);
+    }
+  }
+  return v[0] + __shfl_xor_sync(0xffffffffu, v[0], 1);
 }
 
 // Deterministic block sum of NV values per thread; thread 0 gets the totals in out[].

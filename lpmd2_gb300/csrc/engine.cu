@@ -279,7 +279,7 @@ struct Engine::Impl {
   double opt_skin = -1.0;
   int graph_block = 10;
   int graph_mode = 2;  // 0 direct, 1 captured, 2 captured with conditional rebuild
-  int lanes = 1;       // lanes per atom of the mixed LJ force pass
+  int lanes = 0;       // lanes per atom of the mixed pair passes (0: by the system's size)
   int list_feed = 0;   // list rows of the mixed passes: 0 auto, 1 registers, 2 ring
   int stencil_r = 1;
   int log_cap = 1024;
@@ -505,6 +505,54 @@ struct Engine::Impl {
     }
   }
 
+  // Lanes per atom of the mixed passes unless the option says otherwise: as many as leave all blocks
+  // resident at once (8 a SM), 8 only to half of that.  Measured, force pass of an LJ liquid with 1 /
+  // 2 / 4 / 8 lanes (us): 4,000 atoms 23.7 / - / 11.5 / 10.8, 16,384 24.7 / 17.6 / 14.3 / 15.3,
+  // 32,000 26.4 / 19.8 / 17.5 / 26.6, 55,296 30.0 / 24.6 / 30.6 / 39.3, 78,732 37.5 / 40.4 / 41.0 / 55.1;
+  // a second round of blocks costs what the lanes saved.  Forces, energies and virials do not depend
+  // on the lanes, stress by its FP32 rounding.
+  int auto_lanes() const {
+    for (int lanes : {8, 4, 2}) {
+      long long blocks = 0;
+      for (int s = 0; s < nsys; ++s) blocks += (natoms[s] * lanes + TILE - 1) / TILE;
+      if (blocks <= (lanes == 8 ? 4 : 8) * (long long)sm_count) return lanes;
+    }
+    return 1;
+  }
+  int sm_count = 1;
+
+  // Blocks of the mixed passes.
+  struct Plan32 {
+    int lanes = 0, n = 0;
+    Blk32* blk = nullptr;
+  };
+  Plan32 plan_pair, plan_eam;  // the option lanes_per_atom sets the pair passes' lanes
+  int planned_lanes = -1;
+
+  void make_plan32(Plan32& plan, int lanes_per_atom) {
+    std::vector<Blk32> blk;
+    const int apb = TILE / lanes_per_atom;
+    for (int s = 0; s < nsys; ++s) {
+      for (long long k = 0; k < natoms[s]; k += apb)
+        blk.push_back({s, (int)(atom_base[s] + k), (int)std::min<long long>(apb, natoms[s] - k), 0});
+    }
+    plan.lanes = lanes_per_atom;
+    plan.n = (int)blk.size();
+    if (plan.blk) dev_free(plan.blk);
+    plan.blk = nullptr;
+    CK(dev_malloc(&plan.blk, sizeof(Blk32) * std::max<size_t>(blk.size(), 1)));
+    CK(cudaMemcpyAsync(plan.blk, blk.data(), sizeof(Blk32) * blk.size(), cudaMemcpyHostToDevice, stream));
+    CK(cudaStreamSynchronize(stream));
+  }
+  void ensure_plan32() {
+    if (planned_lanes == lanes) return;
+    CK(cudaStreamSynchronize(stream));
+    drop_graph();
+    make_plan32(plan_pair, lanes ? lanes : auto_lanes());
+    make_plan32(plan_eam, auto_lanes());
+    planned_lanes = lanes;
+  }
+
   // Block table and partial sums of the FP64 passes.
   void alloc_blocks64() {
     std::vector<Blk64> blk;
@@ -661,10 +709,10 @@ struct Engine::Impl {
     D.dacc = alloc<double>(3 * n);
     tile_part = alloc<double>((size_t)ntiles * PART_D);
     {
-      int nsm = 0;
-      CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, device));
-      D.claim_slots = nsm > 0 ? nsm : 1;
-      D.tile_claim = alloc<unsigned>((size_t)D.claim_slots + 1);  // zeroed
+      // a word per SM and one more that nothing reads any more: part of the layout of saved snapshots
+      CK(cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, device));
+      if (sm_count < 1) sm_count = 1;
+      alloc<unsigned>((size_t)sm_count + 1);
     }
     D.shift_tab = alloc<float4>((size_t)nsys * 128);
     D.sys_acc = alloc<unsigned long long>((size_t)nsys * SA_LEN);
@@ -755,6 +803,8 @@ struct Engine::Impl {
     for (auto& a : allocs) dev_free(a.first);
     free_scratch();
     for (auto& a : work) dev_free(a.first);
+    if (plan_pair.blk) dev_free(plan_pair.blk);
+    if (plan_eam.blk) dev_free(plan_eam.blk);
     free_cells();
     if (stream) cudaStreamDestroy(stream);
     if (stream2) cudaStreamDestroy(stream2);
@@ -890,6 +940,7 @@ struct Engine::Impl {
     free_cells();
     free_scratch();
     if (precision == PREC_FP64) alloc_blocks64();
+    planned_lanes = -1;
     alloc_cells(total_cells);
     int maxnb = 0;
     if (any_list) {
@@ -1037,49 +1088,23 @@ struct Engine::Impl {
       const bool ring = list_feed == 2 || (list_feed == 0 && (nsys > 1 || pair_kind(P.kind)));
       if (!pair_kind(P.kind)) {
         int first = (p == first_eam);
-        if (mixed && P.kind == POT_SC && P.int_m == 6)
-          ring ? k_eam_density32<6, FEED_RING><<<ntiles, TILE, 0, s>>>(D, Pe)
-               : k_eam_density32<6, FEED_REGS><<<ntiles, TILE, 0, s>>>(D, Pe);
-        else if (mixed)
-          ring ? k_eam_density32<0, FEED_RING><<<ntiles, TILE, 0, s>>>(D, Pe)
-               : k_eam_density32<0, FEED_REGS><<<ntiles, TILE, 0, s>>>(D, Pe);
+        if (mixed)
+          launch_density32(s, Pe, ring);
         else
           launch_density64(s, P, mode, first);
         launched();
       }
       if (mixed) {
-        if (pair_kind(P.kind) && lanes > 1) {
-          const unsigned g = (unsigned)ntiles * lanes;
-          if (lanes == 2)
-            species ? k_force32_lanes<1, 2><<<g, TILE, 0, s>>>(D, P, sp) : k_force32_lanes<0, 2><<<g, TILE, 0, s>>>(D, P, sp);
-          else if (lanes == 4)
-            species ? k_force32_lanes<1, 4><<<g, TILE, 0, s>>>(D, P, sp) : k_force32_lanes<0, 4><<<g, TILE, 0, s>>>(D, P, sp);
-          else if (lanes == 8)
-            species ? k_force32_lanes<1, 8><<<g, TILE, 0, s>>>(D, P, sp) : k_force32_lanes<0, 8><<<g, TILE, 0, s>>>(D, P, sp);
-          else if (lanes == 16)
-            species ? k_force32_lanes<1, 16><<<g, TILE, 0, s>>>(D, P, sp) : k_force32_lanes<0, 16><<<g, TILE, 0, s>>>(D, P, sp);
-          else
-            species ? k_force32_lanes<1, 32><<<g, TILE, 0, s>>>(D, P, sp) : k_force32_lanes<0, 32><<<g, TILE, 0, s>>>(D, P, sp);
-        } else if (pair_kind(P.kind)) {
-          if (species)
-            ring ? k_force32<PC_PAIR, 1, 0, 0, FEED_RING><<<ntiles, TILE, 0, s>>>(D, P, sp)
-                 : k_force32<PC_PAIR, 1, 0, 0, FEED_REGS><<<ntiles, TILE, 0, s>>>(D, P, sp);
-          else
-            ring ? k_force32<PC_PAIR, 0, 0, 0, FEED_RING><<<ntiles, TILE, 0, s>>>(D, P, sp)
-                 : k_force32<PC_PAIR, 0, 0, 0, FEED_REGS><<<ntiles, TILE, 0, s>>>(D, P, sp);
+        if (pair_kind(P.kind)) {
+          species ? launch_force32<PC_PAIR, 1, 0, 0>(s, P, sp, ring) : launch_force32<PC_PAIR, 0, 0, 0>(s, P, sp, ring);
+        } else if (species) {
+          launch_force32<PC_EAM, 1, 0, 0>(s, Pe, sp, ring);
+        } else if (sc96) {
+          launch_force32<PC_EAM, 0, 9, 6>(s, Pe, sp, ring);
+        } else if (sc126) {
+          launch_force32<PC_EAM, 0, 12, 6>(s, Pe, sp, ring);
         } else {
-          if (species)
-            ring ? k_force32<PC_EAM, 1, 0, 0, FEED_RING><<<ntiles, TILE, 0, s>>>(D, Pe, sp)
-                 : k_force32<PC_EAM, 1, 0, 0, FEED_REGS><<<ntiles, TILE, 0, s>>>(D, Pe, sp);
-          else if (sc96)
-            ring ? k_force32<PC_EAM, 0, 9, 6, FEED_RING><<<ntiles, TILE, 0, s>>>(D, Pe, sp)
-                 : k_force32<PC_EAM, 0, 9, 6, FEED_REGS><<<ntiles, TILE, 0, s>>>(D, Pe, sp);
-          else if (sc126)
-            ring ? k_force32<PC_EAM, 0, 12, 6, FEED_RING><<<ntiles, TILE, 0, s>>>(D, Pe, sp)
-                 : k_force32<PC_EAM, 0, 12, 6, FEED_REGS><<<ntiles, TILE, 0, s>>>(D, Pe, sp);
-          else
-            ring ? k_force32<PC_EAM, 0, 0, 0, FEED_RING><<<ntiles, TILE, 0, s>>>(D, Pe, sp)
-                 : k_force32<PC_EAM, 0, 0, 0, FEED_REGS><<<ntiles, TILE, 0, s>>>(D, Pe, sp);
+          launch_force32<PC_EAM, 0, 0, 0>(s, Pe, sp, ring);
         }
       } else if (nblk64 > 0) {
         launch_force64(s, P, sp, mode);
@@ -1093,6 +1118,51 @@ struct Engine::Impl {
     else
       k_thermo<<<dim3(nsys, shares64), PART_D * THERMO_ROWS, 0, s>>>(D, count_step, decide_next, (unsigned long long)cond_next);
     launched();
+  }
+
+  template <int PC, int SPECIES, int SCN, int SCM>
+  void launch_force32(cudaStream_t s, const PotParams& P, const StepParams& sp, bool ring) {
+    const Plan32& plan = PC == PC_PAIR ? plan_pair : plan_eam;
+    const int n = plan.n;
+    const Blk32* b = plan.blk;
+    if (plan.lanes == 1) {
+      if (ring)
+        k_force32<PC, SPECIES, SCN, SCM, FEED_RING><<<n, TILE, 0, s>>>(D, P, sp, b);
+      else
+        k_force32<PC, SPECIES, SCN, SCM, FEED_REGS><<<n, TILE, 0, s>>>(D, P, sp, b);
+    } else if (plan.lanes == 4) {
+      k_force32_lanes<PC, SPECIES, SCN, SCM, 4><<<n, TILE, 0, s>>>(D, P, sp, b);
+    } else if (plan.lanes == 8) {
+      k_force32_lanes<PC, SPECIES, SCN, SCM, 8><<<n, TILE, 0, s>>>(D, P, sp, b);
+    } else if (plan.lanes == 2) {
+      k_force32_lanes<PC, SPECIES, SCN, SCM, 2><<<n, TILE, 0, s>>>(D, P, sp, b);
+    } else if constexpr (PC == PC_PAIR) {  // by the option alone
+      if (plan.lanes == 16)
+        k_force32_lanes<PC, SPECIES, SCN, SCM, 16><<<n, TILE, 0, s>>>(D, P, sp, b);
+      else
+        k_force32_lanes<PC, SPECIES, SCN, SCM, 32><<<n, TILE, 0, s>>>(D, P, sp, b);
+    }
+  }
+
+  template <int SCM>
+  void launch_density32_m(cudaStream_t s, const PotParams& P, bool ring) {
+    const Plan32& plan = plan_eam;
+    if (plan.lanes == 8)
+      k_eam_density32_lanes<SCM, 8><<<plan.n, TILE, 0, s>>>(D, P, plan.blk);
+    else if (plan.lanes == 4)
+      k_eam_density32_lanes<SCM, 4><<<plan.n, TILE, 0, s>>>(D, P, plan.blk);
+    else if (plan.lanes == 2)
+      k_eam_density32_lanes<SCM, 2><<<plan.n, TILE, 0, s>>>(D, P, plan.blk);
+    else if (ring)
+      k_eam_density32<SCM, FEED_RING><<<plan.n, TILE, 0, s>>>(D, P, plan.blk);
+    else
+      k_eam_density32<SCM, FEED_REGS><<<plan.n, TILE, 0, s>>>(D, P, plan.blk);
+  }
+  void launch_density32(cudaStream_t s, const PotParams& P, bool ring) {
+    if (P.kind == POT_SC && P.int_m == 6)
+      launch_density32_m<6>(s, P, ring);
+    else
+      launch_density32_m<0>(s, P, ring);
   }
 
   void launch_density64(cudaStream_t s, const PotParams& P, int mode, int first) {
@@ -1142,6 +1212,7 @@ struct Engine::Impl {
                        "table bin): use precision fp64");
     if (!configured) configure();
     CK(cudaSetDevice(device));
+    if (precision == PREC_MIXED) ensure_plan32();
     if (!D.g32e && precision == PREC_MIXED)
       for (const auto& P : pots)
         if (!pair_kind(P.kind)) {

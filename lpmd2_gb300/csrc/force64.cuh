@@ -228,22 +228,6 @@ __device__ __forceinline__ double atom_sum3(double x, double y, double z, int su
   return c;
 }
 
-// Sums 16 values per lane over the warp with 16 additions a lane: each exchange halves the values
-// a lane carries.  Lane l returns the total of value l >> 1.
-__device__ __forceinline__ double warp_sum16(double (&v)[16]) {
-  const int lane = threadIdx.x & 31;
-#pragma unroll
-  for (int h = 8, m = 16; h > 0; h >>= 1, m >>= 1) {
-    const bool up = (lane & m) != 0;
-#pragma unroll
-    for (int k = 0; k < h; ++k) {
-      const double keep = up ? v[k + h] : v[k], send = up ? v[k] : v[k + h];
-      v[k] = keep + __shfl_xor_sync(0xffffffffu, send, m);
-    }
-  }
-  return v[0] + __shfl_xor_sync(0xffffffffu, v[0], 1);
-}
-
 // The candidates of one atom (the calling lane's), tested in FP32 and queued: entry = local index of
 // j, plus Q64_EXACT where the FP64 test has to decide.  All lanes of the warp call this together;
 // the lanes of an atom share its queue `q` of cap entries: those with j > i from the front, the

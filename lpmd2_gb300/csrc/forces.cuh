@@ -378,67 +378,19 @@ __device__ __forceinline__ void warp_list_prefetch2(const Dev& D, const SysDev& 
 // with the ring.
 constexpr int FEED_REGS = 0, FEED_RING = 1;
 
-// Tile of a block of the mixed force and density passes: blockIdx.x, or with GBMD_SM_TILES=1 a
-// tile claimed from a contiguous range per SM (a block takes the next tile of the range of the
-// SM it runs on, of the next SM's once that range is used up), so that the blocks resident on an
-// SM at the same time work on neighbouring cells and share their neighbours' positions in L1.
-// Every block gets exactly one tile: a launch has as many blocks as tiles, each block claims at
-// most one, and a block that scanned every range without success would mean that the other
-// blocks had claimed all tiles.  The last block of a launch to finish zeroes the counters.
-// Measured on the GB300 (results bitwise equal): LJ force pass 150 us against 93 us with
-// blockIdx.x, copper density + force 0.590 against 0.480 ms, so the claim is off by default.
-#ifndef GBMD_SM_TILES
-#define GBMD_SM_TILES 0
-#endif
-__device__ __forceinline__ int claim_tile(const Dev& D) {
-#if GBMD_SM_TILES
-  __shared__ int s_tile;
-  if (threadIdx.x == 0) {
-    unsigned smid;
-    asm volatile("mov.u32 %0, %%smid;" : "=r"(smid));
-    const int P = D.claim_slots, T = (int)gridDim.x;
-    int k = (int)(smid % (unsigned)P), tile = -1;
-    for (int probe = 0; probe < P && tile < 0; ++probe) {
-      const int lo = (int)((long long)T * k / P), n = (int)((long long)T * (k + 1) / P) - lo;
-      if (n > 0 && (int)__ldcg(D.tile_claim + k) < n) {
-        const int idx = (int)atomicAdd(D.tile_claim + k, 1u);
-        if (idx < n) tile = lo + idx;
-      }
-      k = (k + 1 == P) ? 0 : k + 1;
-    }
-    s_tile = tile;
-  }
-  __syncthreads();
-  return s_tile;
-#else
-  return (int)blockIdx.x;
-#endif
-}
-__device__ __forceinline__ void release_tile(const Dev& D) {
-#if GBMD_SM_TILES
-  if (threadIdx.x == 0) {
-    __threadfence();
-    if (atomicAdd(D.tile_claim + D.claim_slots, 1u) == gridDim.x - 1) {
-      for (int k = 0; k <= D.claim_slots; ++k) D.tile_claim[k] = 0u;
-      __threadfence();
-    }
-  }
-#endif
-}
-
 template <int PC, int SPECIES, int SCN, int SCM, int FEED>
-__device__ __forceinline__ void force32_tile(const Dev& D, const PotParams& P, const StepParams& sp, const int tile) {
-  const int s = D.tile_sys[tile];
+__device__ __forceinline__ void force32_tile(const Dev& D, const PotParams& P, const StepParams& sp, const Blk32 B) {
+  const int s = B.sys;
   const SysDev& S = D.sysd[s];
-  if (!S.active) {  // whole block: one tile belongs to one system
-    if (sp.epi == EPI_KICK_DRIFT && sp.last) hold_tile(D, S, tile, true);
+  if (!S.active) {  // whole block: its atoms belong to one system
+    if (sp.epi == EPI_KICK_DRIFT && sp.last) hold_range(D, S, B.first, B.count, true);
     return;
   }
   SHIFT_TABLE(shifts);
   const ShiftCorr corr = shift_corr(S);
-  const int li = D.tile_first[tile] - (int)S.atom_base + (int)threadIdx.x;  // index within the system
+  const int li = B.first - (int)S.atom_base + (int)threadIdx.x;  // index within the system
   const long long i = S.atom_base + li;
-  const bool active = (int)threadIdx.x < D.tile_count[tile];
+  const bool active = (int)threadIdx.x < B.count;
   const float4* __restrict__ g32 = D.g32 + S.atom_base;
   // EAM without a species filter gathers the density pass's copy, whose w holds the
   // neighbour's embedding factor (one 16-byte gather per pair instead of 16 + 4 bytes)
@@ -595,8 +547,8 @@ __device__ __forceinline__ void force32_tile(const Dev& D, const PotParams& P, c
       bad |= fmaxf(fabsf(gx), fmaxf(fabsf(gy), fabsf(gz))) > 4000.0f;
     };
     const int ngw = __reduce_max_sync(0xffffffffu, (unsigned)ng);
-    const int wfirst = D.tile_first[tile] - (int)S.atom_base + 32 * w;
-    const int wcount = min(32, max(0, D.tile_count[tile] - 32 * w));
+    const int wfirst = B.first - (int)S.atom_base + 32 * w;
+    const int wcount = min(32, max(0, B.count - 32 * w));
     bool waited = true;
     if constexpr (FEED == FEED_REGS &&
                   ((PC == PC_PAIR && GBMD_PAIR_RING_GROUPS == 2) || (PC == PC_EAM && GBMD_EAM_RING_GROUPS == 2))) {
@@ -738,96 +690,129 @@ __device__ __forceinline__ void force32_tile(const Dev& D, const PotParams& P, c
 
 
 template <int PC, int SPECIES, int SCN = 0, int SCM = 0, int FEED = FEED_REGS>
-__global__ void __launch_bounds__(TILE, GBMD_FORCE_MIN_BLOCKS) k_force32(Dev D, PotParams P, StepParams sp) {
-  const int tile = claim_tile(D);
-  if (tile >= 0) force32_tile<PC, SPECIES, SCN, SCM, FEED>(D, P, sp, tile);
-  release_tile(D);
+__global__ void __launch_bounds__(TILE, GBMD_FORCE_MIN_BLOCKS) k_force32(Dev D, PotParams P, StepParams sp, const Blk32* blk) {
+  force32_tile<PC, SPECIES, SCN, SCM, FEED>(D, P, sp, blk[blockIdx.x]);
 }
 
 // ------------------------------------------------------------------------------------------
-// Mixed LJ force pass with LANES lanes per atom (LANES = 2, 4, 8: 16, 8 or 4 atoms per warp),
-// for systems too small to fill the GPU one lane per atom.  The atom's list groups go
-// round-robin to its lanes (plain cached loads instead of the bulk-copy ring); each group is
-// evaluated and summed exactly as in k_force32, and the lanes' fixed-point partials are
-// combined with integer shuffles, so the forces are bitwise those of k_force32.  Energy and
-// stress partials are rounded to fixed point per lane (a 2^-32 eV-scale difference).  A tile
-// of 128 atoms is spread over LANES blocks of 128 threads.
+// Mixed force pass with LANES lanes per atom (TILE / LANES atoms a block), for systems too small to
+// fill the GPU one lane per atom: there a warp's time is its own chain of some ten iterations of
+// gathers and arithmetic (24 us for 4,000 and for 16,384 atoms of LJ liquid alike, 11 and 14 here),
+// which LANES lanes cut to two or three.  The atom's list groups go round-robin to its lanes (plain
+// cached loads); each group is evaluated and summed exactly as in k_force32, and the lanes'
+// fixed-point partials are combined with integer shuffles, so forces, energy and virial are bitwise
+// those of k_force32; stress is rounded to fixed point per lane.  The per-atom epilogue -- FP64
+// instructions, as long for one atom as for 32 -- runs one thread per atom in as few warps as hold
+// the block's atoms (in every warp, with a few lanes at work, it took longer than the pairs: 15.1 us
+// at 4 lanes and 16,384 atoms, 14.3 so; 20 and 15.3 at 8).
 // ------------------------------------------------------------------------------------------
 
-template <int SPECIES, int LANES>
-__global__ void __launch_bounds__(TILE, GBMD_FORCE_MIN_BLOCKS) k_force32_lanes(Dev D, PotParams P, StepParams sp) {
-  __shared__ float4 shifts[125];
+// g and pair energy of one entry; qi, qj: the embedding factors (metals), folded: times the prefactor.
+template <int PC, bool FOLDED, int SCN, int SCM>
+__device__ __forceinline__ void pair32(const PotParams& P, float r2, float qi, float qj, float& g, float& en) {
+  if constexpr (PC == PC_PAIR)
+    lj_pair32(P, rcp_approx(r2), g, en);
+  else if constexpr (FOLDED)
+    eam_sc_pair32_q<SCN, SCM>(P, r2, qi, qj, g, en);
+  else
+    eam_pair32_t<SCN, SCM>(P, r2, qi, qj, g, en);
+}
+
+// Sum of an atom's fixed-point partials over its LANES adjacent lanes.
+template <int LANES>
+__device__ __forceinline__ void lanes_sum(Fix& f) {
+#pragma unroll
+  for (int m = 1; m < LANES; m <<= 1) {
+    f.hi += __shfl_xor_sync(0xffffffffu, f.hi, m);
+    f.lo += __shfl_xor_sync(0xffffffffu, f.lo, m);
+  }
+}
+
+template <int PC, int SPECIES, int SCN, int SCM, int LANES>
+__global__ void __launch_bounds__(TILE, 8)
+    k_force32_lanes(Dev D, PotParams P, StepParams sp, const Blk32* blk) {
   constexpr int APB = TILE / LANES;  // atoms per block
-  const int tile = blockIdx.x / LANES, part = blockIdx.x % LANES;
-  const int s = D.tile_sys[tile];
+  __shared__ float4 shifts[125];
+  __shared__ long long fsum[3][APB];
+  __shared__ long long esum[TILE / 32][16];
+  const Blk32 B = blk[blockIdx.x];
+  const int s = B.sys;
   const SysDev& S = D.sysd[s];
-  if (!S.active) {  // whole block: one tile belongs to one system
-    if (part == 0 && sp.epi == EPI_KICK_DRIFT && sp.last) hold_tile(D, S, tile, true);
+  if (!S.active) {  // whole block: its atoms belong to one system
+    if (sp.epi == EPI_KICK_DRIFT && sp.last) hold_range(D, S, B.first, B.count, true);
     return;
   }
   load_shifts(S, shifts);
   const ShiftCorr corr = shift_corr(S);
-  const int sub = threadIdx.x % LANES;
-  const int slot = part * APB + (int)threadIdx.x / LANES;  // atom within the tile
-  const int li = D.tile_first[tile] - (int)S.atom_base + slot;
-  const long long i = S.atom_base + li;
-  const bool active = slot < D.tile_count[tile];
+  const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int sub = threadIdx.x % LANES, slot = (int)threadIdx.x / LANES;
   const float4* __restrict__ g32 = D.g32 + S.atom_base;
-  Fix fqx, fqy, fqz, fqe, fqv;
-  float sxx = 0.f, sxy = 0.f, sxz = 0.f, syy = 0.f, syz = 0.f, szz = 0.f;
+  // as in k_force32: metals without a species filter gather the embedding factor with the position
+  constexpr bool PHI_IN_W = PC == PC_EAM && !SPECIES;
+  constexpr bool FOLDED = PHI_IN_W && SCN > 0;
+  const float4* __restrict__ gsrc = PHI_IN_W ? D.g32e + S.atom_base : g32;
   const float rc2_lo = P.f[12], rc2_hi = P.f[13];
+  const float ms = (float)(-0.5 * FIX_E);
   unsigned rechecks = 0;
   bool bad = false;
+  Fix fqe, fqv;
+  const bool active = slot < B.count;
+  const int li = B.first - (int)S.atom_base + (active ? slot : 0);
+  const long long i = S.atom_base + li;
+  Fix fqx, fqy, fqz;
+  float sxx = 0.f, sxy = 0.f, sxz = 0.f, syy = 0.f, syz = 0.f, szz = 0.f;
   const float4 gi = active ? g32[li] : make_float4(0.f, 0.f, 0.f, 0.f);
   const int ti = __float_as_int(gi.w);
+  const float phi_i = (PC == PC_EAM && active) ? (PHI_IN_W ? gsrc[li].w : D.phif[i]) : 0.f;
   const int na = S.natoms;
   const int cnt = active ? D.ncount[i] : 0;
   const int ng = (cnt + 3) >> 2;
   constexpr unsigned NO_BAND = 0xffffffffu;
   unsigned band_e = NO_BAND;
   bool band_more = false;
-  float ge = 0.f, gv = 0.f;
-  auto pair = [&](unsigned e, bool valid, float& dx, float& dy, float& dz) -> float {
-    const int j = (int)(e & LOCAL_MASK);
-    const float4 gj = g32[j];
-    const float r2 = entry_r2(gi, gj, shifts[e >> CODE_SHIFT], corr, dx, dy, dz);
-    bool in = valid && r2 < rc2_lo;
-    if (valid && r2 >= rc2_lo && r2 < rc2_hi) {
-      if (band_e == NO_BAND)
-        band_e = e;
-      else
-        band_more = true;
-    }
-    if (SPECIES) in = in && applies_to(P.spc_sum, ti, __float_as_int(gj.w));
-    float g, en;
-    lj_pair32(P, rcp_approx(r2), g, en);
-    g = in ? g : 0.0f;
-    ge += in ? en : 0.0f;
-    gv = fmaf(g, r2, gv);
-    const float fx = g * dx, fy = g * dy, fz = g * dz;
-    sxx = fmaf(fx, dx, sxx);
-    sxy = fmaf(fx, dy, sxy);
-    sxz = fmaf(fx, dz, sxz);
-    syy = fmaf(fy, dy, syy);
-    syz = fmaf(fy, dz, syz);
-    szz = fmaf(fz, dz, szz);
-    return g;
-  };
   const uint4* L = active ? list_group(D, S, li, 0) : nullptr;
   for (int q = sub; q < ng; q += LANES) {
     const uint4 cur = __ldg(L + (long long)q * na);
+    const unsigned e[4] = {cur.x, cur.y, cur.z, cur.w};
     const int rem = cnt - 4 * q;
-    ge = 0.f;
-    gv = 0.f;
-    float ax, ay, az, bx, by, bz;
-    float g0 = pair(cur.x, true, ax, ay, az);
-    float g1 = pair(cur.y, rem > 1, bx, by, bz);
-    float gx = fmaf(g1, bx, g0 * ax), gy = fmaf(g1, by, g0 * ay), gz = fmaf(g1, bz, g0 * az);
-    g0 = pair(cur.z, rem > 2, ax, ay, az);
-    g1 = pair(cur.w, rem > 3, bx, by, bz);
-    gx = fmaf(g1, bx, fmaf(g0, ax, gx));
-    gy = fmaf(g1, by, fmaf(g0, ay, gy));
-    gz = fmaf(g1, bz, fmaf(g0, az, gz));
+    float4 gj[4];
+    float pj[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      gj[u] = gsrc[e[u] & LOCAL_MASK];
+      pj[u] = (PC == PC_EAM && !PHI_IN_W) ? D.phif[S.atom_base + (e[u] & LOCAL_MASK)] : gj[u].w;
+    }
+    float ge = 0.f, gv = 0.f, gx = 0.f, gy = 0.f, gz = 0.f;
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const bool valid = u == 0 || rem > u;
+      float dx, dy, dz;
+      const float r2 = entry_r2(gi, gj[u], shifts[e[u] >> CODE_SHIFT], corr, dx, dy, dz);
+      bool in = valid && r2 < rc2_lo;
+      if (valid && r2 >= rc2_lo && r2 < rc2_hi) {  // guard band: decided in FP64 after the loop
+        if (band_e == NO_BAND)
+          band_e = e[u];
+        else
+          band_more = true;
+      }
+      if (SPECIES) in = in && applies_to(P.spc_sum, ti, __float_as_int(gj[u].w));
+      float g, en;
+      pair32<PC, FOLDED, SCN, SCM>(P, r2, phi_i, pj[u], g, en);
+      g = in ? g : 0.0f;
+      ge += in ? en : 0.0f;
+      gv = fmaf(g, r2, gv);
+      const float fx = g * dx, fy = g * dy, fz = g * dz;
+      sxx = fmaf(fx, dx, sxx);
+      sxy = fmaf(fx, dy, sxy);
+      sxz = fmaf(fx, dz, sxz);
+      syy = fmaf(fy, dy, syy);
+      syz = fmaf(fy, dz, syz);
+      szz = fmaf(fz, dz, szz);
+      // the group's force in k_force32's order: ((g0 d0 + g1 d1) + g2 d2) + g3 d3, fused
+      gx = u == 0 ? g * dx : fmaf(g, dx, gx);
+      gy = u == 0 ? g * dy : fmaf(g, dy, gy);
+      gz = u == 0 ? g * dz : fmaf(g, dz, gz);
+    }
     fqx.add_scaled32(gx);
     fqy.add_scaled32(gy);
     fqz.add_scaled32(gz);
@@ -846,7 +831,10 @@ __global__ void __launch_bounds__(TILE, GBMD_FORCE_MIN_BLOCKS) k_force32_lanes(D
       if (!exact_inside_cold(&D, &S, i, S.atom_base + j, P.rc2)) return;
       if (SPECIES && !applies_to(P.spc_sum, ti, __float_as_int(gj.w))) return;
       float g, en;
-      lj_pair32(P, rcp_approx(r2), g, en);
+      if (PC == PC_PAIR)
+        lj_pair32(P, rcp_approx(r2), g, en);
+      else  // the unscaled embedding factors of both atoms (rare path)
+        eam_pair32_t<SCN, SCM>(P, r2, D.phif[i], D.phif[S.atom_base + j], g, en);
       const float fx = g * dx, fy = g * dy, fz = g * dz;
       fqx.add_scaled32(fx);
       fqy.add_scaled32(fy);
@@ -874,60 +862,63 @@ __global__ void __launch_bounds__(TILE, GBMD_FORCE_MIN_BLOCKS) k_force32_lanes(D
       }
     }
   }
-  // the atom's lanes are adjacent: exact integer sums of the fixed-point partials
-#pragma unroll
-  for (int m = 1; m < LANES; m <<= 1) {
-    fqx.hi += __shfl_xor_sync(0xffffffffu, fqx.hi, m);
-    fqx.lo += __shfl_xor_sync(0xffffffffu, fqx.lo, m);
-    fqy.hi += __shfl_xor_sync(0xffffffffu, fqy.hi, m);
-    fqy.lo += __shfl_xor_sync(0xffffffffu, fqy.lo, m);
-    fqz.hi += __shfl_xor_sync(0xffffffffu, fqz.hi, m);
-    fqz.lo += __shfl_xor_sync(0xffffffffu, fqz.lo, m);
+  lanes_sum<LANES>(fqx);
+  lanes_sum<LANES>(fqy);
+  lanes_sum<LANES>(fqz);
+  if (sub == 0 && active) {
+    fsum[0][slot] = fqx.value();
+    fsum[1][slot] = fqy.value();
+    fsum[2][slot] = fqz.value();
   }
+  if (rechecks) atomicAdd(&D.sst[s].rechecks, (unsigned long long)rechecks);
+  if (bad) atomicOr(&D.sst[s].error, ERR_FIXED);
+  // energy and virial: every lane's own fixed-point partial (exact integer sums, whatever the lane
+  // count)
+  long long v[16] = {fqe.value() * 64, fqv.value() * 64, fix64(sxx * ms), fix64(sxy * ms), fix64(sxz * ms),
+                     fix64(syy * ms), fix64(syz * ms), fix64(szz * ms), 0, 0, 0, 0, 0, 0, 0, 0};
+  const long long t16 = warp_sum16(v);
+  if ((lane & 1) == 0) esum[w][lane >> 1] = t16;
+  __syncthreads();
+  unsigned long long* acc = D.sys_acc + (long long)s * SA_LEN;
+  if (threadIdx.x >= TILE - 32 && lane < 11) {
+    // energy, virial and the nine stress slots from the eight sums (in the last warp: the first ones
+    // go on with the atoms)
+    const int from[11] = {0, 1, 2, 3, 4, 3, 5, 6, 4, 6, 7};
+    int f = 0;
+#pragma unroll
+    for (int k = 0; k < 11; ++k)
+      if (lane == k) f = from[k];
+    long long t = 0;
+    for (int k = 0; k < TILE / 32; ++k) t += esum[k][f];
+    atomicAdd(acc + lane, (unsigned long long)t);
+  }
+  const int t = threadIdx.x;
+  if (t >= ((B.count + 31) & ~31)) return;  // whole warps
   double ke = 0.0, px = 0.0, py = 0.0, pz = 0.0;
   float d2 = 0.0f;
-  if (active && sub == 0) {
-    const long long N = D.N;
-    long long qx = fqx.value(), qy = fqy.value(), qz = fqz.value();
+  if (t < B.count) {
+    const long long a = B.first + t, N = D.N;
+    long long qx = fsum[0][t], qy = fsum[1][t], qz = fsum[2][t];
     if (!sp.first) {
-      qx += D.facc[i];
-      qy += D.facc[N + i];
-      qz += D.facc[2 * N + i];
+      qx += D.facc[a];
+      qy += D.facc[N + a];
+      qz += D.facc[2 * N + a];
     }
     if (sp.last) {
-      d2 = finish_atom<1>(D, S, i, (double)qx, (double)qy, (double)qz, sp, ke, px, py, pz);
+      d2 = finish_atom<1>(D, S, a, (double)qx, (double)qy, (double)qz, sp, ke, px, py, pz);
     } else {
-      D.facc[i] = qx;
-      D.facc[N + i] = qy;
-      D.facc[2 * N + i] = qz;
+      D.facc[a] = qx;
+      D.facc[N + a] = qy;
+      D.facc[2 * N + a] = qz;
     }
   }
-  if (active) {
-    if (rechecks) atomicAdd(&D.sst[s].rechecks, (unsigned long long)rechecks);
-    if (bad) atomicOr(&D.sst[s].error, ERR_FIXED);
-  }
   track_displacement_warp(D, s, d2);
-  // energy and virial: every lane's own fixed-point partial (exact integer block sums), so they
-  // do not depend on the lane count; stress rounded per lane
-  const float ms = (float)(-0.5 * FIX_E);
-  long long v[11] = {fqe.value() * 64, fqv.value() * 64, fix64(sxx * ms), fix64(sxy * ms), fix64(sxz * ms),
-                     fix64(sxy * ms), fix64(syy * ms), fix64(syz * ms), fix64(sxz * ms), fix64(syz * ms),
-                     fix64(szz * ms)};
-  long long tot[11];
-  block_sum<long long, 11>(v, tot);
-  if (threadIdx.x == 0) {
-    unsigned long long* acc = D.sys_acc + (long long)s * SA_LEN;
-    for (int k = 0; k < 11; ++k) atomicAdd(acc + k, (unsigned long long)tot[k]);
-  }
   if (sp.last) {
     long long k4[4];
     warp_kinetic_fix(ke, px, py, pz, k4);
-    long long kt[4];
-    block_sum<long long, 4>(k4, kt);
-    if (threadIdx.x == 0) {
-      unsigned long long* acc = D.sys_acc + (long long)s * SA_LEN;
-      atomicAdd(acc + SA_KE, (unsigned long long)kt[0]);
-      for (int k = 0; k < 3; ++k) atomicAdd(acc + SA_P + k, (unsigned long long)kt[1 + k]);
+    if (lane == 0) {
+      atomicAdd(acc + SA_KE, (unsigned long long)k4[0]);
+      for (int k = 0; k < 3; ++k) atomicAdd(acc + SA_P + k, (unsigned long long)k4[1 + k]);
     }
   }
 }
@@ -940,17 +931,17 @@ __global__ void __launch_bounds__(TILE, GBMD_FORCE_MIN_BLOCKS) k_force32_lanes(D
 // (branch-free, out-of-range entries masked), the group sum added to the int64 fixed-point
 // density; cutoff decisions in the guard band re-done in FP64 as in the force kernel.
 template <int SCM, int FEED>
-__device__ __forceinline__ void density32_tile(const Dev& D, const PotParams& P, const int tile) {
+__device__ __forceinline__ void density32_tile(const Dev& D, const PotParams& P, const Blk32 B) {
   __shared__ __align__(16) uint4 ring_s[TILE / 32][RING][32];
   __shared__ __align__(8) unsigned long long bar_s[TILE / 32][RING];
-  const int s = D.tile_sys[tile];
+  const int s = B.sys;
   const SysDev& S = D.sysd[s];
-  if (!S.active) return;  // whole block: one tile belongs to one system
+  if (!S.active) return;  // whole block: its atoms belong to one system
   SHIFT_TABLE(shifts);
   const ShiftCorr corr = shift_corr(S);
-  const int li = D.tile_first[tile] - (int)S.atom_base + (int)threadIdx.x;
+  const int li = B.first - (int)S.atom_base + (int)threadIdx.x;
   const long long i = S.atom_base + li;
-  const bool active = (int)threadIdx.x < D.tile_count[tile];
+  const bool active = (int)threadIdx.x < B.count;
   const float4* __restrict__ g32 = D.g32 + S.atom_base;
   const float4 gi = active ? g32[li] : make_float4(0.f, 0.f, 0.f, 0.f);
   const float rc2_lo = P.f[12], rc2_hi = P.f[13];
@@ -979,8 +970,8 @@ __device__ __forceinline__ void density32_tile(const Dev& D, const PotParams& P,
   const float scale = (float)FIX_RHO;
   // every lane of the warp takes part in the ring (lanes without an atom have no groups)
   const int w = threadIdx.x >> 5;
-  const int wfirst = D.tile_first[tile] - (int)S.atom_base + 32 * w;
-  const int wcount = min(32, max(0, D.tile_count[tile] - 32 * w));
+  const int wfirst = B.first - (int)S.atom_base + 32 * w;
+  const int wcount = min(32, max(0, B.count - 32 * w));
   const int ngw = __reduce_max_sync(0xffffffffu, (unsigned)ng);
   auto row = [&](int g, const uint4& e4) {
     if (g < ng) {
@@ -1038,11 +1029,90 @@ __device__ __forceinline__ void density32_tile(const Dev& D, const PotParams& P,
 
 
 template <int SCM, int FEED = FEED_REGS>
-__global__ void GBMD_DENSITY_BOUNDS k_eam_density32(Dev D, PotParams P) {
-  const int tile = claim_tile(D);
-  if (tile >= 0) density32_tile<SCM, FEED>(D, P, tile);
-  release_tile(D);
+__global__ void GBMD_DENSITY_BOUNDS k_eam_density32(Dev D, PotParams P, const Blk32* blk) {
+  density32_tile<SCM, FEED>(D, P, blk[blockIdx.x]);
 }
+
+// The same with LANES lanes per atom (see k_force32_lanes): densities bitwise those of one lane.
+template <int SCM, int LANES>
+__global__ void __launch_bounds__(TILE, 8)
+    k_eam_density32_lanes(Dev D, PotParams P, const Blk32* blk) {
+  constexpr int APB = TILE / LANES;
+  __shared__ float4 shifts[125];
+  __shared__ long long rsum[APB];
+  const Blk32 B = blk[blockIdx.x];
+  const SysDev& S = D.sysd[B.sys];
+  if (!S.active) return;  // whole block: its atoms belong to one system
+  load_shifts(S, shifts);
+  const ShiftCorr corr = shift_corr(S);
+  const int lane = threadIdx.x & 31;
+  const int sub = threadIdx.x % LANES, slot = (int)threadIdx.x / LANES;
+  const float4* __restrict__ g32 = D.g32 + S.atom_base;
+  const float rc2_lo = P.f[12], rc2_hi = P.f[13];
+  const float scale = (float)FIX_RHO;
+  unsigned rechecks = 0;
+  const bool active = slot < B.count;
+  const int li = B.first - (int)S.atom_base + (active ? slot : 0);
+  const long long i = S.atom_base + li;
+  const float4 gi = active ? g32[li] : make_float4(0.f, 0.f, 0.f, 0.f);
+  const int cnt = active ? D.ncount[i] : 0;
+  const int ng = (cnt + 3) >> 2;
+  Fix rho;
+  const uint4* L = active ? list_group(D, S, li, 0) : nullptr;
+  for (int q = sub; q < ng; q += LANES) {
+    const uint4 cur = __ldg(L + (long long)q * S.natoms);
+    const unsigned e[4] = {cur.x, cur.y, cur.z, cur.w};
+    const int rem = cnt - 4 * q;
+    float4 gj[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) gj[u] = g32[e[u] & LOCAL_MASK];
+    float part = 0.f;
+    bool band = false;
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const bool valid = u == 0 || rem > u;
+      float dx, dy, dz;
+      const float r2 = entry_r2(gi, gj[u], shifts[e[u] >> CODE_SHIFT], corr, dx, dy, dz);
+      band = band || (valid && r2 >= rc2_lo && r2 < rc2_hi);
+      const float v = eam_rho32_t<SCM>(P, r2);
+      const float t = valid && r2 < rc2_lo ? v : 0.0f;
+      part = u == 0 ? t : part + t;
+    }
+    rho.add(part * scale);
+    if (band) {  // exact FP64 cutoff decision for the group's guard-band entries
+      for (int u = 0; u < 4 && u < rem; ++u) {
+        const int j = (int)(e[u] & LOCAL_MASK);
+        float dx, dy, dz;
+        const float r2 = entry_r2(gi, g32[j], shifts[e[u] >> CODE_SHIFT], corr, dx, dy, dz);
+        if (!(r2 >= rc2_lo && r2 < rc2_hi)) continue;
+        ++rechecks;
+        if (exact_inside_cold(&D, &S, i, S.atom_base + j, P.rc2)) rho.add(eam_rho32_t<SCM>(P, r2) * scale);
+      }
+    }
+  }
+  lanes_sum<LANES>(rho);
+  if (sub == 0 && active) rsum[slot] = rho.value();
+  if (rechecks) atomicAdd(&D.sst[B.sys].rechecks, (unsigned long long)rechecks);
+  __syncthreads();
+  const int t = threadIdx.x;
+  if (t >= ((B.count + 31) & ~31)) return;  // whole warps
+  long long f = 0;
+  if (t < B.count) {
+    const long long a = B.first + t;
+    const double r = (double)rsum[t] * (1.0 / FIX_RHO);
+    double F, phi;
+    eam_embed64(P, r, F, phi);
+    D.rho[a] = r;
+    D.phi[a] = phi;
+    D.phif[a] = (float)phi;
+    const float4 g = g32[a - S.atom_base];
+    D.g32e[a] = make_float4(g.x, g.y, g.z, (float)((double)P.f[14] * phi));
+    f = __double2ll_rn(F * FIX_E);
+  }
+  f = warp_sum(f);
+  if (lane == 0) atomicAdd(D.sys_acc + (long long)B.sys * SA_LEN + SA_EEMBED, (unsigned long long)f);
+}
+
 
 // ------------------------------------------------------------------------------------------
 // Tail of an FP64 force evaluation: sums the partial records of the system's blocks in a fixed
