@@ -322,13 +322,12 @@ gbmd_status gbmd_selftest_bounded_wait(int device, int64_t polls, int* gave_up);
  *   stream  cudaStream_t the two kernels are queued on (NULL: the default stream); the call
  *           returns without waiting for them
  *
- * Scratch: the per-block partial sums live in a fixed 11 KB device array inside the
+ * Scratch: the per-block partial sums live in a fixed 38 KB device array inside the
  * library, overwritten by every call; the caller's output buffers need not start at zero.
- * The first call on a device (with that device current) looks the array up, which may load
- * the module: make that first call before anything that must not see module loading, such
- * as stream capture.  The address is kept for the life of the process, so do not call this
- * entry point on a device after cudaDeviceReset on it.  Calls that overlap in time on one
- * device (other host threads, other streams) share the array and race: serialise them. */
+ * The first call on a device (with that device current) may load the module: make that
+ * first call before anything that must not see module loading, such as stream capture.
+ * Calls that overlap in time on one device (other host threads, other streams) share the
+ * array and race: serialise them. */
 gbmd_status gbmd_pair_forces_static(const gbmd_plugin* plugin, const double* pos, int n, const double* box,
                                     double* force, double* out, void* stream);
 

@@ -32,17 +32,6 @@ __device__ __forceinline__ float ipow_f(float x, int n) {
 // FP64
 // ------------------------------------------------------------------------------------------
 
-// LennardJones pairForce/pairEnergy: ff = -48 (eps/r^2) (s^12 - 0.5 s^6), E = 4 eps (s^12 - s^6)
-// with s^6 = (sigma^2/r^2)^3.
-__device__ __forceinline__ void lj_pair64(const PotParams& P, double r2, double& g, double& e) {
-  const double sigma = P.p[0], eps = P.p[1];
-  double x = ddiv(dmul(sigma, sigma), r2);
-  double r6 = dmul(dmul(x, x), x);
-  double r12 = dmul(r6, r6);
-  g = dmul(dmul(-48.0, ddiv(eps, r2)), dsub(r12, dmul(0.5, r6)));
-  e = dmul(dmul(4.0, eps), dsub(r12, r6));
-}
-
 // FastLJ pairEnergy / pairForce (plugins/fastlj.cc:56-73): the tabulated LJ values of bin
 // k = floor(bins r / cutoff) (no interpolation).  k is clamped to the last bin, which a distance
 // that rounds to the cutoff would otherwise pass (the reference reads past its table there).
