@@ -623,6 +623,7 @@ struct Engine::Impl {
     }
     if (dev < 0 || dev >= count) throw Error(1, "device index out of range");
     CK(cudaSetDevice(dev));
+    CK(cudaFuncSetAttribute(k_sort_cluster, cudaFuncAttributeMaxDynamicSharedMemorySize, CLUSTER_SORT_BYTES));
     CK(cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking));
     CK(cudaStreamCreateWithFlags(&stream2, cudaStreamNonBlocking));
     natoms = na;
@@ -1005,35 +1006,62 @@ struct Engine::Impl {
 
   void launch_rebuild(cudaStream_t s) {
     Range r("gbmd:enqueue_rebuild");
+    if (sysd[0].mode == NB_ALLPAIRS) return;  // nothing is sorted or listed
     launch_rebuild_kernels(s);
     if (lcb_exact() && !capturing) lcb_grow_until_single(s);
   }
 
   static constexpr unsigned REBUILD_GRID = 4864;  // 32 blocks for each of the 152 SMs
+  long long most_atoms() const {
+    long long m = 0;
+    for (auto n : natoms) m = std::max<long long>(m, n);
+    return m;
+  }
+  bool cluster_sort() const { return most_atoms() <= (nsys == 1 ? CLUSTER_ATOMS : CLUSTER_ATOMS_BATCH); }
   void launch_rebuild_kernels(cudaStream_t s) {
     mark_begin(s, T_REBUILD);
     // a batch's chain runs over the systems listed by its first kernel, in grids that the list may
     // exceed or fall short of
     unsigned nb = 0, nc = (unsigned)D.total_cells;
     for (int q = 0; q < nsys; ++q) nb += nblocks(natoms[q], REBUILD_CHUNK);
-    if (nsys > 1) {
+    if (nsys > 1 || cluster_sort()) {
       nb = std::min(nb, REBUILD_GRID);
       nc = std::min(nc, REBUILD_GRID);
+    }
+    if (nsys > 1) {
       k_rebuild_list<<<1, RLIST_THREADS, 0, s>>>(D);
       launched();
     }
-    k_bin<<<nb, REBUILD_CHUNK, 0, s>>>(D);
-    k_scan<<<nsys, 1024, 0, s>>>(D);
-    k_scatter<<<nb, REBUILD_CHUNK, 0, s>>>(D);
-    k_cellsort<<<nblocks(nc, SORT_WARPS), 32 * SORT_WARPS, 0, s>>>(D);
-    k_permute<<<nb, REBUILD_CHUNK, 0, s>>>(D);
-    k_copyback<<<nb, REBUILD_CHUNK, 0, s>>>(D);
-    launched(6);
+    if (cluster_sort()) {
+      const int blocks = cluster_blocks(most_atoms());
+      cudaLaunchConfig_t cfg = {};
+      cfg.gridDim = dim3((unsigned)(nsys * blocks));
+      cfg.blockDim = dim3(CLUSTER_THREADS);
+      cfg.dynamicSmemBytes = CLUSTER_SORT_BYTES;
+      cfg.stream = s;
+      cudaLaunchAttribute attr = {};
+      attr.id = cudaLaunchAttributeClusterDimension;
+      attr.val.clusterDim.x = (unsigned)blocks;
+      attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+      cfg.attrs = &attr;
+      cfg.numAttrs = 1;
+      CK(cudaLaunchKernelEx(&cfg, k_sort_cluster, D, blocks));
+      launched();
+    } else {
+      k_bin<<<nb, REBUILD_CHUNK, 0, s>>>(D);
+      k_scan<<<nsys, 1024, 0, s>>>(D);
+      k_scatter<<<nb, REBUILD_CHUNK, 0, s>>>(D);
+      k_cellsort<<<nblocks(nc, SORT_WARPS), 32 * SORT_WARPS, 0, s>>>(D);
+      k_permute<<<nb, REBUILD_CHUNK, 0, s>>>(D);
+      k_copyback<<<nb, REBUILD_CHUNK, 0, s>>>(D);
+      launched(6);
+    }
     if (any_list) {
       bool block = false, warp = false;
       for (const auto& S : sysd) (S.ncells > LIST_BLOCK_CELLS ? warp : block) = true;
       if (block) {
         const int batch = list_batch(D.maxnb);
+        if (cluster_sort()) nc = std::min(nc, 4u * sm_count);  // the blocks that are resident at once
         if (batch > 0)
           k_buildlist_block<true><<<nc, 32 * LIST_WARPS, sizeof(unsigned) * batch * (D.maxnb + 4), s>>>(D, batch);
         else
@@ -1041,7 +1069,9 @@ struct Engine::Impl {
         launched();
       }
       if (warp) {
-        k_buildlist_warp<<<nblocks(nc, LIST_CELLS), 32 * LIST_CELLS, 0, s>>>(D);
+        unsigned ng = nblocks(nc, LIST_CELLS);
+        if (cluster_sort()) ng = std::min(ng, 6u * sm_count);
+        k_buildlist_warp<<<ng, 32 * LIST_CELLS, 0, s>>>(D);
         launched();
       }
     }
@@ -1344,7 +1374,10 @@ struct Engine::Impl {
     std::lock_guard<std::recursive_mutex> lk(g_dev_mu);
     drop_graph();
     CK(cudaGraphCreate(&graph, 0));
-    bool cond = graph_mode == 2;
+    // a conditional node costs 8.5 us a step whether its body runs or not: as much as the whole chain's
+    // empty launches.  So it only pays for a single system too large for the one-launch sort; of a
+    // batch some system rebuilds in nearly every step
+    bool cond = graph_mode == 2 && !cluster_sort() && nsys == 1 && sysd[0].mode != NB_ALLPAIRS;
     std::vector<cudaGraphConditionalHandle> handles(nsteps);
     if (cond) {
       for (int k = 0; k < nsteps; ++k) {

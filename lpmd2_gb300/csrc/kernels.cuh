@@ -193,33 +193,35 @@ __device__ __forceinline__ void for_rebuild_atoms(const Dev& D, F&& body) {
   }
 }
 
+__device__ __forceinline__ void bin_atom(const Dev& D, int s, long long i) {
+  const SysDev& S = D.sysd[s];
+  bool ok = true;
+  int cx, cy, cz;
+  if (S.mode == NB_LIST) {
+    // Verlet-list grid: cells are wider than the list radius by a margin, so the binning may
+    // round differently from LinkedCell's; one multiply instead of a division per axis
+    cx = list_cell_coord(D.x[i] * S.ninv[0], S.n[0], ok);
+    cy = list_cell_coord(D.y[i] * S.ninv[1], S.n[1], ok);
+    cz = list_cell_coord(D.z[i] * S.ninv[2], S.n[2], ok);
+  } else {
+    cx = ref_cell_coord(D.x[i], S.L[0], S.n[0], ok);
+    cy = ref_cell_coord(D.y[i], S.L[1], S.n[1], ok);
+    cz = ref_cell_coord(D.z[i], S.L[2], S.n[2], ok);
+  }
+  if (!ok) {
+    atomicOr(&D.sst[s].error, ERR_OUTSIDE);
+    cx = cy = cz = 0;
+  }
+  const int c = S.cell_base + (cz * S.n[1] + cy) * S.n[0] + cx;
+  D.acell[i] = c;
+  // consecutive atoms mostly share a cell (the arrays are in the previous cell order): one
+  // atomic per cell and warp
+  const unsigned peers = __match_any_sync(__activemask(), c);
+  if ((threadIdx.x & 31) == __ffs(peers) - 1) atomicAdd(&D.ccount[c], __popc(peers));
+}
+
 __global__ void __launch_bounds__(REBUILD_CHUNK) k_bin(Dev D) {
-  for_rebuild_atoms(D, [&](int s, long long i) {
-    const SysDev& S = D.sysd[s];
-    bool ok = true;
-    int cx, cy, cz;
-    if (S.mode == NB_LIST) {
-      // Verlet-list grid: cells are wider than the list radius by a margin, so the binning may
-      // round differently from LinkedCell's; one multiply instead of a division per axis
-      cx = list_cell_coord(D.x[i] * S.ninv[0], S.n[0], ok);
-      cy = list_cell_coord(D.y[i] * S.ninv[1], S.n[1], ok);
-      cz = list_cell_coord(D.z[i] * S.ninv[2], S.n[2], ok);
-    } else {
-      cx = ref_cell_coord(D.x[i], S.L[0], S.n[0], ok);
-      cy = ref_cell_coord(D.y[i], S.L[1], S.n[1], ok);
-      cz = ref_cell_coord(D.z[i], S.L[2], S.n[2], ok);
-    }
-    if (!ok) {
-      atomicOr(&D.sst[s].error, ERR_OUTSIDE);
-      cx = cy = cz = 0;
-    }
-    const int c = S.cell_base + (cz * S.n[1] + cy) * S.n[0] + cx;
-    D.acell[i] = c;
-    // consecutive atoms mostly share a cell (the arrays are in the previous cell order): one
-    // atomic per cell and warp
-    const unsigned peers = __match_any_sync(__activemask(), c);
-    if ((threadIdx.x & 31) == __ffs(peers) - 1) atomicAdd(&D.ccount[c], __popc(peers));
-  });
+  for_rebuild_atoms(D, [&](int s, long long i) { bin_atom(D, s, i); });
 }
 
 // One block per system: exclusive scan of the cell counts; resets counts and cursors.  A thread takes
@@ -228,9 +230,7 @@ __global__ void __launch_bounds__(REBUILD_CHUNK) k_bin(Dev D) {
 // barriers, not bandwidth, is the time (4 cells a thread: 123 us for the 110,592 cells of a 2 M atom
 // liquid, 63 so; 16 -> 9 us for 13,824).
 constexpr int SCAN_CELLS = 16;
-__global__ void __launch_bounds__(1024) k_scan(Dev D) {
-  const int s = blockIdx.x;
-  if (!D.sst[s].need_rebuild) return;
+__device__ __forceinline__ void scan_cells(const Dev& D, int s) {
   const SysDev& S = D.sysd[s];
   const int cb = S.cell_base, ce = cb + S.ncells, a0 = cb & ~3;
   __shared__ int warp_tot[32];
@@ -299,6 +299,9 @@ __global__ void __launch_bounds__(1024) k_scan(Dev D) {
     __syncthreads();  // warp_tot is written again
   }
 }
+__global__ void __launch_bounds__(1024) k_scan(Dev D) {
+  if (D.sst[blockIdx.x].need_rebuild) scan_cells(D, blockIdx.x);
+}
 
 // LCBinary::UpdateCell keeps at most one atom per sub-cell (plugins/lcbinary.cc:162-193): flags
 // the systems whose re-sort put two atoms into one cell (their grid then grows by 2 per axis).
@@ -314,18 +317,20 @@ __global__ void k_binary_clear(Dev D) {
   for (int s = threadIdx.x; s < D.nsys; s += blockDim.x) D.sst[s].collide = 0;
 }
 
+__device__ __forceinline__ void scatter_atom(const Dev& D, long long i) {
+  const int c = D.acell[i];
+  // the warp's atoms of one cell take consecutive slots from one atomic (their order inside
+  // the cell is set by k_cellsort either way)
+  const unsigned peers = __match_any_sync(__activemask(), c);
+  const int lane = threadIdx.x & 31, lead = __ffs(peers) - 1;
+  int first = 0;
+  if (lane == lead) first = atomicAdd(&D.ccursor[c], __popc(peers));
+  first = __shfl_sync(peers, first, lead);
+  D.perm[D.cstart[c] + first + __popc(peers & ((1u << lane) - 1u))] = (int)i;
+}
+
 __global__ void __launch_bounds__(REBUILD_CHUNK) k_scatter(Dev D) {
-  for_rebuild_atoms(D, [&](int, long long i) {
-    const int c = D.acell[i];
-    // the warp's atoms of one cell take consecutive slots from one atomic (their order inside
-    // the cell is set by k_cellsort either way)
-    const unsigned peers = __match_any_sync(__activemask(), c);
-    const int lane = threadIdx.x & 31, lead = __ffs(peers) - 1;
-    int first = 0;
-    if (lane == lead) first = atomicAdd(&D.ccursor[c], __popc(peers));
-    first = __shfl_sync(peers, first, lead);
-    D.perm[D.cstart[c] + first + __popc(peers & ((1u << lane) - 1u))] = (int)i;
-  });
+  for_rebuild_atoms(D, [&](int, long long i) { scatter_atom(D, i); });
 }
 
 // One warp per cell of the rebuilding systems: orders the cell's slots by original index, the order in which LinkedCell's head/next lists
@@ -391,30 +396,32 @@ __global__ void __launch_bounds__(32 * SORT_WARPS) k_cellsort(Dev D) {
   }
 }
 
+__device__ __forceinline__ void permute_atom(const Dev& D, long long p) {
+  const long long N = D.N;
+  const int o = D.perm[p];
+  double* sd = D.sdbl;
+  sd[0 * N + p] = D.x[o];
+  sd[1 * N + p] = D.y[o];
+  sd[2 * N + p] = D.z[o];
+  sd[3 * N + p] = D.vx[o];
+  sd[4 * N + p] = D.vy[o];
+  sd[5 * N + p] = D.vz[o];
+  sd[6 * N + p] = D.ax[o];
+  sd[7 * N + p] = D.ay[o];
+  sd[8 * N + p] = D.az[o];
+  sd[9 * N + p] = D.mass[o];
+  sd[10 * N + p] = D.fm[o];
+  int* si = D.sint;
+  si[0 * N + p] = D.type[o];
+  si[1 * N + p] = D.tag[o];
+  si[2 * N + p] = D.acell[o];
+  if (D.has_flags) D.sflags[p] = D.flags[o];
+  if (D.ist)
+    for (int k = 0; k < IST_K; ++k) D.ist_alt[k * N + p] = D.ist[k * N + o];
+}
+
 __global__ void __launch_bounds__(REBUILD_CHUNK) k_permute(Dev D) {
-  for_rebuild_atoms(D, [&](int, long long p) {
-    const long long N = D.N;
-    const int o = D.perm[p];
-    double* sd = D.sdbl;
-    sd[0 * N + p] = D.x[o];
-    sd[1 * N + p] = D.y[o];
-    sd[2 * N + p] = D.z[o];
-    sd[3 * N + p] = D.vx[o];
-    sd[4 * N + p] = D.vy[o];
-    sd[5 * N + p] = D.vz[o];
-    sd[6 * N + p] = D.ax[o];
-    sd[7 * N + p] = D.ay[o];
-    sd[8 * N + p] = D.az[o];
-    sd[9 * N + p] = D.mass[o];
-    sd[10 * N + p] = D.fm[o];
-    int* si = D.sint;
-    si[0 * N + p] = D.type[o];
-    si[1 * N + p] = D.tag[o];
-    si[2 * N + p] = D.acell[o];
-    if (D.has_flags) D.sflags[p] = D.flags[o];
-    if (D.ist)
-      for (int k = 0; k < IST_K; ++k) D.ist_alt[k * N + p] = D.ist[k * N + o];
-  });
+  for_rebuild_atoms(D, [&](int, long long i) { permute_atom(D, i); });
 }
 
 // Offset of x from the centre xc of its home cell, wrapped into [-L/2, L/2).  Two FP64-pipe
@@ -467,30 +474,82 @@ __device__ __forceinline__ void track_displacement_warp(const Dev& D, int s, flo
   if ((threadIdx.x & 31) == 0 && m) atomicMax(&D.sst[s].maxdisp2, m);
 }
 
+__device__ __forceinline__ void copyback_atom(const Dev& D, int s, long long p) {
+  const long long N = D.N;
+  const double* sd = D.sdbl;
+  D.x[p] = sd[0 * N + p];
+  D.y[p] = sd[1 * N + p];
+  D.z[p] = sd[2 * N + p];
+  D.vx[p] = sd[3 * N + p];
+  D.vy[p] = sd[4 * N + p];
+  D.vz[p] = sd[5 * N + p];
+  D.ax[p] = sd[6 * N + p];
+  D.ay[p] = sd[7 * N + p];
+  D.az[p] = sd[8 * N + p];
+  D.mass[p] = sd[9 * N + p];
+  D.fm[p] = sd[10 * N + p];
+  const int* si = D.sint;
+  D.type[p] = si[0 * N + p];
+  D.tag[p] = si[1 * N + p];
+  D.home[p] = si[2 * N + p];
+  if (D.has_flags) D.flags[p] = D.sflags[p];
+  if (D.ist)
+    for (int k = 0; k < IST_K; ++k) D.ist[k * N + p] = D.ist_alt[k * N + p];
+  refresh_gather(D, D.sysd[s], p, true);
+}
+
 __global__ void __launch_bounds__(REBUILD_CHUNK) k_copyback(Dev D) {
-  for_rebuild_atoms(D, [&](int s, long long p) {
-    const long long N = D.N;
-    const double* sd = D.sdbl;
-    D.x[p] = sd[0 * N + p];
-    D.y[p] = sd[1 * N + p];
-    D.z[p] = sd[2 * N + p];
-    D.vx[p] = sd[3 * N + p];
-    D.vy[p] = sd[4 * N + p];
-    D.vz[p] = sd[5 * N + p];
-    D.ax[p] = sd[6 * N + p];
-    D.ay[p] = sd[7 * N + p];
-    D.az[p] = sd[8 * N + p];
-    D.mass[p] = sd[9 * N + p];
-    D.fm[p] = sd[10 * N + p];
-    const int* si = D.sint;
-    D.type[p] = si[0 * N + p];
-    D.tag[p] = si[1 * N + p];
-    D.home[p] = si[2 * N + p];
-    if (D.has_flags) D.flags[p] = D.sflags[p];
-    if (D.ist)
-      for (int k = 0; k < IST_K; ++k) D.ist[k * N + p] = D.ist_alt[k * N + p];
-    refresh_gather(D, D.sysd[s], p, true);
-  });
+  for_rebuild_atoms(D, [&](int s, long long i) { copyback_atom(D, s, i); });
+}
+
+// ---------------------------------------------------------------------------------------------
+// The same sort in one launch: a cluster of blocks per system goes through the phases above with
+// the hardware's cluster barrier between them (release / acquire, so that each phase sees the others'
+// writes to global memory).  Bound by latency: six phases on at most 8 SMs.  It replaces six launches
+// when the system rebuilds, and when it does not it costs one empty launch, with which a graph step
+// does without its conditional node.  Measured against the chain of kernels (conditional node
+// included), us a step: single LJ liquids of 500 / 4,000 / 8,788 / 16,384 / 32,000 atoms 21.2 / 24.8 /
+// 25.8 / 30.0 / 38.5 against 27.8 / 28.0 / 29.9 / 32.9 / 37.3; batches of 512 x 256 atoms 101 against
+// 110, of 33 systems up to 4,000 87 against 77.
+// ---------------------------------------------------------------------------------------------
+constexpr int CLUSTER_ATOMS = 24000;       // a single system
+constexpr int CLUSTER_ATOMS_BATCH = 2048;  // the largest system of a batch
+constexpr int CLUSTER_THREADS = 1024;
+constexpr int CLUSTER_SORT_BYTES = CLUSTER_THREADS / 32 * 2 * SORT_STAGE * (int)sizeof(int);
+
+// Blocks of a system's cluster (at most 8, the portable size): two or more atoms a thread.
+inline int cluster_blocks(long long natoms) {
+  int b = 1;
+  while (b < 8 && (long long)b * 2 * CLUSTER_THREADS < natoms) b *= 2;
+  return b;
+}
+
+__device__ __forceinline__ void cluster_barrier() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+__global__ void __launch_bounds__(CLUSTER_THREADS, 1) k_sort_cluster(Dev D, int blocks) {
+  extern __shared__ int stage[];  // SORT_STAGE tags and indices per warp
+  const int s = blockIdx.x / blocks, rank = blockIdx.x % blocks;
+  if (!D.sst[s].need_rebuild) return;  // the whole cluster
+  const SysDev& S = D.sysd[s];
+  const int n = S.natoms, t0 = rank * CLUSTER_THREADS + (int)threadIdx.x, step = blocks * CLUSTER_THREADS;
+  for (int k = t0; k < n; k += step) bin_atom(D, s, S.atom_base + k);
+  cluster_barrier();
+  if (rank == 0) scan_cells(D, s);
+  cluster_barrier();
+  for (int k = t0; k < n; k += step) scatter_atom(D, S.atom_base + k);
+  cluster_barrier();
+  const int w = threadIdx.x >> 5;
+  int* const mine = stage + w * 2 * SORT_STAGE;
+  for (int c = rank * (CLUSTER_THREADS / 32) + w; c < S.ncells; c += blocks * (CLUSTER_THREADS / 32)) {
+    sort_cell(D, S.cell_base + c, mine, mine + SORT_STAGE);
+    __syncwarp();
+  }
+  cluster_barrier();
+  for (int k = t0; k < n; k += step) permute_atom(D, S.atom_base + k);
+  cluster_barrier();
+  for (int k = t0; k < n; k += step) copyback_atom(D, s, S.atom_base + k);
 }
 
 // ---------------------------------------------------------------------------------------------
