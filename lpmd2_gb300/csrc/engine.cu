@@ -1377,7 +1377,8 @@ struct Engine::Impl {
     // a conditional node costs 8.5 us a step whether its body runs or not: as much as the whole chain's
     // empty launches.  So it only pays for a single system too large for the one-launch sort; of a
     // batch some system rebuilds in nearly every step
-    bool cond = graph_mode == 2 && !cluster_sort() && nsys == 1 && sysd[0].mode != NB_ALLPAIRS;
+    const bool plain = integ.kind != INT_VV;  // step_plain keeps its chain in line
+    bool cond = graph_mode == 2 && !plain && !cluster_sort() && nsys == 1 && sysd[0].mode != NB_ALLPAIRS;
     std::vector<cudaGraphConditionalHandle> handles(nsteps);
     if (cond) {
       for (int k = 0; k < nsteps; ++k) {
@@ -1397,8 +1398,13 @@ struct Engine::Impl {
     int64_t base_launches = 0;
     try {
       for (int k = 0; k < nsteps; ++k) {
-        set_buffers(1 - cbuf);
         int64_t before = st.kernel_launches;
+        if (plain) {
+          step_plain();
+          base_launches += st.kernel_launches - before;
+          continue;
+        }
+        set_buffers(1 - cbuf);
         if (k == 0) launch_decide(stream, 2, 0, cond ? handles[k] : 0, cond ? 1 : 0);
         if (!cond) launch_rebuild(stream);
         base_launches += st.kernel_launches - before;
@@ -1584,7 +1590,29 @@ struct Engine::Impl {
         init_integrator();
         initialized = true;
       }
-      for (int64_t k = 0; k < nsteps; ++k) step_plain();
+      // a step is a dozen or more short launches: blocks of steps are captured as for velocityverlet,
+      // once there are enough of them to pay for the capture (LJ liquid of 16,384 atoms under Beeman:
+      // 74 us a step launched, 51 captured)
+      int64_t done = 0;
+      const int gbe = lcb_exact() || graph_mode == 0 ? 0 : graph_block & ~1;
+      if (gbe > 0 && pending_ucalls > 0) {
+        step_plain();  // the UpdateCell calls owed to the set-up
+        ++done;
+      }
+      if (gbe > 0) {
+        if (gexec && gsteps == gbe && gparity != cbuf && nsteps - done > gbe) {
+          step_plain();  // to the buffers that the graph was captured for
+          ++done;
+        }
+        const bool built = gexec && gparity == cbuf && gsteps == gbe;
+        if (!built && nsteps - done >= 2 * gbe) build_graph(gbe);
+        while (gexec && gparity == cbuf && gsteps == gbe && nsteps - done >= gbe) {
+          CK(cudaGraphLaunch(gexec, stream));
+          st.kernel_launches += graph_launches;
+          done += gbe;
+        }
+      }
+      for (; done < nsteps; ++done) step_plain();
       st.steps += nsteps;
       st.force_evaluations += nsteps;
       check_errors();
@@ -1610,6 +1638,14 @@ struct Engine::Impl {
       // a block of gb steps flips the buffers gb times: keep its parity even so one graph
       // serves every block
       const int gbe = gb & ~1;
+      if (gexec && gsteps == gbe && gparity != cbuf && nsteps - done > gbe) {
+        // an odd number of steps since the last block: one more brings back the buffers that the
+        // graph was captured for, where a second capture would cost more than the block
+        launch_step_head(stream, 2, false, 0);
+        launch_step_tail(stream);
+        check_launch("step");
+        ++done;
+      }
       if (gbe > 0 && (cbuf != gparity || !gexec || gsteps != gbe) && nsteps - done >= gbe)
         build_graph(gbe);
       while (gbe > 0 && nsteps - done >= gbe && gparity == cbuf) {
