@@ -386,10 +386,14 @@ struct Engine::Impl {
     D.g32o = G32buf[1 - in];
   }
 
-  cudaGraphExec_t gexec = nullptr;
-  cudaGraph_t graph = nullptr;
-  int gsteps = 0;
-  int gparity = -1;  // cbuf the graph was captured for
+  // captured blocks of steps, one for each position buffer to start from: calls of any number of
+  // steps find theirs (with one graph, an odd count between blocks meant a new capture)
+  struct StepGraph {
+    cudaGraphExec_t exec = nullptr;
+    cudaGraph_t graph = nullptr;
+    int steps = 0;
+  };
+  StepGraph graphs[2];
   std::map<int, long long> read_from;  // next thermo-log step to hand out, per system
   int pending_ucalls = 0;              // UpdateCell calls owed to SetCellManager
 
@@ -597,13 +601,13 @@ struct Engine::Impl {
     cell_bytes = 0;
   }
 
+  static void drop_graph(StepGraph& g) {
+    if (g.exec) cudaGraphExecDestroy(g.exec);
+    if (g.graph) cudaGraphDestroy(g.graph);
+    g = StepGraph();
+  }
   void drop_graph() {
-    if (gexec) cudaGraphExecDestroy(gexec);
-    if (graph) cudaGraphDestroy(graph);
-    gexec = nullptr;
-    graph = nullptr;
-    gsteps = 0;
-    gparity = -1;
+    for (StepGraph& g : graphs) drop_graph(g);
   }
 
   void launched(int n = 1) { st.kernel_launches += n; }
@@ -721,6 +725,10 @@ struct Engine::Impl {
     D.log_cap = log_cap;
     D.nsys = nsys;
     D.thermo_log = alloc<double>((size_t)nsys * log_cap * THERMO_LEN);
+    {
+      std::lock_guard<std::recursive_mutex> lk(g_dev_mu);
+      CK(cudaMallocHost(&h_sst, sizeof(SysState) * nsys));
+    }
     d_sysd = alloc<SysDev>(nsys);
     d_sst = alloc<SysState>(nsys);
     d_tile_sys = alloc<int>(ntiles);
@@ -802,6 +810,10 @@ struct Engine::Impl {
     }
     for (cudaEvent_t e : event_pool) cudaEventDestroy(e);
     for (auto& a : allocs) dev_free(a.first);
+    if (h_sst) {
+      std::lock_guard<std::recursive_mutex> lk(g_dev_mu);
+      cudaFreeHost(h_sst);
+    }
     free_scratch();
     for (auto& a : work) dev_free(a.first);
     if (plan_pair.blk) dev_free(plan_pair.blk);
@@ -1259,17 +1271,24 @@ struct Engine::Impl {
     }
   }
 
+  // The per-system states, read behind everything queued on the stream into page-locked memory (one
+  // wait; a copy to pageable memory after a wait of its own cost 10 us more a call).
+  const SysState* read_states() {
+    CK(cudaMemcpyAsync(h_sst, d_sst, sizeof(SysState) * nsys, cudaMemcpyDeviceToHost, stream));
+    CK(cudaStreamSynchronize(stream));
+    return h_sst;
+  }
+  SysState* h_sst = nullptr;
+
   // Reads the per-system error words and the list statistics (synchronises the stream).
   void check_errors() {
-    CK(cudaStreamSynchronize(stream));
+    const SysState* hs = read_states();
     collect_marks();
-    std::vector<SysState> hs(nsys);
-    CK(cudaMemcpyAsync(hs.data(), d_sst, sizeof(SysState) * nsys, cudaMemcpyDeviceToHost, stream));
-    CK(cudaStreamSynchronize(stream));
     int err = 0, maxc = 0;
     long long rb = 0;
     unsigned long long rech = 0;
-    for (const auto& x : hs) {
+    for (int s = 0; s < nsys; ++s) {
+      const SysState& x = hs[s];
       err |= x.error;
       maxc = std::max(maxc, x.max_count);
       rb += x.rebuilds;
@@ -1293,14 +1312,11 @@ struct Engine::Impl {
       launch_decide(stream, attempt == 0 ? 1 + pending_ucalls : 0, 1, 0, 0);
       launch_rebuild(stream);
       check_launch("rebuild");
-      CK(cudaStreamSynchronize(stream));
-      std::vector<SysState> hs(nsys);
-      CK(cudaMemcpyAsync(hs.data(), d_sst, sizeof(SysState) * nsys, cudaMemcpyDeviceToHost, stream));
-      CK(cudaStreamSynchronize(stream));
+      const SysState* hs = read_states();
       int maxc = 0, err = 0;
-      for (const auto& x : hs) {
-        maxc = std::max(maxc, x.max_count);
-        err |= x.error;
+      for (int s = 0; s < nsys; ++s) {
+        maxc = std::max(maxc, hs[s].max_count);
+        err |= hs[s].error;
       }
       if (err & ERR_OUTSIDE) throw Error(8, "RuntimeError: atom position is not finite or far outside the simulation box");
       pending_ucalls = 0;
@@ -1369,10 +1385,13 @@ struct Engine::Impl {
     cbuf = 1 - cbuf;
   }
 
+  // Captures a block of nsteps steps from the current position buffer.
   void build_graph(int nsteps) {
     Range r("gbmd:capture_graph");
     std::lock_guard<std::recursive_mutex> lk(g_dev_mu);
-    drop_graph();
+    StepGraph& built = graphs[cbuf];
+    drop_graph(built);
+    cudaGraph_t& graph = built.graph;
     CK(cudaGraphCreate(&graph, 0));
     // a conditional node costs 8.5 us a step whether its body runs or not: as much as the whole chain's
     // empty launches.  So it only pays for a single system too large for the one-launch sort; of a
@@ -1440,7 +1459,7 @@ struct Engine::Impl {
       cudaStreamEndCapture(stream, &tmp);
       cudaGetLastError();
       st.kernel_launches = saved;
-      drop_graph();
+      drop_graph(built);
       throw;
     }
     capturing = false;
@@ -1448,9 +1467,8 @@ struct Engine::Impl {
     cudaGraph_t out;
     CK(cudaStreamEndCapture(stream, &out));
     st.kernel_launches = saved;
-    CK(cudaGraphInstantiate(&gexec, graph, 0));
-    gsteps = nsteps;
-    gparity = cbuf0;
+    CK(cudaGraphInstantiate(&built.exec, graph, 0));
+    built.steps = nsteps;
     graph_cond = cond;
     graph_launches = base_launches;
   }
@@ -1600,14 +1618,9 @@ struct Engine::Impl {
         ++done;
       }
       if (gbe > 0) {
-        if (gexec && gsteps == gbe && gparity != cbuf && nsteps - done > gbe) {
-          step_plain();  // to the buffers that the graph was captured for
-          ++done;
-        }
-        const bool built = gexec && gparity == cbuf && gsteps == gbe;
-        if (!built && nsteps - done >= 2 * gbe) build_graph(gbe);
-        while (gexec && gparity == cbuf && gsteps == gbe && nsteps - done >= gbe) {
-          CK(cudaGraphLaunch(gexec, stream));
+        if (graphs[cbuf].steps != gbe && nsteps - done >= 2 * gbe) build_graph(gbe);
+        while (graphs[cbuf].steps == gbe && nsteps - done >= gbe) {
+          CK(cudaGraphLaunch(graphs[cbuf].exec, stream));
           st.kernel_launches += graph_launches;
           done += gbe;
         }
@@ -1635,21 +1648,12 @@ struct Engine::Impl {
     }
     const int gb = lcb_exact() ? 0 : graph_block;  // lcbinary grows its grid on the host
     if (graph_mode > 0 && gb > 0) {
-      // a block of gb steps flips the buffers gb times: keep its parity even so one graph
-      // serves every block
+      // a block of gb steps flips the buffers gb times: keep its parity even so that one graph
+      // serves every block of a call
       const int gbe = gb & ~1;
-      if (gexec && gsteps == gbe && gparity != cbuf && nsteps - done > gbe) {
-        // an odd number of steps since the last block: one more brings back the buffers that the
-        // graph was captured for, where a second capture would cost more than the block
-        launch_step_head(stream, 2, false, 0);
-        launch_step_tail(stream);
-        check_launch("step");
-        ++done;
-      }
-      if (gbe > 0 && (cbuf != gparity || !gexec || gsteps != gbe) && nsteps - done >= gbe)
-        build_graph(gbe);
-      while (gbe > 0 && nsteps - done >= gbe && gparity == cbuf) {
-        CK(cudaGraphLaunch(gexec, stream));
+      if (gbe > 0 && graphs[cbuf].steps != gbe && nsteps - done >= gbe) build_graph(gbe);
+      while (gbe > 0 && nsteps - done >= gbe) {
+        CK(cudaGraphLaunch(graphs[cbuf].exec, stream));
         st.kernel_launches += graph_launches;
         done += gbe;
       }
