@@ -195,8 +195,7 @@ __device__ __forceinline__ void scan64(const Dev& D, const SysDev& S, int li, bo
     const float xi = trunc32(pi.x), yi = trunc32(pi.y), zi = trunc32(pi.z);
     const float Lx = (float)S.L[0], Ly = (float)S.L[1], Lz = (float)S.L[2];
     const float rc2up = (float)rc2 * 1.000002f;
-    auto near = [&](int j) {
-      const double4_32a pj = D.g64[S.atom_base + j];
+    auto near = [&](const double4_32a& pj) {
       const float dx = axis_bound(xi, trunc32(pj.x), Lx), dy = axis_bound(yi, trunc32(pj.y), Ly),
                   dz = axis_bound(zi, trunc32(pj.z), Lz);
       return !(fmaf(dx, dx, fmaf(dy, dy, dz * dz)) > rc2up);
@@ -221,15 +220,29 @@ __device__ __forceinline__ void scan64(const Dev& D, const SysDev& S, int li, bo
         for (int k = 0; k < mw; ++k) {
           flush(lanes);
           const int j = b + k;
-          push(k < m && j != li && near(j) && species_ok(j), (unsigned)j | Q64_EXACT);
+          push(k < m && j != li && near(D.g64[S.atom_base + j]) && species_ok(j), (unsigned)j | Q64_EXACT);
         }
       }
     } else {
+      // four candidates a lane at a time: their loads overlap
       const int na = S.natoms;
-      for (int j0 = 0; j0 < na; j0 += lanes) {
-        flush(lanes);
-        const int j = j0 + sub;
-        push(active && j < na && j != li && near(j) && species_ok(j), (unsigned)j | Q64_EXACT);
+      for (int j0 = 0; j0 < na; j0 += 4 * lanes) {
+        flush(4 * lanes);
+        double4_32a pj[4];
+        bool in[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const int j = j0 + u * lanes + sub;
+          in[u] = active && j < na && j != li;
+          pj[u] = D.g64[S.atom_base + (j < na ? j : li)];
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) in[u] = in[u] && near(pj[u]);
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const int j = j0 + u * lanes + sub;
+          push(in[u] && species_ok(j), (unsigned)j | Q64_EXACT);
+        }
       }
     }
   }
