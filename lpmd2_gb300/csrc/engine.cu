@@ -169,7 +169,7 @@ __global__ void k_get_atoms(Dev D, long long base, int n, double* pos, double* v
 template <int NB, int MIXED>
 __global__ void k_export(Dev D, int s, double rc2, float rc2_lo, float rc2_hi, int half, long long* counts,
                          const long long* offsets, long long* idx) {
-  __shared__ float4 shifts[125];
+  __shared__ ShiftTable<> shifts;
   const SysDev& S = D.sysd[s];
   if (MIXED) load_shifts(S, shifts);
   long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x;

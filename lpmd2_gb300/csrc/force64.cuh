@@ -133,9 +133,9 @@ __device__ __forceinline__ double eam_body64(const PotParams& P, const Pair64& c
 // the lanes of an atom share its queue `q` of cap entries: those with j > i from the front, the
 // others from the back.  drain(nf, nb) consumes the nf front and nb back entries of the atom; it is
 // called whenever some atom's queue could overflow, and at the end.
-template <int NB, class F>
+template <int NB, class SH, class F>
 __device__ __forceinline__ void scan64(const Dev& D, const SysDev& S, int li, bool active, int lanes, int sub,
-                                       unsigned* q, int cap, const float4* shifts, double rc2, float lo, float hi,
+                                       unsigned* q, int cap, const SH& shifts, double rc2, float lo, float hi,
                                        int spc_sum, F&& drain) {
   const unsigned all = 0xffffffffu;
   const int lane = threadIdx.x & 31;
@@ -287,14 +287,14 @@ __global__ void __launch_bounds__(TILE, 5) k_force64(Dev D, PotParams P, Pair64 
   __shared__ unsigned queue[TILE / 32][Q64_WARP];
   __shared__ double fs[3][TILE];
   __shared__ double red[TILE / 32][16];
-  __shared__ float4 shifts[NB == NB_LIST ? 125 : 1];
+  __shared__ ShiftTable<NB == NB_LIST ? 125 : 1> shifts;
   const Blk64 B = D.blk64[blockIdx.x];
   const SysDev& S = D.sysd[B.sys];
   if (!S.active) {
     if (sp.epi == EPI_KICK_DRIFT && sp.last) hold_range(D, S, B.first, B.count, true);
     return;
   }
-  if (NB == NB_LIST) load_shifts(S, shifts);
+  if constexpr (NB == NB_LIST) load_shifts(S, shifts);
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int lanes = B.lanes, sub = lane & (lanes - 1), slot = lane / lanes, per = 32 / lanes;
   const int cap = Q64_WARP / per;
@@ -406,11 +406,11 @@ template <int NB, int SCM>
 __global__ void __launch_bounds__(TILE, 8) k_eam_density(Dev D, PotParams P, Pair64 c, int first) {
   __shared__ unsigned queue[TILE / 32][Q64_WARP];
   __shared__ double rs[TILE];
-  __shared__ float4 shifts[NB == NB_LIST ? 125 : 1];
+  __shared__ ShiftTable<NB == NB_LIST ? 125 : 1> shifts;
   const Blk64 B = D.blk64[blockIdx.x];
   const SysDev& S = D.sysd[B.sys];
   if (!S.active) return;
-  if (NB == NB_LIST) load_shifts(S, shifts);
+  if constexpr (NB == NB_LIST) load_shifts(S, shifts);
   const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int lanes = B.lanes, sub = lane & (lanes - 1), slot = lane / lanes, per = 32 / lanes;
   const int cap = Q64_WARP / per;

@@ -61,11 +61,28 @@ __device__ __noinline__ bool exact_inside_cold(const Dev* D, const SysDev* S, lo
   return exact_inside(*D, *S, i, j, rc2);
 }
 
-// Loads the cell-shift table (k * cell edge, k in -2..2 per axis) of system S into shared memory.
-__device__ __forceinline__ void load_shifts(const SysDev& S, float4* sh) {
+// The cell-shift table (k * cell edge, k in -2..2 per axis) of a block in shared memory, an array
+// per axis: a 4-byte word a lane takes one pass of the shared-memory port for most code patterns
+// (a code's bank is code mod 32), the 16 bytes of a float4 a lane at least four, and that port,
+// which the neighbour gathers use too, is what the mixed passes wait for most (80 % busy at
+// 2,048,000 atoms).  Measured, float4 / float2 + float / three floats: LJ forces of 2,048,000
+// atoms 526 / 520 / 511 us, of 128 systems of 6,400 atoms 226 / 222 / 218; 495,000 copper atoms'
+// forces 254 / 248 / 246 us, densities 159 / 152 / 147.
+template <int N = 125>
+struct ShiftTable {
+  float x[N], y[N], z[N];
+  __device__ __forceinline__ float4 operator[](unsigned code) const {
+    return make_float4(x[code], y[code], z[code], 0.f);
+  }
+};
+
+// Fills the table for system S (whole block).
+__device__ __forceinline__ void load_shifts(const SysDev& S, ShiftTable<>& sh) {
   for (int c = threadIdx.x; c < 125; c += blockDim.x) {
     int kx = c % 5 - 2, ky = (c / 5) % 5 - 2, kz = c / 25 - 2;
-    sh[c] = make_float4((float)kx * S.df[0], (float)ky * S.df[1], (float)kz * S.df[2], 0.0f);
+    sh.x[c] = (float)kx * S.df[0];
+    sh.y[c] = (float)ky * S.df[1];
+    sh.z[c] = (float)kz * S.df[2];
   }
   __syncthreads();
 }
@@ -80,7 +97,7 @@ __device__ __forceinline__ void load_shifts(const SysDev& S, float4* sh) {
 #define SHIFT_TABLE(name) const float4* __restrict__ name = D.shift_tab + (long long)s * 128
 #else
 #define SHIFT_TABLE(name)   \
-  __shared__ float4 name[125]; \
+  __shared__ ShiftTable<> name; \
   load_shifts(S, name)
 #endif
 
@@ -732,7 +749,7 @@ template <int PC, int SPECIES, int SCN, int SCM, int LANES>
 __global__ void __launch_bounds__(TILE, 8)
     k_force32_lanes(Dev D, PotParams P, StepParams sp, const Blk32* blk) {
   constexpr int APB = TILE / LANES;  // atoms per block
-  __shared__ float4 shifts[125];
+  __shared__ ShiftTable<> shifts;
   __shared__ long long fsum[3][APB];
   __shared__ long long esum[TILE / 32][16];
   const Blk32 B = blk[blockIdx.x];
@@ -1038,7 +1055,7 @@ template <int SCM, int LANES>
 __global__ void __launch_bounds__(TILE, 8)
     k_eam_density32_lanes(Dev D, PotParams P, const Blk32* blk) {
   constexpr int APB = TILE / LANES;
-  __shared__ float4 shifts[125];
+  __shared__ ShiftTable<> shifts;
   __shared__ long long rsum[APB];
   const Blk32 B = blk[blockIdx.x];
   const SysDev& S = D.sysd[B.sys];
