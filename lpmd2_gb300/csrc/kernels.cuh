@@ -565,7 +565,8 @@ __device__ __forceinline__ int shift_code(int kx, int ky, int kz) { return (kx +
 // batch rebuild in a step; the block's chain is a quarter of that.  Measured (block / warp per cell):
 // 125 cells (4,000 atoms) 25 / 69 us, 1,728 cells (32,000) 32 / 40, an ensemble of 128 systems
 // 88 / 159 us a step; but 5,832 cells (32,000 atoms of iron) 45.6 / 39.0, 12,167 (256k LJ liquid)
-// 173 / 157, 13,824 (495k copper) 590 / 569, 97,336 (2 M atoms) 1396 / 1146.  (The warp form with
+// 173 / 157, 13,824 (495k copper) 590 / 569, 97,336 (2 M atoms) 1396 / 1146 (the warp form's figures
+// from before its look-ups and loads ran ahead, see list_cell).  (The warp form with
 // its distance tests as compares and selects instead of shifted signs: 171, 629 and 1239.)
 constexpr int LIST_BLOCK_CELLS = 4096;
 constexpr int LIST_WARPS = 8;
@@ -792,10 +793,23 @@ __global__ void __launch_bounds__(32 * LIST_WARPS, 4) k_buildlist_block(Dev D, i
 // cell are staged through shared memory 32 at a time; every lane then tests the staged candidates
 // against its own atom (broadcast reads, no divergence between lanes, since all atoms of a cell share
 // the stencil and its cell-shift codes; the sign of r^2 - rl^2 shifts into a mask), and appends its
-// hits in candidate order.
+// hits in candidate order.  Bound by instruction issue (64 %, the integer unit 60 %), half of it
+// tests and half the appending, with latency behind.  The lanes look the stencil's cells up together,
+// and the next candidates are loaded while the last are tested; with 72 registers seven blocks fit
+// an SM.  Measured, a cell looked up at a time with its own load / this at 4 / 7 / 8 blocks an SM:
+// 2,048,000 LJ atoms 1167 / 1173 / 1092 / 1130 us, 107,963 75 / 72 / 69 / 74, 32,000 of iron
+// 40 / 34 / 33 / 37, 495,000 of copper 578 / 574 / 578 / 605.  (A group of four entries gathered
+// in registers and written as 16 bytes instead of an entry at a time: 1272 us for 2,048,000.)
 constexpr int LIST_CELLS = 4;  // home cells (warps) of a block
-__device__ __forceinline__ void list_cell(const Dev& D, const SysDev& S, int s, int c, float* stx, float* sty,
-                                          float* stz) {
+// A warp's shared memory: the staged candidates' coordinates as three arrays, so that one 16-byte
+// load gives the x (y, z) of four consecutive candidates (two packed pairs), and up to 32 cells of
+// the stencil: first atom (index within the system) and atoms, offset from the home cell and code bits.
+struct ListStage {
+  float x[32], y[32], z[32];
+  float4 shift[32];
+  int2 run[32];
+};
+__device__ __forceinline__ void list_cell(const Dev& D, const SysDev& S, int s, int c, ListStage& st) {
   const int lane = threadIdx.x & 31;
   // the system's grid in registers: the list stores below may alias any global memory, so
   // fields read through the SysDev reference would be re-read after every store
@@ -809,8 +823,9 @@ __device__ __forceinline__ void list_cell(const Dev& D, const SysDev& S, int s, 
   unsigned* const nl = D.nl + S.nl_base;
   const int* __restrict__ cstart = D.cstart;
   const int* __restrict__ ccnt = D.ccnt;
-  const float4* __restrict__ g32 = D.g32;
+  const float4* __restrict__ g32 = D.g32 + atom_base;
   const int maxnb = D.maxnb;
+  const int W = 2 * R + 1, nst = W * W * W;
   const int b0 = cstart[cell_base + c], n0 = ccnt[cell_base + c];
   const int cx = c % nx, cy = (c / nx) % ny, cz = c / (nx * ny);
   int most = 0;
@@ -818,71 +833,83 @@ __device__ __forceinline__ void list_cell(const Dev& D, const SysDev& S, int s, 
     const bool has = base + lane < n0;
     const long long i = (long long)b0 + base + lane;
     const int li = (int)(i - atom_base);
-    const float4 gi = has ? g32[i] : make_float4(0.f, 0.f, 0.f, 0.f);
+    const float4 gi = has ? g32[li] : make_float4(0.f, 0.f, 0.f, 0.f);
     const float out = has ? -rlist2 : 1.0f;  // lanes without an atom never match
     const f32x2 out2 = f2_pack(out, out);
     const long long gstride = (long long)na * 4;  // words between consecutive groups of four
     int cnt = 0;
     unsigned* wp = nl + (long long)li * 4;
-    for (int dz = -R; dz <= R; ++dz) {
-      const int zc = wrap_around(cz + dz, nz);
-      const float sz = (float)dz * dfz;
-      for (int dy = -R; dy <= R; ++dy) {
-        const int yc = wrap_around(cy + dy, ny);
-        const float sy = (float)dy * dfy;
-        for (int dx = -R; dx <= R; ++dx) {
-          const int xc = wrap_around(cx + dx, nx);
-          const float sx = (float)dx * dfx;
-          const int g = cell_base + (zc * ny + yc) * nx + xc;
-          const int b = cstart[g], n = ccnt[g];
-          const unsigned code = (unsigned)shift_code(dx, dy, dz) << CODE_SHIFT;
-          const float ox = sx - gi.x, oy = sy - gi.y, oz = sz - gi.z;
-          const f32x2 ox2 = f2_pack(ox, ox), oy2 = f2_pack(oy, oy), oz2 = f2_pack(oz, oz);
-          for (int jb = 0; jb < n; jb += 32) {
-            __syncwarp();
-            {
-              const float4 gj = jb + lane < n ? g32[b + jb + lane] : make_float4(1e18f, 1e18f, 1e18f, 0.f);
-              stx[lane] = gj.x;
-              sty[lane] = gj.y;
-              stz[lane] = gj.z;
-            }
-            __syncwarp();
-            const int m = min(32, n - jb);
-            const int jl0 = b + jb - (int)atom_base;
-            // pass 1: a bit per staged candidate inside the list radius (branch-free), candidate k
-            // in bit 31 - k
-            unsigned hits = 0u;
-            for (int k = 0; k < m; k += 4) {
-              // candidates k..k+3 as two packed pairs
-              const float4 X = *reinterpret_cast<const float4*>(stx + k);
-              const float4 Y = *reinterpret_cast<const float4*>(sty + k);
-              const float4 Z = *reinterpret_cast<const float4*>(stz + k);
-              const f32x2 rx01 = f2_add(ox2, f2_pack(X.x, X.y)), rx23 = f2_add(ox2, f2_pack(X.z, X.w));
-              const f32x2 ry01 = f2_add(oy2, f2_pack(Y.x, Y.y)), ry23 = f2_add(oy2, f2_pack(Y.z, Y.w));
-              const f32x2 rz01 = f2_add(oz2, f2_pack(Z.x, Z.y)), rz23 = f2_add(oz2, f2_pack(Z.z, Z.w));
-              const f32x2 q01 = f2_fma(rx01, rx01, f2_fma(ry01, ry01, f2_mul(rz01, rz01)));
-              const f32x2 q23 = f2_fma(rx23, rx23, f2_fma(ry23, ry23, f2_mul(rz23, rz23)));
-              float d0, d1, d2, d3;  // r^2 - rl^2, whose sign no rounding changes
-              f2_unpack(f2_add(q01, out2), d0, d1);
-              f2_unpack(f2_add(q23, out2), d2, d3);
-              hits = __funnelshift_l(__float_as_uint(d0), hits, 1);
-              hits = __funnelshift_l(__float_as_uint(d1), hits, 1);
-              hits = __funnelshift_l(__float_as_uint(d2), hits, 1);
-              hits = __funnelshift_l(__float_as_uint(d3), hits, 1);
-            }
-            hits <<= 32 - ((m + 3) & ~3);
-            const int self = li - jl0;  // drop the atom itself
-            if (self >= 0 && self < 32) hits &= ~(0x80000000u >> self);
-            // pass 2: append the hits in candidate order
-            while (hits) {
-              const int k = __clz(hits);
-              hits ^= 0x80000000u >> k;
-              // running write position: entry cnt of the atom lives at group cnt/4, slot cnt%4
-              if (cnt < maxnb) *wp = code | (unsigned)(jl0 + k);
-              wp += (cnt & 3) == 3 ? gstride - 3 : 1;
-              ++cnt;
-            }
-          }
+    for (int t0 = 0; t0 < nst; t0 += 32) {
+      __syncwarp();
+      if (t0 + lane < nst) {
+        const int t = t0 + lane, dx = t % W - R, dy = (t / W) % W - R, dz = t / (W * W) - R;
+        const int xc = wrap_around(cx + dx, nx), yc = wrap_around(cy + dy, ny), zc = wrap_around(cz + dz, nz);
+        const int g = cell_base + (zc * ny + yc) * nx + xc;
+        st.run[lane] = make_int2((int)(cstart[g] - atom_base), ccnt[g]);
+        st.shift[lane] = make_float4((float)dx * dfx, (float)dy * dfy, (float)dz * dfz,
+                                     __uint_as_float((unsigned)shift_code(dx, dy, dz) << CODE_SHIFT));
+      }
+      __syncwarp();
+      const int cells = min(32, nst - t0);
+      // the next 32 candidates (of one cell) on their way while the last are tested
+      int t = -1, from = 0, left = 0;
+      float4 gj;
+      auto fetch = [&]() -> bool {
+        while (left <= 0) {
+          if (++t >= cells) return false;
+          const int2 run = st.run[t];
+          from = run.x;
+          left = run.y;
+        }
+        gj = lane < left ? g32[from + lane] : make_float4(1e18f, 1e18f, 1e18f, 0.f);
+        return true;
+      };
+      for (bool more = fetch(); more;) {
+        __syncwarp();
+        st.x[lane] = gj.x;
+        st.y[lane] = gj.y;
+        st.z[lane] = gj.z;
+        __syncwarp();
+        const int m = min(32, left), jl0 = from;
+        const float4 sh = st.shift[t];
+        const unsigned code = __float_as_uint(sh.w);
+        from += 32;
+        left -= 32;
+        more = fetch();
+        const float ox = sh.x - gi.x, oy = sh.y - gi.y, oz = sh.z - gi.z;
+        const f32x2 ox2 = f2_pack(ox, ox), oy2 = f2_pack(oy, oy), oz2 = f2_pack(oz, oz);
+        // pass 1: a bit per staged candidate inside the list radius (branch-free), candidate k
+        // in bit 31 - k
+        unsigned hits = 0u;
+        for (int k = 0; k < m; k += 4) {
+          // candidates k..k+3 as two packed pairs
+          const float4 X = *reinterpret_cast<const float4*>(st.x + k);
+          const float4 Y = *reinterpret_cast<const float4*>(st.y + k);
+          const float4 Z = *reinterpret_cast<const float4*>(st.z + k);
+          const f32x2 rx01 = f2_add(ox2, f2_pack(X.x, X.y)), rx23 = f2_add(ox2, f2_pack(X.z, X.w));
+          const f32x2 ry01 = f2_add(oy2, f2_pack(Y.x, Y.y)), ry23 = f2_add(oy2, f2_pack(Y.z, Y.w));
+          const f32x2 rz01 = f2_add(oz2, f2_pack(Z.x, Z.y)), rz23 = f2_add(oz2, f2_pack(Z.z, Z.w));
+          const f32x2 q01 = f2_fma(rx01, rx01, f2_fma(ry01, ry01, f2_mul(rz01, rz01)));
+          const f32x2 q23 = f2_fma(rx23, rx23, f2_fma(ry23, ry23, f2_mul(rz23, rz23)));
+          float d0, d1, d2, d3;  // r^2 - rl^2, whose sign no rounding changes
+          f2_unpack(f2_add(q01, out2), d0, d1);
+          f2_unpack(f2_add(q23, out2), d2, d3);
+          hits = __funnelshift_l(__float_as_uint(d0), hits, 1);
+          hits = __funnelshift_l(__float_as_uint(d1), hits, 1);
+          hits = __funnelshift_l(__float_as_uint(d2), hits, 1);
+          hits = __funnelshift_l(__float_as_uint(d3), hits, 1);
+        }
+        hits <<= 32 - ((m + 3) & ~3);
+        const int self = li - jl0;  // drop the atom itself
+        if (self >= 0 && self < 32) hits &= ~(0x80000000u >> self);
+        // pass 2: append the hits in candidate order
+        while (hits) {
+          const int k = __clz(hits);
+          hits ^= 0x80000000u >> k;
+          // running write position: entry cnt of the atom lives at group cnt/4, slot cnt%4
+          if (cnt < maxnb) *wp = code | (unsigned)(jl0 + k);
+          wp += (cnt & 3) == 3 ? gstride - 3 : 1;
+          ++cnt;
         }
       }
     }
@@ -898,15 +925,13 @@ __device__ __forceinline__ void list_cell(const Dev& D, const SysDev& S, int s, 
   }
 }
 
-__global__ void __launch_bounds__(32 * LIST_CELLS, 4) k_buildlist_warp(Dev D) {
-  // coordinates staged as three arrays, so that one 16-byte shared load gives the x (y, z)
-  // of four consecutive candidates: two packed pairs
-  __shared__ __align__(16) float stage[LIST_CELLS][3][32];
+__global__ void __launch_bounds__(32 * LIST_CELLS, 7) k_buildlist_warp(Dev D) {
+  __shared__ __align__(16) ListStage stage[LIST_CELLS];
   const int w = threadIdx.x >> 5;
   int s, c;
   for (int u = blockIdx.x * LIST_CELLS + w; rebuild_unit<true>(D, u, s, c); u += gridDim.x * LIST_CELLS)
     if (D.sysd[s].mode == NB_LIST && D.sysd[s].ncells > LIST_BLOCK_CELLS)
-      list_cell(D, D.sysd[s], s, c, stage[w][0], stage[w][1], stage[w][2]);
+      list_cell(D, D.sysd[s], s, c, stage[w]);
 }
 
 // ---------------------------------------------------------------------------------------------
