@@ -563,11 +563,9 @@ __device__ __forceinline__ int shift_code(int kx, int ky, int kz) { return (kx +
 // A warp per cell needs fewer instructions an atom, but is a serial chain 27 cells long, which is
 // all there is where the grid does not fill the GPU several times over, or where a few systems of a
 // batch rebuild in a step; the block's chain is a quarter of that.  Measured (block / warp per cell):
-// 125 cells (4,000 atoms) 25 / 69 us, 1,728 cells (32,000) 32 / 40, an ensemble of 128 systems
-// 88 / 159 us a step; but 5,832 cells (32,000 atoms of iron) 45.6 / 39.0, 12,167 (256k LJ liquid)
-// 173 / 157, 13,824 (495k copper) 590 / 569, 97,336 (2 M atoms) 1396 / 1146 (the warp form's figures
-// from before its look-ups and loads ran ahead, see list_cell).  (The warp form with
-// its distance tests as compares and selects instead of shifted signs: 171, 629 and 1239.)
+// 729 cells (16,000 LJ atoms) 24 / 29 us, 1,728 (32,000) 31 / 30, 3,375 (54,000 of copper) 109 / 114,
+// an ensemble of 128 systems 95 / 125 us a step; but 5,832 (32,000 of iron) 46 / 33, 13,824
+// (495,000 of copper) 590 / 578, 97,336 (2 M LJ atoms) 1396 / 1092.
 constexpr int LIST_BLOCK_CELLS = 4096;
 constexpr int LIST_WARPS = 8;
 constexpr int LIST_STAGE = 1024;
