@@ -185,8 +185,9 @@ gbmd_status gbmd_sim_set_precision(gbmd_sim* sim, int precision);
  *                      energies and virials bit for bit; stress moves by FP32 rounding).  Unset,
  *                      as many as keep every block resident: 8 to 2 for small systems, else 1
  *   "list_feed"        how the mixed passes read their Verlet-list rows: 0 auto (default:
- *                      registers for a single EAM system, a shared-memory ring of bulk copies
- *                      otherwise), 1 registers, 2 ring (the same results either way) */
+ *                      registers for the density pass of a single EAM system and, but for the
+ *                      common Sutton-Chen metals, its force pass; a shared-memory ring of bulk
+ *                      copies otherwise), 1 registers, 2 ring (the same results either way) */
 gbmd_status gbmd_sim_set_option(gbmd_sim* sim, const char* key, const char* value);
 
 /* CombinedPotential::UpdateForces (liblpmd/lpmd/combinedpotential.h:39-52): zeroes

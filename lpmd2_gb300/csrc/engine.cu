@@ -1124,14 +1124,20 @@ struct Engine::Impl {
       const bool sc126 = P.kind == POT_SC && P.int_n == 12 && P.int_m == 6;
       PotParams Pe = P;
       Pe.f[14] = (!species && (sc96 || sc126)) ? P.f[2] : 1.0f;  // scale of the density pass's copy
-      // list rows through the shared-memory ring for ensembles and pair potentials, through
-      // registers for a single EAM system (the faster of the two on the GB300 for each), unless
-      // the option says otherwise
-      const bool ring = list_feed == 2 || (list_feed == 0 && (nsys > 1 || pair_kind(P.kind)));
+      // list rows through the shared-memory ring, in a single system through registers for the
+      // density pass and the force pass of the metals without compiled powers (the faster of the
+      // two on the GB300 for each), unless the option says otherwise.  Measured (us, registers /
+      // ring): copper 9/6 forces 64.0 / 63.0 at 103,000 atoms, 112.3 / 110.6 at 181,624, 245.5 /
+      // 240.7 at 495,000, 475 / 472 at 1,043,576, its densities there 41.2 / 40.6, 82.4 / 73.8,
+      // 147.0 / 154.5, 292 / 307; iron 126.3 / 126.7 and 49.8 / 51.2 at 499,987; LJ forces 547 /
+      // 513 at 2,048,000
+      const bool compiled = (sc96 || sc126) && !species;
+      const bool ring = list_feed == 2 || (list_feed == 0 && (nsys > 1 || pair_kind(P.kind) || compiled));
+      const bool ring_rho = list_feed == 2 || (list_feed == 0 && nsys > 1);
       if (!pair_kind(P.kind)) {
         int first = (p == first_eam);
         if (mixed)
-          launch_density32(s, Pe, ring);
+          launch_density32(s, Pe, ring_rho);
         else
           launch_density64(s, P, mode, first);
         launched();
@@ -1612,7 +1618,7 @@ struct Engine::Impl {
       // once there are enough of them to pay for the capture (LJ liquid of 16,384 atoms under Beeman:
       // 74 us a step launched, 51 captured)
       int64_t done = 0;
-      const int gbe = lcb_exact() || graph_mode == 0 ? 0 : graph_block & ~1;
+      const int gbe = lcb_exact() || graph_mode == 0 || time_kernels ? 0 : graph_block & ~1;  // timed launches are direct
       if (gbe > 0 && pending_ucalls > 0) {
         step_plain();  // the UpdateCell calls owed to the set-up
         ++done;

