@@ -321,13 +321,14 @@ __device__ __forceinline__ T warp_sum(T v) {
   return v;
 }
 
-// Sums 16 values per lane over the warp with 16 additions a lane: each exchange halves the values
-// a lane carries.  Lane l returns the total of value l >> 1.
-template <typename T>
-__device__ __forceinline__ T warp_sum16(T (&v)[16]) {
+// Sums N values per lane (4, 8 or 16) over the warp with N + log2(32 / N) - 1 additions a lane: each
+// exchange halves the values a lane carries.  Lane l returns the total of value l * N / 32, added in
+// the order of warp_sum.
+template <typename T, int N>
+__device__ __forceinline__ T warp_sums(T (&v)[N]) {
   const int lane = threadIdx.x & 31;
 #pragma unroll
-  for (int h = 8, m = 16; h > 0; h >>= 1, m >>= 1) {
+  for (int h = N / 2, m = 16; h > 0; h >>= 1, m >>= 1) {
     const bool up = (lane & m) != 0;
 #pragma unroll
     for (int k = 0; k < h; ++k) {
@@ -335,7 +336,10 @@ __device__ __forceinline__ T warp_sum16(T (&v)[16]) {
       v[k] = keep + __shfl_xor_sync(0xffffffffu, send, m);
     }
   }
-  return v[0] + __shfl_xor_sync(0xffffffffu, v[0], 1);
+  T t = v[0];
+#pragma unroll
+  for (int m = 16 / N; m > 0; m >>= 1) t += __shfl_xor_sync(0xffffffffu, t, m);
+  return t;
 }
 
 // Deterministic block sum of NV values per thread; thread 0 gets the totals in out[].

@@ -369,7 +369,7 @@ __global__ void __launch_bounds__(TILE, 5) k_force64(Dev D, PotParams P, Pair64 
   }
   track_displacement_warp(D, B.sys, d2);
   double v[16] = {ep, sxx, sxy, sxz, syy, syz, szz, ke, px, py, pz, 0.0, 0.0, 0.0, 0.0, 0.0};
-  const double s = warp_sum16(v);
+  const double s = warp_sums(v);
   if ((lane & 1) == 0) red[w][lane >> 1] = s;
   __syncthreads();
   if (threadIdx.x < 11) {

@@ -150,14 +150,23 @@ __device__ __forceinline__ float finish_atom(const Dev& D, const SysDev& S, long
 }
 
 // Kinetic energy and momentum of the calling warp's atoms as int64 fixed point (2^-44 units):
-// FP64 warp sums in a fixed shuffle order, rounded once, on lane 0 (zeros elsewhere).  A warp
+// FP64 warp sums in a fixed shuffle order, rounded once; lane l returns value l / 8 of the four.  A warp
 // never spans two systems (tiles start at a system's first atom), so the sums are the same in a
 // batch and alone.
-__device__ __forceinline__ void warp_kinetic_fix(double ke, double px, double py, double pz, long long (&k4)[4]) {
-  const double s[4] = {warp_sum(ke), warp_sum(px), warp_sum(py), warp_sum(pz)};
-  const bool lead = (threadIdx.x & 31) == 0;
+__device__ __forceinline__ long long warp_kinetic_fix(double ke, double px, double py, double pz) {
+  double v[4] = {ke, px, py, pz};
+  return __double2ll_rn(warp_sums(v) * FIX_KE);
+}
+
+// The eight sums of a mixed pass -- energy, virial, and the stress's xx, xy, xz, yy, yz, zz -- as
+// the system's eleven accumulator slots hold them: the sum that goes to slot k.
+__device__ __forceinline__ int sum_of_slot(int k) {
+  const int from[11] = {0, 1, 2, 3, 4, 3, 5, 6, 4, 6, 7};
+  int f = 0;
 #pragma unroll
-  for (int k = 0; k < 4; ++k) k4[k] = lead ? __double2ll_rn(s[k] * FIX_KE) : 0ll;
+  for (int q = 0; q < 11; ++q)
+    if (k == q) f = from[q];
+  return f;
 }
 
 // ------------------------------------------------------------------------------------------
@@ -678,29 +687,33 @@ __device__ __forceinline__ void force32_tile(const Dev& D, const PotParams& P, c
   }
   track_displacement_warp(D, s, d2);
   // energy and virial already in fixed point; per-atom stress (halved: full list) rounded to
-  // int64 once; exact block sums and one integer atomic per quantity into the system's slots
-  const float ms = (float)(-0.5 * FIX_E);
-  long long v[11] = {fqe.value() * 64, fqv.value() * 64, fix64(sxx * ms), fix64(sxy * ms), fix64(sxz * ms),
-                     fix64(sxy * ms), fix64(syy * ms), fix64(syz * ms), fix64(sxz * ms), fix64(syz * ms),
-                     fix64(szz * ms)};
-  long long tot[11];
-  block_sum<long long, 11>(v, tot);
-  if (threadIdx.x == 0) {
-    unsigned long long* acc = D.sys_acc + (long long)s * SA_LEN;
-    for (int k = 0; k < 11; ++k) atomicAdd(acc + k, (unsigned long long)tot[k]);
-  }
-  if (sp.last) {
-    // kinetic energy and momentum: FP64 warp sums in a fixed order, rounded once per warp to
-    // int64 (2^-44 units); exact int64 sums from there on
-    long long k4[4];
-    warp_kinetic_fix(ke, px, py, pz, k4);
-    long long kt[4];
-    block_sum<long long, 4>(k4, kt);
-    if (threadIdx.x == 0) {
-      unsigned long long* acc = D.sys_acc + (long long)s * SA_LEN;
-      atomicAdd(acc + SA_KE, (unsigned long long)kt[0]);
-      for (int k = 0; k < 3; ++k) atomicAdd(acc + SA_P + k, (unsigned long long)kt[1 + k]);
+  // int64 once, kinetic energy and momentum as FP64 warp sums in a fixed order rounded once per warp;
+  // exact int64 sums from there on, one integer atomic per quantity into the system's slots.  The warp
+  // sums halve the values a lane carries with each exchange: 9 additions a lane instead of 55 for the
+  // eight integers, 6 on the FP64 unit instead of 20 for the four kinetic ones (a third of the
+  // epilogue's FP64 instructions with their roundings).
+  __shared__ long long esum[TILE / 32][8], ksum[TILE / 32][4];
+  {
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const float ms = (float)(-0.5 * FIX_E);
+    long long v[8] = {fqe.value() * 64, fqv.value() * 64, fix64(sxx * ms), fix64(sxy * ms), fix64(sxz * ms),
+                      fix64(syy * ms),  fix64(syz * ms),  fix64(szz * ms)};
+    const long long t = warp_sums(v);
+    if ((lane & 3) == 0) esum[w][lane >> 2] = t;
+    if (sp.last) {
+      const long long k = warp_kinetic_fix(ke, px, py, pz);
+      if ((lane & 7) == 0) ksum[w][lane >> 3] = k;
     }
+  }
+  __syncthreads();
+  const int slot = threadIdx.x;
+  if (slot < (sp.last ? 15 : 11)) {
+    const long long* from = slot < 11 ? &esum[0][sum_of_slot(slot)] : &ksum[0][slot - 11];
+    const int stride = slot < 11 ? 8 : 4;
+    long long t = 0;
+    for (int w = 0; w < TILE / 32; ++w) t += from[w * stride];
+    static_assert(SA_STRESS == 2 && SA_KE == 11 && SA_P == 12, "slots in the order of the sums");
+    atomicAdd(D.sys_acc + (long long)s * SA_LEN + slot, (unsigned long long)t);
   }
 }
 
@@ -750,7 +763,7 @@ __global__ void __launch_bounds__(TILE, 8)
   constexpr int APB = TILE / LANES;  // atoms per block
   __shared__ ShiftTable<> shifts;
   __shared__ long long fsum[3][APB];
-  __shared__ long long esum[TILE / 32][16];
+  __shared__ long long esum[TILE / 32][8];
   const Blk32 B = blk[blockIdx.x];
   const int s = B.sys;
   const SysDev& S = D.sysd[s];
@@ -890,20 +903,16 @@ __global__ void __launch_bounds__(TILE, 8)
   if (bad) atomicOr(&D.sst[s].error, ERR_FIXED);
   // energy and virial: every lane's own fixed-point partial (exact integer sums, whatever the lane
   // count)
-  long long v[16] = {fqe.value() * 64, fqv.value() * 64, fix64(sxx * ms), fix64(sxy * ms), fix64(sxz * ms),
-                     fix64(syy * ms), fix64(syz * ms), fix64(szz * ms), 0, 0, 0, 0, 0, 0, 0, 0};
-  const long long t16 = warp_sum16(v);
-  if ((lane & 1) == 0) esum[w][lane >> 1] = t16;
+  long long v[8] = {fqe.value() * 64, fqv.value() * 64, fix64(sxx * ms), fix64(sxy * ms), fix64(sxz * ms),
+                    fix64(syy * ms),  fix64(syz * ms),  fix64(szz * ms)};
+  const long long t8 = warp_sums(v);
+  if ((lane & 3) == 0) esum[w][lane >> 2] = t8;
   __syncthreads();
   unsigned long long* acc = D.sys_acc + (long long)s * SA_LEN;
   if (threadIdx.x >= TILE - 32 && lane < 11) {
     // energy, virial and the nine stress slots from the eight sums (in the last warp: the first ones
     // go on with the atoms)
-    const int from[11] = {0, 1, 2, 3, 4, 3, 5, 6, 4, 6, 7};
-    int f = 0;
-#pragma unroll
-    for (int k = 0; k < 11; ++k)
-      if (lane == k) f = from[k];
+    const int f = sum_of_slot(lane);
     long long t = 0;
     for (int k = 0; k < TILE / 32; ++k) t += esum[k][f];
     atomicAdd(acc + lane, (unsigned long long)t);
@@ -930,12 +939,8 @@ __global__ void __launch_bounds__(TILE, 8)
   }
   track_displacement_warp(D, s, d2);
   if (sp.last) {
-    long long k4[4];
-    warp_kinetic_fix(ke, px, py, pz, k4);
-    if (lane == 0) {
-      atomicAdd(acc + SA_KE, (unsigned long long)k4[0]);
-      for (int k = 0; k < 3; ++k) atomicAdd(acc + SA_P + k, (unsigned long long)k4[1 + k]);
-    }
+    const long long k = warp_kinetic_fix(ke, px, py, pz);
+    if ((lane & 7) == 0) atomicAdd(acc + SA_KE + (lane >> 3), (unsigned long long)k);  // SA_P follows SA_KE
   }
 }
 

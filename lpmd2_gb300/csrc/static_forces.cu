@@ -112,7 +112,7 @@ __global__ void __launch_bounds__(32 * ST_WARPS)
     if ((lane & 7) == 0 && lane < 24) force[3 * i + (lane >> 3)] = f;
   }
   double v[16] = {ep, sxx, sxy, sxz, syy, syz, szz, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
-  const double t = warp_sum16(v);
+  const double t = warp_sums(v);
   if ((lane & 1) == 0 && lane < 16) red[w][lane >> 1] = t;
   __syncthreads();
   if (threadIdx.x < 8) {
