@@ -691,7 +691,8 @@ __device__ __forceinline__ void force32_tile(const Dev& D, const PotParams& P, c
   // exact int64 sums from there on, one integer atomic per quantity into the system's slots.  The warp
   // sums halve the values a lane carries with each exchange: 9 additions a lane instead of 55 for the
   // eight integers, 6 on the FP64 unit instead of 20 for the four kinetic ones (a third of the
-  // epilogue's FP64 instructions with their roundings).
+  // epilogue's FP64 instructions with their roundings): 2,048,000 LJ atoms 511 -> 473 us, 495,000 of
+  // copper 241 -> 233, 128 systems 218 -> 200.
   __shared__ long long esum[TILE / 32][8], ksum[TILE / 32][4];
   {
     const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
