@@ -3,11 +3,11 @@
 // What bounds them: GB300's FP64 unit takes 16 clocks per warp instruction and SM (2 lanes a
 // clock), so the number of FP64 instructions a warp issues is the time; FP32, integer and memory
 // work beside them is nearly free.  So
-//   * candidates are tested in FP32 (list mode: cell-relative offsets, with a guard band; stencil and
-//     all-pairs modes: a lower bound of the distance from truncated coordinates), and only pairs that
-//     pass reach the FP64 unit, where the reference's own cutoff test decides each of them (the FP32
-//     test sees the nearest image, the reference the one it reaches with a single wrap: for atoms
-//     outside the box they may differ by box lengths);
+//   * candidates are tested in FP32 against a lower bound of their distance (list mode: the nearest
+//     image from cell-relative offsets; stencil and all-pairs modes: truncated coordinates), and only
+//     pairs that pass reach the FP64 unit, where the reference's own cutoff test decides each of them
+//     (its distance is that of the image it reaches with a single wrap: for atoms outside the box
+//     that may be box lengths further than the nearest);
 //   * the passing pairs of an atom are queued in shared memory and shared out over the atom's
 //     lanes, so that a warp's FP64 instructions run with nearly all lanes at work whatever the
 //     lists' lengths (8 lanes an atom: an LJ liquid's 55 pairs fill 7 rounds of 8);
@@ -167,6 +167,14 @@ __device__ __forceinline__ void scan64(const Dev& D, const SysDev& S, int li, bo
     const float4* __restrict__ g32 = D.g32 + S.atom_base;
     const float4 gi = active ? g32[li] : make_float4(0.f, 0.f, 0.f, 0.f);
     const int cnt = active ? D.ncount[i] : 0;
+    // The entry's image was the nearest when the list was built; on the clock of an `each` manager it
+    // need not be any more, so each component is folded once (exact where it does not fold).  A
+    // component is off by at most tol: roundings of the two offsets (box lengths, for atoms far
+    // outside), the shift, the box edge and their sums.
+    const float Lx = (float)S.L[0], Ly = (float)S.L[1], Lz = (float)S.L[2];
+    const float tol = 1e-6f * (fmaxf(fabsf(gi.x), fmaxf(fabsf(gi.y), fabsf(gi.z))) + fmaxf(Lx, fmaxf(Ly, Lz)));
+    const float far2 = hi + tol * fmaf(3.5f, sqrtf(hi), 3.0f * tol);  // (sqrt(hi) + sqrt(3) tol)^2
+    auto fold = [](float d, float L) { return fminf(fabsf(d), fabsf(fabsf(d) - L)); };
     const int ng = (cnt + 3) >> 2;
     const int ngw = (int)__reduce_max_sync(all, (unsigned)ng);
     const uint4* L = list_group(D, S, li, 0);
@@ -183,8 +191,11 @@ __device__ __forceinline__ void scan64(const Dev& D, const SysDev& S, int li, bo
         const unsigned j = e[u] & LOCAL_MASK;
         const float4 gj = valid ? g32[j] : gi;
         float dx, dy, dz;
-        const float r2 = entry_r2(gi, gj, shifts[e[u] >> CODE_SHIFT], corr, dx, dy, dz);
-        in[u] = valid && r2 < hi && (spc_sum < 0 || applies_to(spc_sum, __float_as_int(gi.w), __float_as_int(gj.w)));
+        entry_r2(gi, gj, shifts[e[u] >> CODE_SHIFT], corr, dx, dy, dz);
+        dx = fold(dx, Lx);
+        dy = fold(dy, Ly);
+        dz = fold(dz, Lz);
+        in[u] = valid && fmaf(dx, dx, fmaf(dy, dy, dz * dz)) < far2 && (spc_sum < 0 || applies_to(spc_sum, __float_as_int(gi.w), __float_as_int(gj.w)));
         w[u] = j;
       }
 #pragma unroll

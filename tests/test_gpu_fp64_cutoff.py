@@ -3,7 +3,8 @@ test look at different distances.
 
 The reference wraps a difference of coordinates once, wherever the atoms are.  The list's FP32 offsets
 see the nearest image.  Positions are not folded into the box when they are set, and atoms with a fixed
-position never are, so the two differ by box lengths.  Tolerances are those of the FP64 path elsewhere:
+position never are, so the two differ by box lengths; and a list on the `each` clock alone outlives the images
+that it was built with.  Tolerances are those of the FP64 path elsewhere:
 forces and energies 1e-12, virial 1e-11 relative.
 """
 import numpy as np
@@ -99,4 +100,47 @@ def test_a_fixed_atom_outside_the_box_over_steps():
     assert sim.stats()["neighbor_mode"] == "verlet"
     assert np.array_equal(sim.atoms()[0][[7, 123]], pos[[7, 123]])
     agree(sim, ref, 1e-11)  # five steps pass the forces' rounding on
+    sim.close()
+
+
+def test_a_list_that_outlives_its_images():
+    """Layers sliding along x for longer than the list is valid: pairs listed through one image come
+    inside through the other, which the reference, wrapping afresh, then takes."""
+    L = np.full(3, 20.0)
+    k = np.arange(4) * 5.0
+    pos = np.stack(np.meshgrid(k, k, k, indexing="ij"), -1).reshape(-1, 3)
+    odd = (pos[:, 1] / 5.0).astype(int) % 2 == 1
+    pos[odd, 0] += 2.6
+    pos = np.mod(I.jitter(pos, 0.1, seed=3), L)
+    vel = np.zeros_like(pos)
+    vel[:, 0] = np.where(odd, 0.04, -0.04)
+    rc = 8.5
+    pot = ("lennardjones", f"sigma 3.405 epsilon 0.0103 cutoff {rc}")
+    sim, ref = pair_of(pos, L, pot, "verletlist", "cutoff 8.5 maxneighbors 400 each 100000", mass=1000.0, vel=vel)
+    # the same list without libgbmd's own rebuild on displacement
+    sim.set_cell_manager(gbmd.Plugin("verletlist", f"cutoff 8.5 skin {0.08 * rc!r} maxneighbors 400 each 100000 rebuild each"))
+    sim.update_forces()
+    agree(sim, ref)
+    before = sim.stats()["list_rebuilds"]
+    sim.do_steps(80)
+    ref.do_steps(80)
+    assert sim.stats()["list_rebuilds"] == before and sim.stats()["neighbor_mode"] == "verlet"
+    agree(sim, ref, 1e-11)
+    sim.close()
+
+
+def test_coordinates_many_box_lengths_outside():
+    """Pairs within 3e-5 of the cutoff, five box lengths up: FP32 offsets resolve 1e-4 A there."""
+    L = np.full(3, 400.0)
+    k = 12.0 + 25.0 * np.arange(15)
+    first = np.stack(np.meshgrid(k, k[:5], k[:4], indexing="ij"), -1).reshape(-1, 3)
+    rng = np.random.default_rng(5)
+    u = rng.normal(size=first.shape)
+    u /= np.linalg.norm(u, axis=1)[:, None]
+    second = first + u * (RC * (1.0 + np.linspace(-3e-5, 3e-5, len(first))))[:, None]
+    pos = np.concatenate([first, second]) + 5.0 * L
+    name, args, rc, _, _ = POTS["lj"]
+    sim, ref = pair_of(pos, L, (name, args), "verletlist", list_manager("verletlist", rc, L))
+    assert sim.stats()["neighbor_mode"] == "verlet"
+    agree(sim, ref)
     sim.close()
