@@ -280,9 +280,7 @@ __device__ __forceinline__ bool pair_geometry64(const double4_32a& pi, const dou
   dy = dsub(pj.y, pi.y);
   dz = dsub(pj.z, pi.z);
   const bool wx = wraps_bits(dx, lhb[0]), wy = wraps_bits(dy, lhb[1]), wz = wraps_bits(dz, lhb[2]);
-  // a vote, so that the subtractions are branched over, not issued under a predicate, in the
-  // warps without such a pair (most of them)
-  if (__any_sync(__activemask(), wx || wy || wz)) {
+  if (wx || wy || wz) {
     if (wx) dx = dsub(dx, copysign(S.L[0], dx));
     if (wy) dy = dsub(dy, copysign(S.L[1], dy));
     if (wz) dz = dsub(dz, copysign(S.L[2], dz));
