@@ -145,6 +145,7 @@ struct Dev {
   int* rb_sys;
   int* rb_chunk0;
   int* rb_cell0;
+  int* outside;  // per system: at the last re-sort some atom was outside [0, L] (list mode)
   // permutation scratch
   double* sdbl;   // 11*N doubles
   // integrator history of the integrators other than velocityverlet (IST_K*N doubles, moved
@@ -216,15 +217,19 @@ __device__ __forceinline__ double ref_sq(double x, double y, double z) {
   return dadd(dadd(dmul(x, x), dmul(y, y)), dmul(z, z));
 }
 
+// Whether v is outside [0, L] on the bit patterns (what ref_fitted folds; NaN too).
+__device__ __forceinline__ bool outside_bits(double v, double L) {
+  const long long b = __double_as_longlong(v);
+  return (b < 0 && b != (long long)0x8000000000000000ULL) || b > __double_as_longlong(L);
+}
+
 // One axis of OrthogonalCell::FittedInside (liblpmd/lpmd/orthogonalcell.h:102-114).
 // The test (v < 0.0 || v > L) is decided on the bit patterns with integer compares instead of
 // two compares on GB300's scarce FP64 pipe: v < 0 <=> sign bit set and v is not -0.0; for
 // v >= +0, v > L <=> bits(v) > bits(L).  (A NaN is wrapped here and not in the reference; it
 // stays NaN either way.)
 __device__ __forceinline__ double ref_fitted(double v, double L) {
-  const long long b = __double_as_longlong(v);
-  if ((b < 0 && b != (long long)0x8000000000000000ULL) || b > __double_as_longlong(L))
-    v = dsub(v, dmul(L, floor(ddiv(v, L))));
+  if (outside_bits(v, L)) v = dsub(v, dmul(L, floor(ddiv(v, L))));
   return v;
 }
 

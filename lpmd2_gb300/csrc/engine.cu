@@ -742,6 +742,7 @@ struct Engine::Impl {
     D.tile_sys = d_tile_sys;
     D.tile_first = d_tile_first;
     D.tile_count = d_tile_count;
+    D.outside = alloc_work<int>(nsys);
     if (nsys > 1) {
       D.rb_n = alloc_work<int>(1);
       D.rb_sys = alloc_work<int>(nsys);
@@ -2262,6 +2263,7 @@ void Engine::checkpoint_load(const void* buf, size_t bytes) {
       CK(cudaMemcpyAsync(a.first, in, a.second, cudaMemcpyHostToDevice, I.stream));
       in += a.second;
     }
+  CK(cudaMemsetAsync(I.D.outside, 1, sizeof(int) * I.nsys, I.stream));  // unknown until the next re-sort
   CK(cudaStreamSynchronize(I.stream));
   I.sysd = sysd;
   I.read_from = rf;

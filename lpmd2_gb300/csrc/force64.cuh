@@ -5,9 +5,10 @@
 // work beside them is nearly free.  So
 //   * candidates are tested in FP32 against a lower bound of their distance (list mode: the nearest
 //     image from cell-relative offsets; stencil and all-pairs modes: truncated coordinates), and only
-//     pairs that pass reach the FP64 unit, where the reference's own cutoff test decides each of them
-//     (its distance is that of the image it reaches with a single wrap: for atoms outside the box
-//     that may be box lengths further than the nearest);
+//     pairs that pass reach the FP64 unit, where the reference's own cutoff test decides those that
+//     FP32 cannot.  FP32 can where a listed pair is inside by more than its error and every atom of the
+//     system is in the box: the reference's distance is that of the image it reaches with a single
+//     wrap, which for atoms outside may be box lengths further than the nearest;
 //   * the passing pairs of an atom are queued in shared memory and shared out over the atom's
 //     lanes, so that a warp's FP64 instructions run with nearly all lanes at work whatever the
 //     lists' lengths (8 lanes an atom: an LJ liquid's 55 pairs fill 7 rounds of 8);
@@ -32,7 +33,7 @@
 namespace gbmd {
 
 constexpr int Q64_WARP = 1024;  // queue entries of a warp (split evenly over its atoms)
-constexpr unsigned long long R2_ULPS = 8;  // see pair_geometry64
+constexpr unsigned Q64_EXACT = 0x80000000u;
 
 // x^n, n >= 0, by repeated squaring.
 __device__ __forceinline__ double ipow64(double x, int n) {
@@ -130,14 +131,14 @@ __device__ __forceinline__ double eam_body64(const PotParams& P, const Pair64& c
 }
 
 // The candidates of one atom (the calling lane's), tested in FP32 and queued: entry = local index of
-// j.  All lanes of the warp call this together; the lanes of an atom share its queue `q` of cap
-// entries: those with j > i from the front, the others from the back.  drain(nf, nb) consumes the nf
-// front and nb back entries of the atom; it is called whenever some atom's queue could overflow, and
-// at the end.
+// j, plus Q64_EXACT where the FP64 test has to decide.  All lanes of the warp call this together; the
+// lanes of an atom share its queue `q` of cap entries: those with j > i from the front, the others
+// from the back.  drain(nf, nb) consumes the nf front and nb back entries of the atom; it is called
+// whenever some atom's queue could overflow, and at the end.
 template <int NB, class SH, class F>
-__device__ __forceinline__ void scan64(const Dev& D, const SysDev& S, int li, bool active, int lanes, int sub,
-                                       unsigned* q, int cap, const SH& shifts, double rc2, float hi, int spc_sum,
-                                       F&& drain) {
+__device__ __forceinline__ void scan64(const Dev& D, const SysDev& S, int s, int li, bool active, int lanes, int sub,
+                                       unsigned* q, int cap, const SH& shifts, double rc2, float lo,
+                                       float hi, int spc_sum, F&& drain) {
   const unsigned all = 0xffffffffu;
   const int lane = threadIdx.x & 31;
   const int at = lane - sub;  // first lane of the atom
@@ -145,7 +146,7 @@ __device__ __forceinline__ void scan64(const Dev& D, const SysDev& S, int li, bo
   const unsigned below = mine & ((1u << lane) - 1u);
   int nf = 0, nb = 0;
   auto push = [&](bool in, unsigned e) {
-    const bool front = (int)e > li;
+    const bool front = (int)(e & LOCAL_MASK) > li;
     const unsigned mf = __ballot_sync(all, in && front), mb = __ballot_sync(all, in && !front);
     if (in) q[front ? nf + __popc(mf & below) : cap - 1 - (nb + __popc(mb & below))] = e;
     nf += __popc(mf & mine);
@@ -173,7 +174,8 @@ __device__ __forceinline__ void scan64(const Dev& D, const SysDev& S, int li, bo
     // outside), the shift, the box edge and their sums.
     const float Lx = (float)S.L[0], Ly = (float)S.L[1], Lz = (float)S.L[2];
     const float tol = 1e-6f * (fmaxf(fabsf(gi.x), fmaxf(fabsf(gi.y), fabsf(gi.z))) + fmaxf(Lx, fmaxf(Ly, Lz)));
-    const float far2 = hi + tol * fmaf(3.5f, sqrtf(hi), 3.0f * tol);  // (sqrt(hi) + sqrt(3) tol)^2
+    const float band = tol * fmaf(3.5f, sqrtf(hi), 3.0f * tol);  // (sqrt(hi) + sqrt(3) tol)^2 - hi
+    const float near2 = D.outside[s] ? -1.0f : lo - band, far2 = hi + band;
     auto fold = [](float d, float L) { return fminf(fabsf(d), fabsf(fabsf(d) - L)); };
     const int ng = (cnt + 3) >> 2;
     const int ngw = (int)__reduce_max_sync(all, (unsigned)ng);
@@ -195,8 +197,9 @@ __device__ __forceinline__ void scan64(const Dev& D, const SysDev& S, int li, bo
         dx = fold(dx, Lx);
         dy = fold(dy, Ly);
         dz = fold(dz, Lz);
-        in[u] = valid && fmaf(dx, dx, fmaf(dy, dy, dz * dz)) < far2 && (spc_sum < 0 || applies_to(spc_sum, __float_as_int(gi.w), __float_as_int(gj.w)));
-        w[u] = j;
+        const float r2 = fmaf(dx, dx, fmaf(dy, dy, dz * dz));
+        in[u] = valid && r2 < far2 && (spc_sum < 0 || applies_to(spc_sum, __float_as_int(gi.w), __float_as_int(gj.w)));
+        w[u] = j | (r2 >= near2 ? Q64_EXACT : 0u);
       }
 #pragma unroll
       for (int u = 0; u < 4; ++u) push(in[u], w[u]);
@@ -232,7 +235,7 @@ __device__ __forceinline__ void scan64(const Dev& D, const SysDev& S, int li, bo
         for (int k = 0; k < mw; ++k) {
           flush(lanes);
           const int j = b + k;
-          push(k < m && j != li && near(D.g64[S.atom_base + j]) && species_ok(j), (unsigned)j);
+          push(k < m && j != li && near(D.g64[S.atom_base + j]) && species_ok(j), (unsigned)j | Q64_EXACT);
         }
       }
     } else {
@@ -253,7 +256,7 @@ __device__ __forceinline__ void scan64(const Dev& D, const SysDev& S, int li, bo
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
           const int j = j0 + u * lanes + sub;
-          push(in[u] && species_ok(j), (unsigned)j);
+          push(in[u] && species_ok(j), (unsigned)j | Q64_EXACT);
         }
       }
     }
@@ -268,13 +271,12 @@ __device__ __forceinline__ unsigned queued64(const unsigned* q, int cap, int nf,
   return q[k < nf ? k : cap - 1 - (k - nf)];
 }
 
-// r_ij and its square (ref: in the reference's operation order, else with fused multiply-adds), and
-// whether the pair is inside the cutoff, as the reference decides it: r^2 in its operation order,
-// compared on the bit patterns.  The two forms of r^2 are at most 5 units in the last place apart, so
-// the fused one decides all pairs but those within R2_ULPS units of rc2.  (As unsigned numbers the
-// patterns of negative values and of NaNs lie above any rc2.)
+// r_ij and its square in the reference's operation order or, where the pair is known to be inside,
+// with fused multiply-adds.  (One more test of the wrapped components here, in place of the flag
+// D.outside, cost 4 % of the force passes and 9 % of the density pass; the exact test of every pair
+// on the bits of the fused r^2 14 % of the LJ force pass.)
 __device__ __forceinline__ bool pair_geometry64(const double4_32a& pi, const double4_32a& pj, const SysDev& S,
-                                                const long long (&lhb)[3], unsigned long long rc2b, bool ref,
+                                                const long long (&lhb)[3], long long rc2b, bool exact, bool ref,
                                                 double& dx, double& dy, double& dz, double& r2) {
   dx = dsub(pj.x, pi.x);
   dy = dsub(pj.y, pi.y);
@@ -285,11 +287,14 @@ __device__ __forceinline__ bool pair_geometry64(const double4_32a& pi, const dou
     if (wy) dy = dsub(dy, copysign(S.L[1], dy));
     if (wz) dz = dsub(dz, copysign(S.L[2], dz));
   }
+  if (exact) {
+    r2 = ref_sq(dx, dy, dz);
+    // r2 < rc2 on the bit patterns (both are >= 0; a NaN's bits are above any rc2)
+    if (!(__double_as_longlong(r2) >= 0 && __double_as_longlong(r2) < rc2b)) return false;
+    if (ref) return true;
+  }
   r2 = ref ? ref_sq(dx, dy, dz) : fma(dx, dx, fma(dy, dy, dz * dz));
-  const unsigned long long b = (unsigned long long)__double_as_longlong(r2);
-  if (b >= rc2b + R2_ULPS) return false;
-  if (b + R2_ULPS < rc2b) return true;
-  return (unsigned long long)__double_as_longlong(ref_sq(dx, dy, dz)) < rc2b;
+  return true;
 }
 
 template <int NB, int PC, int SCN>
@@ -310,7 +315,7 @@ __global__ void __launch_bounds__(TILE, 5) k_force64(Dev D, PotParams P, Pair64 
   const int cap = Q64_WARP / per;
   unsigned* const q = queue[w] + slot * cap;
   const long long lhb[3] = {__double_as_longlong(S.Lh[0]), __double_as_longlong(S.Lh[1]), __double_as_longlong(S.Lh[2])};
-  const unsigned long long rc2b = (unsigned long long)__double_as_longlong(P.rc2);
+  const long long rc2b = __double_as_longlong(P.rc2);
   const bool tabulated = PC == PC_PAIR && P.kind == POT_FASTLJ;  // its bin needs the reference's r^2
   double ep = 0.0, sxx = 0.0, sxy = 0.0, sxz = 0.0, syy = 0.0, syz = 0.0, szz = 0.0;
   const int w0 = w * B.apw;                                // the warp's first atom within the block
@@ -321,12 +326,12 @@ __global__ void __launch_bounds__(TILE, 5) k_force64(Dev D, PotParams P, Pair64 
     const double4_32a pi = D.g64[S.atom_base + li];
     const double phi_i = PC == PC_EAM ? D.phi[S.atom_base + li] : 0.0;
     double fx = 0.0, fy = 0.0, fz = 0.0;
-    scan64<NB>(D, S, li, active, lanes, sub, q, cap, shifts, P.rc2, P.f[13], P.spc_sum, [&](int nf, int nb) {
+    scan64<NB>(D, S, B.sys, li, active, lanes, sub, q, cap, shifts, P.rc2, P.f[12], P.f[13], P.spc_sum, [&](int nf, int nb) {
       for (int k = sub; k < nf + nb; k += lanes) {
         const unsigned e = queued64(q, cap, nf, k);
-        const long long j = S.atom_base + e;
+        const long long j = S.atom_base + (e & LOCAL_MASK);
         double dx, dy, dz, r2;
-        if (!pair_geometry64(pi, D.g64[j], S, lhb, rc2b, tabulated, dx, dy, dz, r2)) continue;
+        if (!pair_geometry64(pi, D.g64[j], S, lhb, rc2b, (e & Q64_EXACT) != 0u, tabulated, dx, dy, dz, r2)) continue;
         const bool count = k < nf;  // this end of the pair adds its energy and stress
         double gg;
         if (PC == PC_EAM) {
@@ -426,7 +431,7 @@ __global__ void __launch_bounds__(TILE, 8) k_eam_density(Dev D, PotParams P, Pai
   const int cap = Q64_WARP / per;
   unsigned* const q = queue[w] + slot * cap;
   const long long lhb[3] = {__double_as_longlong(S.Lh[0]), __double_as_longlong(S.Lh[1]), __double_as_longlong(S.Lh[2])};
-  const unsigned long long rc2b = (unsigned long long)__double_as_longlong(P.rc2);
+  const long long rc2b = __double_as_longlong(P.rc2);
   const int w0 = w * B.apw;
   const int wn = min(B.apw, max(0, B.count - w0));
   for (int g = 0; g < wn; g += per) {
@@ -434,11 +439,12 @@ __global__ void __launch_bounds__(TILE, 8) k_eam_density(Dev D, PotParams P, Pai
     const int li = B.first - (int)S.atom_base + w0 + (active ? g + slot : 0);
     const double4_32a pi = D.g64[S.atom_base + li];
     double rho = 0.0;
-    scan64<NB>(D, S, li, active, lanes, sub, q, cap, shifts, P.rc2, P.f[13], -1, [&](int nf, int nb) {
+    scan64<NB>(D, S, B.sys, li, active, lanes, sub, q, cap, shifts, P.rc2, P.f[12], P.f[13], -1, [&](int nf, int nb) {
       for (int k = sub; k < nf + nb; k += lanes) {
         const unsigned e = queued64(q, cap, nf, k);
         double dx, dy, dz, r2;
-        if (pair_geometry64(pi, D.g64[S.atom_base + e], S, lhb, rc2b, false, dx, dy, dz, r2))
+        if (pair_geometry64(pi, D.g64[S.atom_base + (e & LOCAL_MASK)], S, lhb, rc2b, (e & Q64_EXACT) != 0u, false, dx, dy,
+                            dz, r2))
           rho += rho_body64<SCM>(P, c, r2);
       }
     });

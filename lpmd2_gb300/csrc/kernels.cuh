@@ -79,6 +79,7 @@ __device__ __forceinline__ int decide_system(const Dev& D, int s, int ucall_inc,
     st.need_rebuild = need;
     st.force_rebuild = 0;
     if (need) {
+      D.outside[s] = 0;
       st.maxdisp2 = 0u;
       st.rebuilds += (S.mode == NB_LIST) ? 1 : 0;
     }
@@ -495,7 +496,11 @@ __device__ __forceinline__ void copyback_atom(const Dev& D, int s, long long p) 
   if (D.has_flags) D.flags[p] = D.sflags[p];
   if (D.ist)
     for (int k = 0; k < IST_K; ++k) D.ist[k * N + p] = D.ist_alt[k * N + p];
-  refresh_gather(D, D.sysd[s], p, true);
+  const SysDev& S = D.sysd[s];
+  // atoms that move are folded into the box before the next re-sort, those with a fixed position stay
+  if (S.mode == NB_LIST && (outside_bits(D.x[p], S.L[0]) || outside_bits(D.y[p], S.L[1]) || outside_bits(D.z[p], S.L[2])))
+    D.outside[s] = 1;
+  refresh_gather(D, S, p, true);
 }
 
 __global__ void __launch_bounds__(REBUILD_CHUNK) k_copyback(Dev D) {

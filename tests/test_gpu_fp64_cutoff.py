@@ -100,6 +100,14 @@ def test_a_fixed_atom_outside_the_box_over_steps():
     assert sim.stats()["neighbor_mode"] == "verlet"
     assert np.array_equal(sim.atoms()[0][[7, 123]], pos[[7, 123]])
     agree(sim, ref, 1e-11)  # five steps pass the forces' rounding on
+    snapshot = sim.checkpoint()
+    sim.do_steps(12)
+    other, _ = pair_of(pos, L, (name, args), "verletlist", list_manager("verletlist", rc, L), vel=vel, flags=flags)
+    other.restore(snapshot)
+    other.do_steps(12)
+    for a, b in zip(sim.atoms(), other.atoms()):
+        np.testing.assert_array_equal(a, b)
+    other.close()
     sim.close()
 
 
