@@ -70,7 +70,7 @@ __device__ __forceinline__ double rho_body64(const PotParams& P, const Pair64& c
   }
   const double ir = rsqrt64(r2);
   if (P.kind == POT_SC) return P.am * (P.int_m >= 0 ? (P.int_m ? ipow64_r(ir, ir * ir, P.int_m) : 1.0) : pow(ir, P.p[3]));
-  const double r = r2 * ir;
+  const double r = sqrt64(r2, ir);
   if (P.kind == POT_GUPTA) return exp(c.c1 * (r - P.p[1]));
   const double d = P.kind == POT_FS ? P.p[6] : P.p[8];
   if (!le_bits(r, d)) return 0.0;
@@ -104,7 +104,7 @@ __device__ __forceinline__ double eam_body64(const PotParams& P, const Pair64& c
     if (count) ep = fma(c.c0, pn, ep);
     return fma(c.c1, pn * inv, phi * pm);
   }
-  const double r = r2 * ir;
+  const double r = sqrt64(r2, ir);
   if (P.kind == POT_GUPTA) {
     const double dr = r - P.p[1];
     const double ex = exp(c.c0 * dr);

@@ -28,22 +28,34 @@ __device__ __forceinline__ bool wraps_bits(double d, long long lhb) {
   return b < 0 ? m > lhb : m >= lhb;
 }
 
-// 1 / x by one step of Halley's iteration, y (1 + e + e^2) with e = 1 - x y, from the hardware's
-// approximation (relative error below 2^-20, so e^3 is below the last bit).
+// Whether v is infinite or NaN, on the bit pattern.
+__device__ __forceinline__ bool not_finite_bits(double v) {
+  return ((unsigned)__double2hiint(v) & 0x7ff00000u) == 0x7ff00000u;
+}
+
+// 1 / x for x >= 0 by one step of Halley's iteration, y (1 + e + e^2) with e = 1 - x y, from the
+// hardware's approximation (relative error below 2^-20, so e^3 is below the last bit).  1 / 0 is
+// infinite, as with a division: the step alone would give a NaN.
 __device__ __forceinline__ double rcp64(double x) {
   double y;
   asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
   const double e = fma(-x, y, 1.0);
-  return fma(y, fma(e, e, e), y);
+  const double r = fma(y, fma(e, e, e), y);
+  return not_finite_bits(y) ? y : r;
 }
 
-// 1 / sqrt(x) by the corresponding third-order step, y (1 + e/2 + 3 e^2/8) with e = 1 - x y^2.
+// 1 / sqrt(x) for x >= 0 by the third-order step of the same family (Householder's iteration; the
+// binomial series of (1 - e)^(-1/2)): y (1 + e/2 + 3 e^2/8) with e = 1 - x y^2.  1 / sqrt(0) is infinite.
 __device__ __forceinline__ double rsqrt64(double x) {
   double y;
   asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
   const double e = fma(-(x * y), y, 1.0);
-  return fma(y * e, fma(0.375, e, 0.5), y);
+  const double r = fma(y * e, fma(0.375, e, 0.5), y);
+  return not_finite_bits(y) ? y : r;
 }
+
+// sqrt(x) from x and rsqrt64(x); 0 for 0.
+__device__ __forceinline__ double sqrt64(double x, double ir) { return not_finite_bits(ir) ? x : x * ir; }
 
 // Lower bound of one axis of the reference's displacement (one wrap) from truncated coordinates: each
 // is off by at most one unit in the last place, so a component is below its truth by at most tol

@@ -11,7 +11,7 @@ import numpy as np
 import pytest
 
 import oracle
-from helpers import FS_FE, SC_CU, rel_norm_err
+from helpers import FS_FE, FSX_MO, GUPTA_AU, SC_CU, rel_norm_err
 from lpmd2_gb300 import inputs as I
 
 pytestmark = pytest.mark.gpu
@@ -151,4 +151,27 @@ def test_coordinates_many_box_lengths_outside():
     sim, ref = pair_of(pos, L, (name, args), "verletlist", list_manager("verletlist", rc, L))
     assert sim.stats()["neighbor_mode"] == "verlet"
     agree(sim, ref)
+    sim.close()
+
+
+@pytest.mark.parametrize("cm", ["minimumimage", "verletlist"])
+@pytest.mark.parametrize("kind", ["gupta", "fs", "fsx", "sc", "sc126", "sc107"])
+def test_coincident_atoms_spoil_only_themselves(kind, cm):
+    """r = 0 is a distance like any other to the densities of Gupta and Finnis-Sinclair metals, and an
+    infinite density (no embedding factor) to Sutton-Chen: only the two atoms' forces are undefined."""
+    name, args, rc, a, Z = {
+        "gupta": ("gupta", GUPTA_AU, 6.0, 4.08, 79), "fs": ("finnissinclair", FS_FE.replace("B 1.8", "B 0.5"), 3.569745, 3.6, 26),
+        "fsx": ("finnissinclair-ext", FSX_MO, 4.1, 3.6, 42),
+        "sc": POTS["sc"], "sc126": ("suttonchen", "e 0.02 a 4.09 n 12 m 6 c 144.4 cutoff 8.18", 8.18, 4.09, 47),
+        "sc107": ("suttonchen", "e 0.012 a 3.61 n 10 m 7 c 39.4 cutoff 7.22", 7.22, 3.61, 29)}[kind]
+    pos, L = crystal(864, a, seed=8)
+    pos[300] = pos[301]
+    cm_args = f"cutoff {rc!r}" if cm == "minimumimage" else list_manager(cm, rc, L)
+    sim, ref = pair_of(pos, L, (name, args), cm, cm_args, Z=Z)
+    got, want = sim.atoms()[2], ref.atoms()[2]
+    rest = np.delete(np.arange(len(pos)), [300, 301])
+    assert np.isnan(got[[300, 301]]).all() and np.isnan(want[[300, 301]]).all()
+    assert np.isfinite(want[rest]).all()
+    assert rel_norm_err(got[rest], want[rest]) <= 1e-12
+    np.testing.assert_allclose(sim.thermo_raw()[1], ref.energy(), rtol=1e-12)  # NaN where the reference's is
     sim.close()
