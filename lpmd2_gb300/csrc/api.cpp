@@ -125,6 +125,7 @@ PotParams finalize_potential(int kind, const double* v, int s1, int s2) {
     P.f[8] = (float)d;
   }
   P.rc2 = P.cutoff * P.cutoff;
+  if (std::isnan(P.rc2)) P.rc2 = 0.0;  // no distance is below a NaN; the kernels compare bit patterns
   P.f[12] = band_lo(P.rc2);
   P.f[13] = band_hi(P.rc2);
   return P;

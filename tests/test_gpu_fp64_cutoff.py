@@ -175,3 +175,12 @@ def test_coincident_atoms_spoil_only_themselves(kind, cm):
     assert rel_norm_err(got[rest], want[rest]) <= 1e-12
     np.testing.assert_allclose(sim.thermo_raw()[1], ref.energy(), rtol=1e-12)  # NaN where the reference's is
     sim.close()
+
+
+@pytest.mark.parametrize("cm,cm_args", [("minimumimage", "cutoff 8.5"), ("linkedcell", "cutoff 8.5 nx 4 ny 4 nz 4"),
+                                        ("verletlist", "cutoff 8.5 maxneighbors 400 each 5")])
+def test_no_pair_is_inside_a_cutoff_that_is_not_a_number(cm, cm_args):
+    pos, L = crystal(500, 5.6, seed=6)
+    sim, ref = pair_of(pos, L, ("lennardjones", f"sigma {SIGMA} epsilon {EPS} cutoff nan"), cm, cm_args)
+    assert not ref.atoms()[2].any() and not sim.atoms()[2].any() and sim.thermo_raw()[1] == 0.0
+    sim.close()
