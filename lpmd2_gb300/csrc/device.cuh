@@ -233,25 +233,30 @@ __device__ __forceinline__ double ref_fitted(double v, double L) {
   return v;
 }
 
-// WrapAround (plugins/linkedcell.cc:9-15), whose result for a negative multiple of n is n itself: a
-// cell past the grid's last, taken as cell 0 here.
-__device__ __forceinline__ int wrap_around(int i, int n) {
+// WrapAround (plugins/linkedcell.cc:9-15), whose result for a negative multiple of n is n itself.
+__device__ __forceinline__ int ref_wrap_around(int i, int n) {
   if (i < 0)
-    i = i % n == 0 ? 0 : i + ((-i / n) + 1) * n;
+    i += ((-i / n) + 1) * n;
   else if (i > n - 1)
     i -= (i / n) * n;
   return i;
 }
 
+// The same inside the grid: cell 0 for a negative multiple of n.
+__device__ __forceinline__ int wrap_around(int i, int n) {
+  i = ref_wrap_around(i, n);
+  return i == n ? 0 : i;
+}
+
 // Cell coordinate of LinkedCell::UpdateCell (plugins/linkedcell.cc:249-253):
-// WrapAround(int(floor(n * (x / L))), n).  ok=false for NaN / absurdly far positions.
+// WrapAround(int(floor(n * (x / L))), n), which may be n.  ok=false for NaN / absurdly far positions.
 __device__ __forceinline__ int ref_cell_coord(double x, double L, int n, bool& ok) {
   double t = floor(dmul((double)n, ddiv(x, L)));
   if (!(t > -1.0e9 && t < 1.0e9)) {
     ok = false;
     return 0;
   }
-  return wrap_around((int)t, n);
+  return ref_wrap_around((int)t, n);
 }
 
 // ---------------------------------------------------------------------------------------------

@@ -208,6 +208,13 @@ __device__ __forceinline__ void bin_atom(const Dev& D, int s, long long i) {
     cx = ref_cell_coord(D.x[i], S.L[0], S.n[0], ok);
     cy = ref_cell_coord(D.y[i], S.L[1], S.n[1], ok);
     cz = ref_cell_coord(D.z[i], S.L[2], S.n[2], ok);
+    // a coordinate n is the first cell of the next row or plane, as in the reference (linkedcell.cc:253);
+    // past the last plane, where the reference keeps the atom in no cell, it is cell 0
+    if ((cz * S.n[1] + cy) * S.n[0] + cx >= S.ncells) {
+      if (cx == S.n[0]) cx = 0;
+      if (cy == S.n[1]) cy = 0;
+      if (cz == S.n[2]) cz = 0;
+    }
   }
   if (!ok) {
     atomicOr(&D.sst[s].error, ERR_OUTSIDE);

@@ -184,3 +184,19 @@ def test_no_pair_is_inside_a_cutoff_that_is_not_a_number(cm, cm_args):
     sim, ref = pair_of(pos, L, ("lennardjones", f"sigma {SIGMA} epsilon {EPS} cutoff nan"), cm, cm_args)
     assert not ref.atoms()[2].any() and not sim.atoms()[2].any() and sim.thermo_raw()[1] == 0.0
     sim.close()
+
+
+def test_cells_of_atoms_one_box_length_below():
+    """The reference's WrapAround takes cell -n to cell n: along x and y that is the first cell of the next
+    row or plane, which the stencil mode, visiting cells as the reference does, keeps to."""
+    name, args, rc, a, _ = POTS["lj"]
+    pos, L = crystal(500, a, seed=12)
+    d = L / 4
+    low = pos < d
+    pos[low[:, 0] & (pos[:, 2] < 3 * d[2])] -= np.array([1.0, 0.0, 0.0]) * L
+    pos[low[:, 1] & (pos[:, 2] < 3 * d[2]) & (pos[:, 0] > 0)] -= np.array([0.0, 1.0, 0.0]) * L
+    assert (pos < 0).any(axis=0).tolist() == [True, True, False]
+    sim, ref = pair_of(pos, L, (name, args), "linkedcell", f"cutoff {rc!r} nx 4 ny 4 nz 4")
+    assert sim.stats()["neighbor_mode"] == "cells"
+    agree(sim, ref)
+    sim.close()
