@@ -719,7 +719,7 @@ struct Engine::Impl {
       if (sm_count < 1) sm_count = 1;
       alloc<unsigned>((size_t)sm_count + 1);
     }
-    D.shift_tab = alloc<float4>((size_t)nsys * 128);
+    alloc<float4>((size_t)nsys * 128);  // nothing reads it any more: part of the layout of saved snapshots
     D.sys_acc = alloc<unsigned long long>((size_t)nsys * SA_LEN);
     D.thermo_last = alloc<double>((size_t)nsys * THERMO_LEN);
     D.log_cap = log_cap;
@@ -785,21 +785,7 @@ struct Engine::Impl {
 
   void upload_sysd() {
     CK(cudaMemcpyAsync(d_sysd, sysd.data(), sizeof(SysDev) * nsys, cudaMemcpyHostToDevice, stream));
-    if (D.shift_tab) {
-      // k * (FP32 cell edge) per axis, k in -2..2, as load_shifts computes it on the device
-      // (a product with 0, +-1 or +-2 is exact, so host and device agree bit for bit)
-      shift_host.assign((size_t)nsys * 128, make_float4(0.f, 0.f, 0.f, 0.f));
-      for (int s = 0; s < nsys; ++s)
-        for (int c = 0; c < 125; ++c) {
-          const int kx = c % 5 - 2, ky = (c / 5) % 5 - 2, kz = c / 25 - 2;
-          shift_host[(size_t)s * 128 + c] = make_float4((float)kx * sysd[s].df[0], (float)ky * sysd[s].df[1],
-                                                        (float)kz * sysd[s].df[2], 0.0f);
-        }
-      CK(cudaMemcpyAsync(D.shift_tab, shift_host.data(), sizeof(float4) * shift_host.size(), cudaMemcpyHostToDevice,
-                         stream));
-    }
   }
-  std::vector<float4> shift_host;  // pageable: the copy has taken the data when it returns
 
   ~Impl() {
     if (device >= 0) cudaSetDevice(device);

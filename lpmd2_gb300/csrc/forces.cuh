@@ -87,20 +87,6 @@ __device__ __forceinline__ void load_shifts(const SysDev& S, ShiftTable<>& sh) {
   __syncthreads();
 }
 
-// The cell-shift table of the mixed force and density passes: the block's own copy in shared
-// memory, or (GBMD_SHIFTS_GLOBAL) the system's copy in global memory, read through L1 and
-// leaving the shared-memory carve-out to L1 (the host writes the same values, D.shift_tab).
-#ifndef GBMD_SHIFTS_GLOBAL
-#define GBMD_SHIFTS_GLOBAL 0
-#endif
-#if GBMD_SHIFTS_GLOBAL
-#define SHIFT_TABLE(name) const float4* __restrict__ name = D.shift_tab + (long long)s * 128
-#else
-#define SHIFT_TABLE(name)   \
-  __shared__ ShiftTable<> name; \
-  load_shifts(S, name)
-#endif
-
 // Epilogue shared by the force kernels: turns the total force on atom i into its acceleration
 // (a = F * forcefactor/m, liblpmd/simulation/pairpotential.cc:62), applies fixedvel, and unless
 // EPI_FORCES advances the velocity: v = v + (0.5*dt) * (a_old + a) (plugins/velocityverlet.cc:73-74).
@@ -411,7 +397,8 @@ __device__ __forceinline__ void force32_tile(const Dev& D, const PotParams& P, c
     if (sp.epi == EPI_KICK_DRIFT && sp.last) hold_range(D, S, B.first, B.count, true);
     return;
   }
-  SHIFT_TABLE(shifts);
+  __shared__ ShiftTable<> shifts;
+  load_shifts(S, shifts);
   const ShiftCorr corr = shift_corr(S);
   const int li = B.first - (int)S.atom_base + (int)threadIdx.x;  // index within the system
   const long long i = S.atom_base + li;
@@ -959,7 +946,8 @@ __device__ __forceinline__ void density32_tile(const Dev& D, const PotParams& P,
   const int s = B.sys;
   const SysDev& S = D.sysd[s];
   if (!S.active) return;  // whole block: its atoms belong to one system
-  SHIFT_TABLE(shifts);
+  __shared__ ShiftTable<> shifts;
+  load_shifts(S, shifts);
   const ShiftCorr corr = shift_corr(S);
   const int li = B.first - (int)S.atom_base + (int)threadIdx.x;
   const long long i = S.atom_base + li;
