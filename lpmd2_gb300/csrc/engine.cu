@@ -510,11 +510,12 @@ struct Engine::Impl {
   }
 
   // Lanes per atom of the mixed passes unless the option says otherwise: as many as leave all blocks
-  // resident at once (8 a SM), 8 only to half of that.  Measured, force pass of an LJ liquid with 1 /
-  // 2 / 4 / 8 lanes (us): 4,000 atoms 23.7 / - / 11.5 / 10.8, 16,384 24.7 / 17.6 / 14.3 / 15.3,
-  // 32,000 26.4 / 19.8 / 17.5 / 26.6, 55,296 30.0 / 24.6 / 30.6 / 39.3, 78,732 37.5 / 40.4 / 41.0 / 55.1;
-  // a second round of blocks costs what the lanes saved.  Forces, energies and virials do not depend
-  // on the lanes, stress by its FP32 rounding.
+  // resident at once (8 a SM), 8 only to half of that.  Measured, passes of a step with 1 / 2 / 4 / 8
+  // lanes (us between events, tail included), LJ liquid: 4,000 atoms 25.9 / 18.0 / 15.7 / 15.3, 16,384
+  // 26.8 / 19.5 / 18.3 / 22.0, 32,000 29.4 / 23.3 / 23.4 / 33.4, 55,296 31.7 / 29.1 / 35.9 / 48.8, 78,732
+  // 38.0 / 39.5 / 43.9 / 62.8; copper: 8,788 74.9 / 44.1 / 35.3 / 34.3, 32,000 80.7 / 57.1 / 55.1 / 72.8,
+  // 55,296 86.9 / 72.5 / 83.4 / 109; a second round of blocks costs what the lanes saved.  No result
+  // depends on the lanes.
   int auto_lanes() const {
     for (int lanes : {8, 4, 2}) {
       long long blocks = 0;
@@ -535,7 +536,7 @@ struct Engine::Impl {
 
   void make_plan32(Plan32& plan, int lanes_per_atom) {
     std::vector<Blk32> blk;
-    const int apb = TILE / lanes_per_atom;
+    const int apb = lanes_atoms(lanes_per_atom);
     for (int s = 0; s < nsys; ++s) {
       for (long long k = 0; k < natoms[s]; k += apb)
         blk.push_back({s, (int)(atom_base[s] + k), (int)std::min<long long>(apb, natoms[s] - k), 0});
@@ -1166,16 +1167,16 @@ struct Engine::Impl {
       else
         k_force32<PC, SPECIES, SCN, SCM, FEED_REGS><<<n, TILE, 0, s>>>(D, P, sp, b);
     } else if (plan.lanes == 4) {
-      k_force32_lanes<PC, SPECIES, SCN, SCM, 4><<<n, TILE, 0, s>>>(D, P, sp, b);
+      k_force32_lanes<PC, SPECIES, SCN, SCM, 4><<<n, lanes_threads(4), 0, s>>>(D, P, sp, b);
     } else if (plan.lanes == 8) {
-      k_force32_lanes<PC, SPECIES, SCN, SCM, 8><<<n, TILE, 0, s>>>(D, P, sp, b);
+      k_force32_lanes<PC, SPECIES, SCN, SCM, 8><<<n, lanes_threads(8), 0, s>>>(D, P, sp, b);
     } else if (plan.lanes == 2) {
-      k_force32_lanes<PC, SPECIES, SCN, SCM, 2><<<n, TILE, 0, s>>>(D, P, sp, b);
+      k_force32_lanes<PC, SPECIES, SCN, SCM, 2><<<n, lanes_threads(2), 0, s>>>(D, P, sp, b);
     } else if constexpr (PC == PC_PAIR) {  // by the option alone
       if (plan.lanes == 16)
-        k_force32_lanes<PC, SPECIES, SCN, SCM, 16><<<n, TILE, 0, s>>>(D, P, sp, b);
+        k_force32_lanes<PC, SPECIES, SCN, SCM, 16><<<n, lanes_threads(16), 0, s>>>(D, P, sp, b);
       else
-        k_force32_lanes<PC, SPECIES, SCN, SCM, 32><<<n, TILE, 0, s>>>(D, P, sp, b);
+        k_force32_lanes<PC, SPECIES, SCN, SCM, 32><<<n, lanes_threads(32), 0, s>>>(D, P, sp, b);
     }
   }
 
@@ -1183,11 +1184,11 @@ struct Engine::Impl {
   void launch_density32_m(cudaStream_t s, const PotParams& P, bool ring) {
     const Plan32& plan = plan_eam;
     if (plan.lanes == 8)
-      k_eam_density32_lanes<SCM, 8><<<plan.n, TILE, 0, s>>>(D, P, plan.blk);
+      k_eam_density32_lanes<SCM, 8><<<plan.n, lanes_threads(8), 0, s>>>(D, P, plan.blk);
     else if (plan.lanes == 4)
-      k_eam_density32_lanes<SCM, 4><<<plan.n, TILE, 0, s>>>(D, P, plan.blk);
+      k_eam_density32_lanes<SCM, 4><<<plan.n, lanes_threads(4), 0, s>>>(D, P, plan.blk);
     else if (plan.lanes == 2)
-      k_eam_density32_lanes<SCM, 2><<<plan.n, TILE, 0, s>>>(D, P, plan.blk);
+      k_eam_density32_lanes<SCM, 2><<<plan.n, lanes_threads(2), 0, s>>>(D, P, plan.blk);
     else if (ring)
       k_eam_density32<SCM, FEED_RING><<<plan.n, TILE, 0, s>>>(D, P, plan.blk);
     else

@@ -714,14 +714,18 @@ __global__ void __launch_bounds__(TILE, GBMD_FORCE_MIN_BLOCKS) k_force32(Dev D, 
 // ------------------------------------------------------------------------------------------
 // Mixed force pass with LANES lanes per atom (TILE / LANES atoms a block), for systems too small to
 // fill the GPU one lane per atom: there a warp's time is its own chain of some ten iterations of
-// gathers and arithmetic (24 us for 4,000 and for 16,384 atoms of LJ liquid alike, 11 and 14 here),
+// gathers and arithmetic (26 us with the tail for 4,000 and for 16,384 atoms of LJ liquid alike, 15 and 18 here),
 // which LANES lanes cut to two or three.  The atom's list groups go round-robin to its lanes (plain
 // cached loads); each group is evaluated and summed exactly as in k_force32, and the lanes'
-// fixed-point partials are combined with integer shuffles, so forces, energy and virial are bitwise
-// those of k_force32; stress is rounded to fixed point per lane.  The per-atom epilogue -- FP64
-// instructions, as long for one atom as for 32 -- runs one thread per atom in as few warps as hold
-// the block's atoms (in every warp, with a few lanes at work, it took longer than the pairs: 15.1 us
-// at 4 lanes and 16,384 atoms, 14.3 so; 20 and 15.3 at 8).
+// fixed-point partials are combined with integer shuffles.  Stress, an FP32 sum over the whole list in
+// k_force32, is handed from lane to lane: after each round of groups every lane in turn adds its four
+// entries and all go on from its sums (0.9 us of the pass at 16,384 LJ atoms, 1.3 at 32,000 of iron; through
+// shared memory 5 and 3).  So every result is bitwise that of k_force32, and what a
+// system gets does not depend on the lanes, which go by what else is in the batch.  The per-atom
+// epilogue -- FP64 instructions, as long for one atom as for 32 -- runs one thread per atom in as few
+// warps as hold the block's atoms (in every warp, with a few lanes at work, it took longer than the
+// pairs: 15.1 us at 4 lanes and 16,384 atoms, 14.3 so; 20 and 15.3 at 8).  A block has whole groups of
+// 32 atoms of its system, whose kinetic terms are summed in FP64 as a warp of k_force32 sums them.
 // ------------------------------------------------------------------------------------------
 
 // g and pair energy of one entry; qi, qj: the embedding factors (metals), folded: times the prefactor.
@@ -745,13 +749,17 @@ __device__ __forceinline__ void lanes_sum(Fix& f) {
   }
 }
 
+// Atoms and threads of a block with `lanes` lanes an atom.
+constexpr int lanes_atoms(int lanes) { return lanes <= TILE / 32 ? TILE / lanes : 32; }
+constexpr int lanes_threads(int lanes) { return lanes * lanes_atoms(lanes); }
+
 template <int PC, int SPECIES, int SCN, int SCM, int LANES>
-__global__ void __launch_bounds__(TILE, 8)
+__global__ void __launch_bounds__(lanes_threads(LANES), 8 * TILE / lanes_threads(LANES))
     k_force32_lanes(Dev D, PotParams P, StepParams sp, const Blk32* blk) {
-  constexpr int APB = TILE / LANES;  // atoms per block
+  constexpr int APB = lanes_atoms(LANES), WARPS = lanes_threads(LANES) / 32;
   __shared__ ShiftTable<> shifts;
   __shared__ long long fsum[3][APB];
-  __shared__ long long esum[TILE / 32][8];
+  __shared__ long long esum[WARPS][8];
   const Blk32 B = blk[blockIdx.x];
   const int s = B.sys;
   const SysDev& S = D.sysd[s];
@@ -769,7 +777,6 @@ __global__ void __launch_bounds__(TILE, 8)
   constexpr bool FOLDED = PHI_IN_W && SCN > 0;
   const float4* __restrict__ gsrc = PHI_IN_W ? D.g32e + S.atom_base : g32;
   const float rc2_lo = P.f[12], rc2_hi = P.f[13];
-  const float ms = (float)(-0.5 * FIX_E);
   unsigned rechecks = 0;
   bool bad = false;
   Fix fqe, fqv;
@@ -777,7 +784,7 @@ __global__ void __launch_bounds__(TILE, 8)
   const int li = B.first - (int)S.atom_base + (active ? slot : 0);
   const long long i = S.atom_base + li;
   Fix fqx, fqy, fqz;
-  float sxx = 0.f, sxy = 0.f, sxz = 0.f, syy = 0.f, syz = 0.f, szz = 0.f;
+  float stress[6] = {};  // xx, xy, xz, yy, yz, zz of the atom, in each of its lanes
   const float4 gi = active ? g32[li] : make_float4(0.f, 0.f, 0.f, 0.f);
   const int ti = __float_as_int(gi.w);
   const float phi_i = (PC == PC_EAM && active) ? (PHI_IN_W ? gsrc[li].w : D.phif[i]) : 0.f;
@@ -788,63 +795,85 @@ __global__ void __launch_bounds__(TILE, 8)
   unsigned band_e = NO_BAND;
   bool band_more = false;
   const uint4* L = active ? list_group(D, S, li, 0) : nullptr;
-  for (int q = sub; q < ng; q += LANES) {
-    const uint4 cur = __ldg(L + (long long)q * na);
-    const unsigned e[4] = {cur.x, cur.y, cur.z, cur.w};
-    const int rem = cnt - 4 * q;
-    float4 gj[4];
-    float pj[4];
+  const int ngw = (int)__reduce_max_sync(0xffffffffu, (unsigned)ng);
+  for (int q0 = 0; q0 < ngw; q0 += LANES) {
+    const int q = q0 + sub;
+    float f[3][4] = {}, d[3][4] = {};
+    if (q < ng) {
+      const uint4 cur = __ldg(L + (long long)q * na);
+      const unsigned e[4] = {cur.x, cur.y, cur.z, cur.w};
+      const int rem = cnt - 4 * q;
+      float4 gj[4];
+      float pj[4];
 #pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      gj[u] = gsrc[e[u] & LOCAL_MASK];
-      pj[u] = (PC == PC_EAM && !PHI_IN_W) ? D.phif[S.atom_base + (e[u] & LOCAL_MASK)] : gj[u].w;
-    }
-    float ge = 0.f, gv = 0.f, gx = 0.f, gy = 0.f, gz = 0.f;
-#pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      const bool valid = u == 0 || rem > u;
-      float dx, dy, dz;
-      const float r2 = entry_r2(gi, gj[u], shifts[e[u] >> CODE_SHIFT], corr, dx, dy, dz);
-      bool in = valid && r2 < rc2_lo;
-      if (valid && r2 >= rc2_lo && r2 < rc2_hi) {  // guard band: decided in FP64 after the loop
-        if (band_e == NO_BAND)
-          band_e = e[u];
-        else
-          band_more = true;
+      for (int u = 0; u < 4; ++u) {
+        gj[u] = gsrc[e[u] & LOCAL_MASK];
+        pj[u] = (PC == PC_EAM && !PHI_IN_W) ? D.phif[S.atom_base + (e[u] & LOCAL_MASK)] : gj[u].w;
       }
-      if (SPECIES) in = in && applies_to(P.spc_sum, ti, __float_as_int(gj[u].w));
-      float g, en;
-      pair32<PC, FOLDED, SCN, SCM>(P, r2, phi_i, pj[u], g, en);
-      g = in ? g : 0.0f;
-      ge += in ? en : 0.0f;
-      gv = fmaf(g, r2, gv);
-      const float fx = g * dx, fy = g * dy, fz = g * dz;
-      sxx = fmaf(fx, dx, sxx);
-      sxy = fmaf(fx, dy, sxy);
-      sxz = fmaf(fx, dz, sxz);
-      syy = fmaf(fy, dy, syy);
-      syz = fmaf(fy, dz, syz);
-      szz = fmaf(fz, dz, szz);
-      // the group's force in k_force32's order: ((g0 d0 + g1 d1) + g2 d2) + g3 d3, fused
-      gx = u == 0 ? g * dx : fmaf(g, dx, gx);
-      gy = u == 0 ? g * dy : fmaf(g, dy, gy);
-      gz = u == 0 ? g * dz : fmaf(g, dz, gz);
+      float ge = 0.f, gv = 0.f, gx = 0.f, gy = 0.f, gz = 0.f;
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const bool valid = u == 0 || rem > u;
+        float dx, dy, dz;
+        const float r2 = entry_r2(gi, gj[u], shifts[e[u] >> CODE_SHIFT], corr, dx, dy, dz);
+        bool in = valid && r2 < rc2_lo;
+        if (valid && r2 >= rc2_lo && r2 < rc2_hi) {  // guard band: decided in FP64 after the loop
+          if (band_e == NO_BAND)
+            band_e = e[u];
+          else
+            band_more = true;
+        }
+        if (SPECIES) in = in && applies_to(P.spc_sum, ti, __float_as_int(gj[u].w));
+        float g, en;
+        pair32<PC, FOLDED, SCN, SCM>(P, r2, phi_i, pj[u], g, en);
+        g = in ? g : 0.0f;
+        ge += in ? en : 0.0f;
+        gv = fmaf(g, r2, gv);
+        d[0][u] = dx;
+        d[1][u] = dy;
+        d[2][u] = dz;
+        f[0][u] = g * dx;
+        f[1][u] = g * dy;
+        f[2][u] = g * dz;
+        // the group's force in k_force32's order: ((g0 d0 + g1 d1) + g2 d2) + g3 d3, fused
+        gx = u == 0 ? g * dx : fmaf(g, dx, gx);
+        gy = u == 0 ? g * dy : fmaf(g, dy, gy);
+        gz = u == 0 ? g * dz : fmaf(g, dz, gz);
+      }
+      fqx.add_scaled32(gx);
+      fqy.add_scaled32(gy);
+      fqz.add_scaled32(gz);
+      fqe.add_scaled26(0.5f * ge);
+      fqv.add_scaled26(-0.5f * gv);
+      bad |= fmaxf(fabsf(gx), fmaxf(fabsf(gy), fabsf(gz))) > 4000.0f;
     }
-    fqx.add_scaled32(gx);
-    fqy.add_scaled32(gy);
-    fqz.add_scaled32(gz);
-    fqe.add_scaled26(0.5f * ge);
-    fqv.add_scaled26(-0.5f * gv);
-    bad |= fmaxf(fabsf(gx), fmaxf(fabsf(gy), fabsf(gz))) > 4000.0f;
+    // the round's groups in list order: each lane in turn adds its own, and all go on from its sums (a
+    // lane without a group adds zeros, which change none)
+#pragma unroll
+    for (int l = 0; l < LANES; ++l) {
+#pragma unroll
+      for (int k = 0; k < 6; ++k) {
+        const int a = k < 3 ? 0 : k < 5 ? 1 : 2, b = k < 3 ? k : k < 5 ? k - 2 : 2;
+        float t = stress[k];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) t = fmaf(f[a][u], d[b][u], t);
+        stress[k] = __shfl_sync(0xffffffffu, t, l, LANES);
+      }
+    }
   }
-  if (band_e != NO_BAND) {
+  // guard-band entries, as in k_force32 in list order: all lanes of the atom settle each of them, and
+  // the first one adds it to the fixed-point sums
+  const unsigned mine = (LANES == 32 ? 0xffffffffu : (1u << (LANES & 31)) - 1u) << (lane - sub);
+  const unsigned noted = __ballot_sync(0xffffffffu, band_e != NO_BAND) & mine;
+  const unsigned more = __ballot_sync(0xffffffffu, band_more) & mine;
+  if (noted) {
     auto settle = [&](unsigned e) {
       const int j = (int)(e & LOCAL_MASK);
       const float4 gj = g32[j];
       float dx, dy, dz;
       const float r2 = entry_r2(gi, gj, shifts[e >> CODE_SHIFT], corr, dx, dy, dz);
       if (!(r2 >= rc2_lo && r2 < rc2_hi)) return;
-      ++rechecks;
+      if (sub == 0) ++rechecks;
       if (!exact_inside_cold(&D, &S, i, S.atom_base + j, P.rc2)) return;
       if (SPECIES && !applies_to(P.spc_sum, ti, __float_as_int(gj.w))) return;
       float g, en;
@@ -853,23 +882,25 @@ __global__ void __launch_bounds__(TILE, 8)
       else  // the unscaled embedding factors of both atoms (rare path)
         eam_pair32_t<SCN, SCM>(P, r2, D.phif[i], D.phif[S.atom_base + j], g, en);
       const float fx = g * dx, fy = g * dy, fz = g * dz;
-      fqx.add_scaled32(fx);
-      fqy.add_scaled32(fy);
-      fqz.add_scaled32(fz);
-      fqe.add_scaled26(0.5f * en);
-      fqv.add_scaled26(-0.5f * (g * r2));
-      bad |= fmaxf(fabsf(fx), fmaxf(fabsf(fy), fabsf(fz))) > 4000.0f;
-      sxx = fmaf(fx, dx, sxx);
-      sxy = fmaf(fx, dy, sxy);
-      sxz = fmaf(fx, dz, sxz);
-      syy = fmaf(fy, dy, syy);
-      syz = fmaf(fy, dz, syz);
-      szz = fmaf(fz, dz, szz);
+      if (sub == 0) {
+        fqx.add_scaled32(fx);
+        fqy.add_scaled32(fy);
+        fqz.add_scaled32(fz);
+        fqe.add_scaled26(0.5f * en);
+        fqv.add_scaled26(-0.5f * (g * r2));
+        bad |= fmaxf(fabsf(fx), fmaxf(fabsf(fy), fabsf(fz))) > 4000.0f;
+      }
+      stress[0] = fmaf(fx, dx, stress[0]);
+      stress[1] = fmaf(fx, dy, stress[1]);
+      stress[2] = fmaf(fx, dz, stress[2]);
+      stress[3] = fmaf(fy, dy, stress[3]);
+      stress[4] = fmaf(fy, dz, stress[4]);
+      stress[5] = fmaf(fz, dz, stress[5]);
     };
-    if (!band_more) {
-      settle(band_e);
+    if (!more && (noted & (noted - 1)) == 0) {
+      settle(__shfl_sync(mine, band_e, __ffs(noted) - 1));
     } else {
-      for (int q = sub; q < ng; q += LANES) {
+      for (int q = 0; q < ng; ++q) {
         const uint4 e4 = __ldg(L + (long long)q * na);
         const int rem = cnt - 4 * q;
         settle(e4.x);
@@ -890,19 +921,20 @@ __global__ void __launch_bounds__(TILE, 8)
   if (rechecks) atomicAdd(&D.sst[s].rechecks, (unsigned long long)rechecks);
   if (bad) atomicOr(&D.sst[s].error, ERR_FIXED);
   // energy and virial: every lane's own fixed-point partial (exact integer sums, whatever the lane
-  // count)
-  long long v[8] = {fqe.value() * 64, fqv.value() * 64, fix64(sxx * ms), fix64(sxy * ms), fix64(sxz * ms),
-                    fix64(syy * ms),  fix64(syz * ms),  fix64(szz * ms)};
+  // count); stress: the atom's sums (halved: full list), rounded once, from its first lane
+  const float ms = sub == 0 ? (float)(-0.5 * FIX_E) : 0.0f;
+  long long v[8] = {fqe.value() * 64,      fqv.value() * 64,      fix64(stress[0] * ms), fix64(stress[1] * ms),
+                    fix64(stress[2] * ms), fix64(stress[3] * ms), fix64(stress[4] * ms), fix64(stress[5] * ms)};
   const long long t8 = warp_sums(v);
   if ((lane & 3) == 0) esum[w][lane >> 2] = t8;
   __syncthreads();
   unsigned long long* acc = D.sys_acc + (long long)s * SA_LEN;
-  if (threadIdx.x >= TILE - 32 && lane < 11) {
+  if (w == WARPS - 1 && lane < 11) {
     // energy, virial and the nine stress slots from the eight sums (in the last warp: the first ones
     // go on with the atoms)
     const int f = sum_of_slot(lane);
     long long t = 0;
-    for (int k = 0; k < TILE / 32; ++k) t += esum[k][f];
+    for (int k = 0; k < WARPS; ++k) t += esum[k][f];
     atomicAdd(acc + lane, (unsigned long long)t);
   }
   const int t = threadIdx.x;
@@ -1045,9 +1077,9 @@ __global__ void GBMD_DENSITY_BOUNDS k_eam_density32(Dev D, PotParams P, const Bl
 
 // The same with LANES lanes per atom (see k_force32_lanes): densities bitwise those of one lane.
 template <int SCM, int LANES>
-__global__ void __launch_bounds__(TILE, 8)
+__global__ void __launch_bounds__(lanes_threads(LANES), 8 * TILE / lanes_threads(LANES))
     k_eam_density32_lanes(Dev D, PotParams P, const Blk32* blk) {
-  constexpr int APB = TILE / LANES;
+  constexpr int APB = lanes_atoms(LANES);
   __shared__ ShiftTable<> shifts;
   __shared__ long long rsum[APB];
   const Blk32 B = blk[blockIdx.x];
