@@ -1017,7 +1017,13 @@ struct Engine::Impl {
     for (auto n : natoms) m = std::max<long long>(m, n);
     return m;
   }
-  bool cluster_sort() const { return most_atoms() <= (nsys == 1 ? CLUSTER_ATOMS : CLUSTER_ATOMS_BATCH); }
+  bool cluster_sort() const {
+    const long long atoms = most_atoms();
+    int cells = 0;
+    for (const auto& S : sysd) cells = std::max(cells, S.ncells);
+    return atoms <= (nsys == 1 ? CLUSTER_ATOMS : CLUSTER_ATOMS_BATCH) &&
+           cells <= (cluster_blocks(atoms) == 1 ? CLUSTER_CELLS_ONE : CLUSTER_CELLS);
+  }
   void launch_rebuild_kernels(cudaStream_t s) {
     mark_begin(s, T_REBUILD);
     // a batch's chain runs over the systems listed by its first kernel, in grids that the list may
@@ -1028,6 +1034,8 @@ struct Engine::Impl {
       nb = std::min(nb, REBUILD_GRID);
       nc = std::min(nc, REBUILD_GRID);
     }
+    // the blocks of a sparse grid cost even where nothing rebuilds (1.2 M cells: 320 us a force call)
+    nc = std::min(nc, 32 * REBUILD_GRID);
     if (nsys > 1) {
       k_rebuild_list<<<1, RLIST_THREADS, 0, s>>>(D);
       launched();

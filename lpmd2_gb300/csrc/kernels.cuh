@@ -522,10 +522,15 @@ __global__ void __launch_bounds__(REBUILD_CHUNK) k_copyback(Dev D) {
 // does without its conditional node.  Measured against the chain of kernels (conditional node
 // included), us a step: single LJ liquids of 500 / 4,000 / 8,788 / 16,384 / 32,000 atoms 21.2 / 24.8 /
 // 25.8 / 30.0 / 38.5 against 27.8 / 28.0 / 29.9 / 32.9 / 37.3; batches of 512 x 256 atoms 101 against
-// 110, of 33 systems up to 4,000 87 against 77.
+// 110, of 33 systems up to 4,000 87 against 77.  Cells cost as well: gases of 500 atoms on 8,000 cells
+// 20.8 against 26.3, 2,000 on 32,768 32.9 / 32.3, 8,000 on 2,197 / 15,625 cells 31.0 / 34.2 against
+// 31.0 / 32.8, 20,000 on 2,197 / 39,304 36.9 / 54.0 against 35.2 / 46.8 (with one cell a
+// warp at a time and no line by cells 37.0, 115, 42.0 and 66.2, and 3,820 for 1,000 on 1.2 M: 240 so).
 // ---------------------------------------------------------------------------------------------
 constexpr int CLUSTER_ATOMS = 24000;       // a single system
 constexpr int CLUSTER_ATOMS_BATCH = 2048;  // the largest system of a batch
+constexpr int CLUSTER_CELLS = 4096;        // of a system on several blocks
+constexpr int CLUSTER_CELLS_ONE = 32768;   // of a system on one
 constexpr int CLUSTER_THREADS = 1024;
 constexpr int CLUSTER_SORT_BYTES = CLUSTER_THREADS / 32 * 2 * SORT_STAGE * (int)sizeof(int);
 
@@ -554,9 +559,20 @@ __global__ void __launch_bounds__(CLUSTER_THREADS, 1) k_sort_cluster(Dev D, int 
   cluster_barrier();
   const int w = threadIdx.x >> 5;
   int* const mine = stage + w * 2 * SORT_STAGE;
-  for (int c = rank * (CLUSTER_THREADS / 32) + w; c < S.ncells; c += blocks * (CLUSTER_THREADS / 32)) {
-    sort_cell(D, S.cell_base + c, mine, mine + SORT_STAGE);
-    __syncwarp();
+  if (S.ncells <= step) {
+    for (int c = rank * (CLUSTER_THREADS / 32) + w; c < S.ncells; c += blocks * (CLUSTER_THREADS / 32)) {
+      sort_cell(D, S.cell_base + c, mine, mine + SORT_STAGE);
+      __syncwarp();
+    }
+  } else {  // 32 cells at a time, of which most have one atom or none
+    const int lane = threadIdx.x & 31;
+    for (int c0 = (w * blocks + rank) * 32; c0 < S.ncells; c0 += step) {
+      const int c = c0 + lane;
+      for (unsigned todo = __ballot_sync(0xffffffffu, c < S.ncells && D.ccnt[S.cell_base + c] > 1); todo; todo &= todo - 1) {
+        sort_cell(D, S.cell_base + c0 + __ffs(todo) - 1, mine, mine + SORT_STAGE);
+        __syncwarp();
+      }
+    }
   }
   cluster_barrier();
   for (int k = t0; k < n; k += step) permute_atom(D, S.atom_base + k);
