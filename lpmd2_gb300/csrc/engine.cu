@@ -526,15 +526,20 @@ struct Engine::Impl {
   }
   int sm_count = 1;
 
-  // Blocks of the mixed passes.
+  // Blocks of the mixed passes, a table for each lane count in use: they go by the systems' sizes, so
+  // they stay for the engine's life and a change of lanes allocates nothing the second time.
   struct Plan32 {
     int lanes = 0, n = 0;
     Blk32* blk = nullptr;
   };
-  Plan32 plan_pair, plan_eam;  // the option lanes_per_atom sets the pair passes' lanes
-  int planned_lanes = -1;
+  Plan32 plans[6];  // 1, 2, 4, 8, 16, 32 lanes
+  Plan32 plan_pair, plan_eam;  // those in use; the option lanes_per_atom sets the pair passes' lanes
 
-  void make_plan32(Plan32& plan, int lanes_per_atom) {
+  const Plan32& plan32(int lanes_per_atom) {
+    int q = 0;
+    while ((1 << q) < lanes_per_atom) ++q;
+    Plan32& plan = plans[q];
+    if (plan.blk) return plan;
     std::vector<Blk32> blk;
     const int apb = lanes_atoms(lanes_per_atom);
     for (int s = 0; s < nsys; ++s) {
@@ -543,19 +548,16 @@ struct Engine::Impl {
     }
     plan.lanes = lanes_per_atom;
     plan.n = (int)blk.size();
-    if (plan.blk) dev_free(plan.blk);
-    plan.blk = nullptr;
     CK(dev_malloc(&plan.blk, sizeof(Blk32) * std::max<size_t>(blk.size(), 1)));
     CK(cudaMemcpyAsync(plan.blk, blk.data(), sizeof(Blk32) * blk.size(), cudaMemcpyHostToDevice, stream));
-    CK(cudaStreamSynchronize(stream));
+    return plan;  // (a copy from pageable memory has read it when it returns)
   }
   void ensure_plan32() {
-    if (planned_lanes == lanes) return;
-    CK(cudaStreamSynchronize(stream));
+    const int wide = auto_lanes(), pair = lanes ? lanes : wide;
+    if (plan_pair.lanes == pair && plan_eam.lanes == wide) return;
     drop_graph();
-    make_plan32(plan_pair, lanes ? lanes : auto_lanes());
-    make_plan32(plan_eam, auto_lanes());
-    planned_lanes = lanes;
+    plan_pair = plan32(pair);
+    plan_eam = plan32(wide);
   }
 
   // Block table and partial sums of the FP64 passes.
@@ -578,21 +580,30 @@ struct Engine::Impl {
       }
       per[s].y = (int)blk.size() - per[s].x;
     }
-    nblk64 = (int)blk.size();
-    Blk64* db = alloc_scratch<Blk64>(blk.size());
-    int2* dp = alloc_scratch<int2>(per.size());
-    CK(cudaMemcpyAsync(db, blk.data(), sizeof(Blk64) * blk.size(), cudaMemcpyHostToDevice, stream));
-    CK(cudaMemcpyAsync(dp, per.data(), sizeof(int2) * per.size(), cudaMemcpyHostToDevice, stream));
-    CK(cudaStreamSynchronize(stream));
-    D.blk64 = db;
-    D.sys64 = dp;
-    // one partial record per tile is part of the set-up pool; finer cuts have their own
-    D.part64 = nblk64 == ntiles ? tile_part : alloc_scratch<double>((size_t)nblk64 * PART_D);
     shares64 = 1;
     for (const int2& x : per) shares64 = std::max(shares64, thermo_shares(x.y));
-    D.share64 = alloc_scratch<double>((size_t)nsys * shares64 * PART_D);
-    D.ticket64 = alloc_scratch<unsigned>(nsys);  // zeroed
+    const bool same = D.blk64 && blk.size() == plan64_blk.size() &&
+                      std::memcmp(blk.data(), plan64_blk.data(), sizeof(Blk64) * blk.size()) == 0;
+    if (same) return;
+    plan64_blk = blk;
+    nblk64 = (int)blk.size();
+    free_scratch();
+    // one allocation: partial sums (one record per tile is part of the set-up pool; finer cuts have their
+    // own), shares, the block table, the systems' runs of blocks, tickets (zeroed)
+    const bool own = nblk64 != ntiles;
+    const size_t np = own ? (size_t)nblk64 * PART_D : 0, ns = (size_t)nsys * shares64 * PART_D;
+    double* d = alloc_scratch<double>(np + ns + (sizeof(int2) * nsys + sizeof(Blk64) * blk.size() + sizeof(unsigned) * nsys + 7) / 8);
+    D.part64 = own ? d : tile_part;
+    D.share64 = d + np;
+    int2* dp = (int2*)(d + np + ns);
+    Blk64* db = (Blk64*)(dp + nsys);
+    D.sys64 = dp;
+    D.blk64 = db;
+    D.ticket64 = (unsigned*)(db + blk.size());
+    CK(cudaMemcpyAsync(dp, per.data(), sizeof(int2) * per.size(), cudaMemcpyHostToDevice, stream));
+    CK(cudaMemcpyAsync(db, blk.data(), sizeof(Blk64) * blk.size(), cudaMemcpyHostToDevice, stream));
   }
+  std::vector<Blk64> plan64_blk;  // as last laid out
   int nblk64 = 0, shares64 = 1;
   double* tile_part = nullptr;
 
@@ -726,10 +737,6 @@ struct Engine::Impl {
     D.log_cap = log_cap;
     D.nsys = nsys;
     D.thermo_log = alloc<double>((size_t)nsys * log_cap * THERMO_LEN);
-    {
-      std::lock_guard<std::recursive_mutex> lk(g_dev_mu);
-      CK(cudaMallocHost(&h_sst, sizeof(SysState) * nsys));
-    }
     d_sysd = alloc<SysDev>(nsys);
     d_sst = alloc<SysState>(nsys);
     d_tile_sys = alloc<int>(ntiles);
@@ -804,8 +811,7 @@ struct Engine::Impl {
     }
     free_scratch();
     for (auto& a : work) dev_free(a.first);
-    if (plan_pair.blk) dev_free(plan_pair.blk);
-    if (plan_eam.blk) dev_free(plan_eam.blk);
+    for (Plan32& p : plans) dev_free(p.blk);
     free_cells();
     if (stream) cudaStreamDestroy(stream);
     if (stream2) cudaStreamDestroy(stream2);
@@ -939,9 +945,7 @@ struct Engine::Impl {
         throw Error(1, "every system of a batch must use the same neighbour mode (box too small for a Verlet list?)");
     // cell arrays and neighbour list
     free_cells();
-    free_scratch();
     if (precision == PREC_FP64) alloc_blocks64();
-    planned_lanes = -1;
     alloc_cells(total_cells);
     int maxnb = 0;
     if (any_list) {
@@ -1274,13 +1278,26 @@ struct Engine::Impl {
   }
 
   // The per-system states, read behind everything queued on the stream into page-locked memory (one
-  // wait; a copy to pageable memory after a wait of its own cost 10 us more a call).
+  // wait; a copy to pageable memory after a wait of its own cost 10 us more a call).  Page-locking costs
+  // 250 us, so an engine of a few calls does without.
+  static constexpr int PAGEABLE_READS = 16;
   const SysState* read_states() {
-    CK(cudaMemcpyAsync(h_sst, d_sst, sizeof(SysState) * nsys, cudaMemcpyDeviceToHost, stream));
+    if (!h_sst && ++state_reads > PAGEABLE_READS) {
+      std::lock_guard<std::recursive_mutex> lk(g_dev_mu);
+      CK(cudaMallocHost(&h_sst, sizeof(SysState) * nsys));
+    }
+    SysState* to = h_sst;
+    if (!to) {
+      h_states.resize(nsys);
+      to = h_states.data();
+    }
+    CK(cudaMemcpyAsync(to, d_sst, sizeof(SysState) * nsys, cudaMemcpyDeviceToHost, stream));
     CK(cudaStreamSynchronize(stream));
-    return h_sst;
+    return to;
   }
   SysState* h_sst = nullptr;
+  std::vector<SysState> h_states;
+  int state_reads = 0;
 
   // Reads the per-system error words and the list statistics (synchronises the stream).
   void check_errors() {
