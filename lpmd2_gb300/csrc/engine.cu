@@ -509,17 +509,18 @@ struct Engine::Impl {
     }
   }
 
-  // Lanes per atom of the mixed passes unless the option says otherwise: as many as leave all blocks
-  // resident at once (8 a SM), 8 only to half of that.  Measured, passes of a step with 1 / 2 / 4 / 8
-  // lanes (us between events, tail included), LJ liquid: 4,000 atoms 25.9 / 18.0 / 15.7 / 15.3, 16,384
-  // 26.8 / 19.5 / 18.3 / 22.0, 32,000 29.4 / 23.3 / 23.4 / 33.4, 55,296 31.7 / 29.1 / 35.9 / 48.8, 78,732
-  // 38.0 / 39.5 / 43.9 / 62.8; copper: 8,788 74.9 / 44.1 / 35.3 / 34.3, 32,000 80.7 / 57.1 / 55.1 / 72.8,
-  // 55,296 86.9 / 72.5 / 83.4 / 109; a second round of blocks costs what the lanes saved.  No result
-  // depends on the lanes.
+  // Lanes per atom of the mixed passes unless the option says otherwise: as many as leave all blocks of
+  // the active systems resident at once (8 a SM), 8 only to half of that.  Measured, passes of a step
+  // with 1 / 2 / 4 / 8 lanes (us between events, tail included), LJ liquid: 4,000 atoms 25.9 / 18.0 / 15.7
+  // / 15.3, 16,384 26.8 / 19.5 / 18.3 / 22.0, 32,000 29.4 / 23.3 / 23.4 / 33.4, 55,296 31.7 / 29.1 / 35.9 /
+  // 48.8, 78,732 38.0 / 39.5 / 43.9 / 62.8; copper: 8,788 74.9 / 44.1 / 35.3 / 34.3, 32,000 80.7 / 57.1 /
+  // 55.1 / 72.8, 55,296 86.9 / 72.5 / 83.4 / 109; a second round of blocks costs what the lanes saved.
+  // No result depends on the lanes.
   int auto_lanes() const {
     for (int lanes : {8, 4, 2}) {
       long long blocks = 0;
-      for (int s = 0; s < nsys; ++s) blocks += (natoms[s] * lanes + TILE - 1) / TILE;
+      for (int s = 0; s < nsys; ++s)
+        if (sysd[s].active) blocks += (natoms[s] * lanes + TILE - 1) / TILE;
       if (blocks <= (lanes == 8 ? 4 : 8) * (long long)sm_count) return lanes;
     }
     return 1;

@@ -97,3 +97,26 @@ def test_record_with_species_filters(n):
         out.append((*sim.atoms(), sim.thermo()["raw"]))
         sim.close()
     same(*out)
+
+
+def test_lanes_follow_the_active_systems():
+    """A large system that retires leaves the small one with the lanes it gets alone, and the same record."""
+    small, filler = crystal(4001, POTS["lj"][3], seed=2), crystal(80001, POTS["lj"][3], seed=5)
+    _, args, rc, _, Z = POTS["lj"]
+    out = []
+    for systems in ([small], [small, filler]):
+        b = gbmd.Batch([len(s[0]) for s in systems], [s[3] for s in systems])
+        for k, (pos, vel, m, _) in enumerate(systems):
+            b.set_atoms(k, pos, vel, Z=Z, mass=m)
+        b.set_cell_manager(gbmd.Plugin("verletlist", f"cutoff {rc!r} skin 0.4 maxneighbors 400"))
+        b.add_potential(gbmd.Plugin("lennardjones", args))
+        b.set_integrator(gbmd.Plugin("velocityverlet", "dt 2.0"))
+        b.set_precision("mixed")
+        b.update_forces()
+        b.do_steps(3)
+        if len(systems) > 1:
+            b.set_active(1, False)
+        b.do_steps(20)
+        out.append((*b.atoms(0), b.thermo(0)["raw"]))
+        b.close()
+    same(*out)
