@@ -1413,11 +1413,17 @@ struct Engine::Impl {
     drop_graph(built);
     cudaGraph_t& graph = built.graph;
     CK(cudaGraphCreate(&graph, 0));
-    // a conditional node costs 8.5 us a step whether its body runs or not: as much as the whole chain's
-    // empty launches.  So it only pays for a single system too large for the one-launch sort; of a
-    // batch some system rebuilds in nearly every step
+    // a conditional node costs 8.5 us a step whether its body runs or not, the whole chain's empty launches
+    // as much for a single system and some 12 us for a batch.  So it pays where the chain has many
+    // launches and few steps rebuild: for a system too large for the one-launch sort, and for batches of
+    // up to 8 active systems (of more, some system rebuilds in nearly every step).  Measured, us a step
+    // without / with the node: 2 systems of 16,384 LJ atoms 42.7 / 40.0, 2 of 108,000 of copper at 50 K
+    // 262 / 254, a small one beside a retired large one 42.3 / 34.4; 8 of 32,000 of copper at 50 / 600 K
+    // 292 / 284 and 307 / 308; 16 of 10,976 at 600 K 262 / 272, 128 LJ liquids 415 / 431.
     const bool plain = integ.kind != INT_VV;  // step_plain keeps its chain in line
-    bool cond = graph_mode == 2 && !plain && !cluster_sort() && nsys == 1 && sysd[0].mode != NB_ALLPAIRS;
+    int active = 0;
+    for (const auto& S : sysd) active += S.active ? 1 : 0;
+    bool cond = graph_mode == 2 && !plain && !cluster_sort() && active <= 8 && sysd[0].mode != NB_ALLPAIRS;
     std::vector<cudaGraphConditionalHandle> handles(nsteps);
     if (cond) {
       for (int k = 0; k < nsteps; ++k) {
