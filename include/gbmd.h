@@ -182,8 +182,8 @@ gbmd_status gbmd_sim_set_precision(gbmd_sim* sim, int precision);
  *                      stream, so read gbmd_*_stream afterwards
  *   "lanes_per_atom"   mixed Lennard-Jones force pass: 1, 2, 4, 8, 16 or 32 lanes share an
  *                      atom's neighbour list, i.e. 32 to 1 atoms per warp (the same results bit
- *                      for bit).  Unset, as many as keep every block resident: 8 to 2 for small
- *                      systems, else 1
+ *                      for bit).  0 (default): as many as keep every block of the active systems
+ *                      resident, 8 to 2 for few atoms, else 1
  *   "list_feed"        how the mixed passes read their Verlet-list rows: 0 auto (default:
  *                      registers for the density pass of a single EAM system and, but for the
  *                      common Sutton-Chen metals, its force pass; a shared-memory ring of bulk

@@ -1915,10 +1915,10 @@ void Engine::set_option(const std::string& key, const std::string& value) {
     I.drop_graph();
     return;
   }
-  if (key == "lanes_per_atom") {  // mixed LJ force pass: 1 (one lane per atom), 2, 4, 8, 16 or 32 lanes per atom
+  if (key == "lanes_per_atom") {  // mixed LJ force pass: 1, 2, 4, 8, 16 or 32 lanes per atom, 0: by size again
     const int l = (int)v;
-    if (l != 1 && l != 2 && l != 4 && l != 8 && l != 16 && l != 32)
-      throw Error(1, "lanes_per_atom must be 1, 2, 4, 8, 16 or 32");
+    if (l != 0 && l != 1 && l != 2 && l != 4 && l != 8 && l != 16 && l != 32)
+      throw Error(1, "lanes_per_atom must be 0 (by size), 1, 2, 4, 8, 16 or 32");
     I.lanes = l;
     I.drop_graph();
     return;

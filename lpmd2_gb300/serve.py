@@ -270,12 +270,9 @@ def summarize(results: list[JobResult], wall_s: float) -> dict:
 
 # ---------------------------------------------------------------------- libgbmd backend
 def lanes_for(live_atoms: int) -> int:
-    """Lanes per atom of the LJ force pass for a batch with this many live atoms: below about
-    60k atoms one lane per atom leaves the GPU partly idle.  Thresholds from GB300 timings of
-    single LJ liquids at rc 2.5 sigma (ms/step with 1/2/4/8/16 lanes: 864 atoms 0.046/0.040/
-    0.036/0.035/0.034; 4,000: 0.051/0.043/0.040/0.039/0.043; 16,384: 0.047/0.039/0.041/0.047/
-    0.062; 55,296: 0.055/0.055/0.065/0.089/0.141; 256,000: 0.140/0.163/0.203/0.319/0.566).
-    Forces are the same for every choice, so changing it never changes a job's trajectory."""
+    """A fixed choice of lanes per atom for a backend that cannot choose for itself, by the batch's live
+    atoms.  The engine can (option lanes_per_atom 0, its default, goes by the active systems, with lines
+    measured on its kernels), so GbmdBackend leaves it to it."""
     if live_atoms < 1_000:
         return 16
     if live_atoms < 10_000:
@@ -331,8 +328,6 @@ class GbmdBackend:
         b.set_option("graph_block", self.graph_block)
         b.live = [int(s["natoms"]) for s in systems]
         b.high = False
-        b.kind = kind
-        b.lanes = 1
         self._prioritise(b)
         b.update_forces()
         return b
@@ -344,10 +339,6 @@ class GbmdBackend:
         if not b.high and sum(b.live) <= self.small_atoms:
             b.set_option("stream_priority", 1)
             b.high = True
-        lanes = lanes_for(sum(b.live)) if b.kind == "lj" and self.precision == "mixed" else 1
-        if lanes != b.lanes:
-            b.set_option("lanes_per_atom", lanes)
-            b.lanes = lanes
 
     def device_bytes(self, b) -> int:
         return int(b.stats()["device_bytes"])

@@ -36,7 +36,7 @@ def crystal(n, a, seed, jitter=0.05):
     return np.mod(pos, L), I.maxwell_boltzmann(m, 300.0, seed=seed), m, L
 
 
-def run(systems, pot, steps, lanes=None):
+def run(systems, pot, steps, lanes=()):
     name, args, rc, _, Z = pot
     b = gbmd.Batch([len(s[0]) for s in systems], [s[3] for s in systems])
     for k, (pos, vel, m, _) in enumerate(systems):
@@ -45,8 +45,8 @@ def run(systems, pot, steps, lanes=None):
     b.add_potential(gbmd.Plugin(name, args))
     b.set_integrator(gbmd.Plugin("velocityverlet", "dt 2.0"))
     b.set_precision("mixed")
-    if lanes:
-        b.set_option("lanes_per_atom", lanes)
+    for ln in lanes:
+        b.set_option("lanes_per_atom", ln)
     b.update_forces()
     first = b.thermo(0)["raw"]
     b.do_steps(steps)
@@ -73,7 +73,16 @@ def test_record_alone_and_beside_a_large_system(kind, n, jitter):
 @pytest.mark.parametrize("lanes", [2, 4, 8, 16, 32])
 def test_record_by_lanes(lanes):
     systems = [crystal(n, POTS["lj"][3], seed=n) for n in (1001, 333)]
-    same(run(systems, POTS["lj"], 13, lanes), run(systems, POTS["lj"], 13, 1))
+    same(run(systems, POTS["lj"], 13, [lanes]), run(systems, POTS["lj"], 13, [1]))
+
+
+def test_lanes_by_size_again():
+    """0 gives the choice back to the engine; other numbers stay refused."""
+    small = crystal(1001, POTS["lj"][3], seed=3)
+    same(run([small], POTS["lj"], 13, [32, 0]), run([small], POTS["lj"], 13))
+    for ln in (3, 64, -1):
+        with pytest.raises(gbmd.GbmdError, match="lanes_per_atom"):
+            run([small], POTS["lj"], 1, [ln])
 
 
 @pytest.mark.parametrize("n", [1500, 12000])
