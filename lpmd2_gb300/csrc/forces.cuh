@@ -922,9 +922,9 @@ __global__ void __launch_bounds__(lanes_threads(LANES), 8 * TILE / lanes_threads
   if (bad) atomicOr(&D.sst[s].error, ERR_FIXED);
   // energy and virial: every lane's own fixed-point partial (exact integer sums, whatever the lane
   // count); stress: the atom's sums (halved: full list), rounded once, from its first lane
-  const float ms = sub == 0 ? (float)(-0.5 * FIX_E) : 0.0f;
-  long long v[8] = {fqe.value() * 64,      fqv.value() * 64,      fix64(stress[0] * ms), fix64(stress[1] * ms),
-                    fix64(stress[2] * ms), fix64(stress[3] * ms), fix64(stress[4] * ms), fix64(stress[5] * ms)};
+  auto fix = [&](float t) { return fix64(sub == 0 ? t * (float)(-0.5 * FIX_E) : 0.0f); };
+  long long v[8] = {fqe.value() * 64, fqv.value() * 64, fix(stress[0]), fix(stress[1]),
+                    fix(stress[2]),   fix(stress[3]),   fix(stress[4]), fix(stress[5])};
   const long long t8 = warp_sums(v);
   if ((lane & 3) == 0) esum[w][lane >> 2] = t8;
   __syncthreads();

@@ -129,3 +129,12 @@ def test_lanes_follow_the_active_systems():
         out.append((*b.atoms(0), b.thermo(0)["raw"]))
         b.close()
     same(*out)
+
+
+@pytest.mark.parametrize("lanes", [2, 4, 8, 16, 32])
+def test_record_beyond_the_fixed_point_range(lanes):
+    """Two atoms 0.001 A apart: sums that leave FP32's range are the same nonsense in every lane count."""
+    pos, vel, m, L = crystal(333, POTS["lj"][3], seed=9)
+    pos[200] = pos[100] + 0.0005
+    system = [(pos, vel, m, L)]
+    same(run(system, POTS["lj"], 0, [lanes])[3:], run(system, POTS["lj"], 0, [1])[3:])
