@@ -498,7 +498,12 @@ struct Engine::Impl {
   // How the FP64 passes cut a system (by its size and neighbour mode alone, so that its sums have the
   // same order in a batch and by itself).  List mode: 8 lanes an atom; fewer atoms a warp while the
   // system is small, so that there are several blocks for every SM.  Below 2,400 atoms, and where
-  // every candidate is tested (stencils, all pairs), a whole warp works on an atom.
+  // every candidate is tested (stencils, all pairs), a whole warp works on an atom.  Measured, LJ liquid
+  // (us between events) with lanes x atoms a warp 32 x 1 / 8 x 4 / 8 x 8 / 8 x 16: 1,372 atoms 23 / 27 / 41 /
+  // 67, 2,916 30 / 33 / 41 / 68, 4,000 47 / 33 / 41 / 68, 32,000 231 / 145 / 152 / 151, 108,000 744 / 429 /
+  // 399 / 424, 340,736 2356 / 1304 / 1189 / 1172; copper 2,048 70 / 81 / 141 / 259, 2,916 82 / 104 / 141 / 258,
+  // 4,000 113 / 107 / 142 / 262, 87,808 1637 / 1287 / 1299 / 1399, 256,000 4667 / 3586 / 3520 / 3568.  All
+  // pairs, 32 x 1 / 2 / 4: 2,048 42 / 50 / 71, 6,912 215 / 255 / 248, 32,000 3582 / 3696 / 3936.
   static void plan64(int natoms, int mode, int& lanes, int& apw) {
     if (mode != NB_LIST || natoms < 2400) {
       lanes = 32;

@@ -460,7 +460,6 @@ __global__ void __launch_bounds__(TILE, 8) k_eam_density(Dev D, PotParams P, Pai
     eam_embed64(P, rho, F, phi);
     D.rho[i] = rho;
     D.phi[i] = c.phi * phi;
-    D.phif[i] = (float)phi;
   }
   double v[1] = {F};
   double t[1];
