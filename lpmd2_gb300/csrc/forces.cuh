@@ -1,6 +1,16 @@
-// forces.cuh -- force, density and thermo kernels (one thread per atom, one block per tile of
-// 128 atoms of one system; every atom gathers over its full neighbour list, so no atomics and
-// every sum has a fixed order).
+// forces.cuh -- mixed-precision force and density kernels, and the thermo kernels of both precisions.
+// A block works on atoms of one system, an atom has one lane or several; every atom gathers over its
+// full neighbour list, so forces need no atomics.  Sums over a system are int64 fixed point (mixed) or
+// have a fixed order (FP64).
+//
+//   k_eam_density32  MetalPotential rho pass + embedding (liblpmd/simulation/metalpotential.cc:118-132,168)
+//   k_force32        PairPotential::UpdateForces (liblpmd/simulation/pairpotential.cc:35-84) or
+//                    MetalPotential's force pass (liblpmd/simulation/metalpotential.cc:137-169), with
+//                    VelocityVerlet::AdvanceVelocity (plugins/velocityverlet.cc:70-75), the next step's
+//                    drift and the thermo sums
+//   ..._lanes        the same with several lanes an atom
+//   k_tail, k_thermo thermo record (SetSimulationTags, liblpmd/simulation/simulationbuilder.cc:84-124) and
+//                    the next step's rebuild decision
 #pragma once
 
 #include "kernels.cuh"

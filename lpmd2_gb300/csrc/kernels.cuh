@@ -11,16 +11,15 @@
 //   k_cellsort     orders each cell by original atom index (the reference's linked-list order)
 //   k_permute      gathers every per-atom field into the new cell-sorted order (scratch)
 //   k_copyback     writes the sorted fields back, refreshes gather copies and home cells
-//   k_buildlist    Verlet list from the 27/125-cell stencil with per-pair cell-shift codes
+//   k_sort_cluster the same sort in one launch, for small systems
+//   k_buildlist_block, k_buildlist_warp
+//                  Verlet list from the 27/125-cell stencil with per-pair cell-shift codes, a block or
+//                  a warp for each home cell
+//   k_scale_*      velocity rescaling between steps
 //   k_drift        VelocityVerlet::AdvancePosition (plugins/velocityverlet.cc:60-68) + wrap,
-//                  gather copies, displacement tracking
-//   k_pair_force   PairPotential::UpdateForces (liblpmd/simulation/pairpotential.cc:35-84)
-//                  as a full-list gather, fused with VelocityVerlet::AdvanceVelocity
-//                  (plugins/velocityverlet.cc:70-75) and the per-tile thermo sums
-//   k_eam_density  MetalPotential rho pass + embedding (liblpmd/simulation/metalpotential.cc:118-132,168)
-//   k_eam_force    MetalPotential force pass (liblpmd/simulation/metalpotential.cc:137-169)
-//   k_thermo       per-system reduction of the tile sums into the thermo record
-//                  (SetSimulationTags, liblpmd/simulation/simulationbuilder.cc:84-124)
+//                  gather copies, displacement tracking (stand-alone; a step's drift is part of the
+//                  force pass before it)
+// The force, density and thermo kernels are in forces.cuh (mixed precision) and force64.cuh (FP64).
 #pragma once
 
 #include <type_traits>
