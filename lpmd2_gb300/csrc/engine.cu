@@ -556,7 +556,8 @@ struct Engine::Impl {
     plan.n = (int)blk.size();
     CK(dev_malloc(&plan.blk, sizeof(Blk32) * std::max<size_t>(blk.size(), 1)));
     CK(cudaMemcpyAsync(plan.blk, blk.data(), sizeof(Blk32) * blk.size(), cudaMemcpyHostToDevice, stream));
-    return plan;  // (a copy from pageable memory has read it when it returns)
+    CK(cudaStreamSynchronize(stream));  // the copy has read the table
+    return plan;
   }
   void ensure_plan32() {
     const int wide = auto_lanes(), pair = lanes ? lanes : wide;
@@ -608,6 +609,7 @@ struct Engine::Impl {
     D.ticket64 = (unsigned*)(db + blk.size());
     CK(cudaMemcpyAsync(dp, per.data(), sizeof(int2) * per.size(), cudaMemcpyHostToDevice, stream));
     CK(cudaMemcpyAsync(db, blk.data(), sizeof(Blk64) * blk.size(), cudaMemcpyHostToDevice, stream));
+    CK(cudaStreamSynchronize(stream));  // the copies have read the tables
   }
   std::vector<Blk64> plan64_blk;  // as last laid out
   int nblk64 = 0, shares64 = 1;
