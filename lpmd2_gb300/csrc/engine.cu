@@ -592,8 +592,8 @@ struct Engine::Impl {
     const bool same = D.blk64 && blk.size() == plan64_blk.size() &&
                       std::memcmp(blk.data(), plan64_blk.data(), sizeof(Blk64) * blk.size()) == 0;
     if (same) return;
-    plan64_blk = blk;
     nblk64 = (int)blk.size();
+    D.blk64 = nullptr;
     free_scratch();
     // one allocation: partial sums (one record per tile is part of the set-up pool; finer cuts have their
     // own), shares, the block table, the systems' runs of blocks, tickets (zeroed)
@@ -605,11 +605,12 @@ struct Engine::Impl {
     int2* dp = (int2*)(d + np + ns);
     Blk64* db = (Blk64*)(dp + nsys);
     D.sys64 = dp;
-    D.blk64 = db;
     D.ticket64 = (unsigned*)(db + blk.size());
     CK(cudaMemcpyAsync(dp, per.data(), sizeof(int2) * per.size(), cudaMemcpyHostToDevice, stream));
     CK(cudaMemcpyAsync(db, blk.data(), sizeof(Blk64) * blk.size(), cudaMemcpyHostToDevice, stream));
     CK(cudaStreamSynchronize(stream));  // the copies have read the tables
+    D.blk64 = db;
+    plan64_blk = blk;
   }
   std::vector<Blk64> plan64_blk;  // as last laid out
   int nblk64 = 0, shares64 = 1;
